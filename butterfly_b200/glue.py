@@ -86,7 +86,9 @@ def butterfly_multiply_glue(twiddle: torch.Tensor, input: torch.Tensor, increasi
     n = 1 << twiddle.shape[2]
     limit = 2048 if twiddle.is_complex() else 4096
     width = input.shape[-1]
-    if n > limit or width > n or (width < n and in_perm is not None) or not input.is_cuda:
+    if in_perm is not None and width < n:  # the gather would read past the row, which a GPU answers with a lost context
+        raise RuntimeError("butterfly_multiply_glue: in_perm needs rows of %d entries, got %d" % (n, width))
+    if n > limit or width > n or not input.is_cuda:
         return _unfused(twiddle, input, increasing_stride, in_perm, out_diag, out_perm, out_real)
     if not (torch.is_grad_enabled() and (input.requires_grad or twiddle.requires_grad
                                          or (out_diag is not None and out_diag.requires_grad))):
@@ -118,6 +120,8 @@ class ButterflyPipeline(nn.Module):
     def forward(self, input):
         b = self.butterfly
         width = input.shape[-1]
+        if b.in_size == b.n and width != b.n:  # (a narrower layer pads or trims its rows, whole ones take none but their own)
+            raise RuntimeError("ButterflyPipeline: rows of %d entries expected, got %d" % (b.n, width))
         rows = input.unsqueeze(1) if input.dim() == 2 else input.reshape(-1, 1, width)
         if not self.real_in and b.complex and not rows.is_complex():
             rows = rows.to(b.twiddle.dtype)
