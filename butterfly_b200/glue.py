@@ -98,6 +98,29 @@ def butterfly_multiply_glue(twiddle: torch.Tensor, input: torch.Tensor, increasi
     return _Glue.apply(twiddle, input, increasing_stride, in_perm, out_diag, out_perm, out_real)
 
 
+def _rename_links(state_dict, prefix, links):
+    """State saved from a chain link by link, under the names of its fused form (no-op for state saved from that form)."""
+    fused = tuple(prefix + new for _, new in links if new.endswith("butterfly."))  # every pipeline has one, no link does
+    if not fused or any(k.startswith(fused) for k in state_dict):
+        return
+    moved = {}
+    for k in list(state_dict):
+        for old, new in links:
+            if k.startswith(prefix + old):
+                moved[prefix + new + k[len(prefix + old):]] = state_dict.pop(k)
+                break
+    state_dict.update(moved)
+
+
+class FusedChain(nn.Sequential):
+    """What fuse() makes of a chain: loads the state of the fused and of the link-by-link form."""
+    links = ()
+
+    def _load_from_state_dict(self, state_dict, prefix, *args):
+        _rename_links(state_dict, prefix, self.links)
+        super()._load_from_state_dict(state_dict, prefix, *args)
+
+
 class ButterflyPipeline(nn.Module):
     """[Real2Complex] [FixedPermutation] Butterfly [Diagonal] [FixedPermutation] [Complex2Real] as one
     module and one launch.  The Butterfly (single stack, no bias; an input narrower than n is zero-padded, an
@@ -116,6 +139,13 @@ class ButterflyPipeline(nn.Module):
         self.real_in, self.real_out = real_in, real_out
         self.register_buffer("in_perm", None if in_perm is None else in_perm.to(torch.int32))
         self.register_buffer("out_perm", None if out_perm is None else out_perm.to(torch.int32))
+
+    #: names of the state a chain kept link by link -> names here (set by fuse)
+    links = ()
+
+    def _load_from_state_dict(self, state_dict, prefix, *args):
+        _rename_links(state_dict, prefix, self.links)
+        super()._load_from_state_dict(state_dict, prefix, *args)
 
     def forward(self, input):
         b = self.butterfly
@@ -140,30 +170,47 @@ def _fusible_butterfly(m) -> bool:
 def fuse(chain: nn.Sequential) -> nn.Sequential:
     """The same function as `chain` with every run of
     [Real2Complex] [FixedPermutation] Butterfly [Diagonal] [FixedPermutation] [Complex2Real]
-    replaced by one ButterflyPipeline.  Links that do not fit the pattern are kept as they are."""
-    mods = list(chain)
-    out, i = [], 0
+    replaced by one ButterflyPipeline.  Links that do not fit the pattern are kept as they are, and so is a Butterfly of
+    padded or cut rows with nothing to fold into it.  The result loads state saved from either form."""
+    names, mods = list(chain._modules), list(chain)
+    out, renames, i = [], [], 0
     while i < len(mods):
         j, real_in, in_perm = i, False, None
         if isinstance(mods[j], Real2Complex) and j + 1 < len(mods):
             real_in, j = True, j + 1
+        links = []
         if isinstance(mods[j], FixedPermutation) and j + 1 < len(mods):
+            links.append((names[j] + ".permutation", "in_perm"))
             in_perm, j = mods[j].permutation, j + 1
-        if not _fusible_butterfly(mods[j]) or (real_in and not mods[j].complex) or (
-                in_perm is not None and (in_perm.shape[-1] != mods[j].n or mods[j].in_size != mods[j].n)):
+        b, at = mods[j], j
+        fits = _fusible_butterfly(b) and (b.complex or not real_in) and (
+            in_perm is None or (in_perm.shape[-1] == b.n and b.in_size == b.n))
+        diagonal, out_perm, real_out = None, None, False
+        if fits:
+            links.append((names[j] + ".", "butterfly."))
+            j += 1
+            whole = b.out_size == b.n
+            if whole and j < len(mods) and isinstance(mods[j], Diagonal) and mods[j].diagonal.shape == (b.n,) \
+                    and mods[j].diagonal.dtype == b.twiddle.dtype:
+                links.append((names[j] + ".", "diagonal."))
+                diagonal, j = mods[j], j + 1
+            if whole and j < len(mods) and isinstance(mods[j], FixedPermutation) and mods[j].permutation.shape[-1] == b.n:
+                links.append((names[j] + ".permutation", "out_perm"))
+                out_perm, j = mods[j].permutation, j + 1
+            if j < len(mods) and isinstance(mods[j], Complex2Real) and b.complex:
+                real_out, j = True, j + 1
+            alone = i == at and j == at + 1
+            fits = not alone or (b.in_size == b.n and whole)
+        if not fits:
+            renames.append((names[i] + ".", "%d." % len(out)))
             out.append(mods[i])
             i += 1
             continue
-        b, j = mods[j], j + 1
-        diagonal, out_perm, real_out = None, None, False
-        whole = b.out_size == b.n
-        if whole and j < len(mods) and isinstance(mods[j], Diagonal) and mods[j].diagonal.shape == (b.n,) \
-                and mods[j].diagonal.dtype == b.twiddle.dtype:
-            diagonal, j = mods[j], j + 1
-        if whole and j < len(mods) and isinstance(mods[j], FixedPermutation) and mods[j].permutation.shape[-1] == b.n:
-            out_perm, j = mods[j].permutation, j + 1
-        if j < len(mods) and isinstance(mods[j], Complex2Real) and b.complex:
-            real_out, j = True, j + 1
-        out.append(ButterflyPipeline(b, in_perm, diagonal, out_perm, real_in, real_out))
+        pipe = ButterflyPipeline(b, in_perm, diagonal, out_perm, real_in, real_out)
+        pipe.links = tuple(links)
+        renames += [(old, "%d.%s" % (len(out), new)) for old, new in links]
+        out.append(pipe)
         i = j
-    return nn.Sequential(*out)
+    fused = FusedChain(*out)
+    fused.links = tuple(renames)
+    return fused
