@@ -48,6 +48,11 @@ Tensor rows_view(const Tensor& t) {
   return r;
 }
 
+// Does a call see a forward-mode tangent on this tensor?  Paths around an autograd node ask, because the node is what
+// refuses tangents (no operator here has a forward-mode rule); without it they would be dropped without a word.
+bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
+bool has_tangent(const c10::optional<Tensor>& t) { return t.has_value() && has_tangent(*t); }
+
 // Shared by the plain operator and the autograd node: with `snapshots` the forward also writes
 // the activations the backward starts its phases from (bfly_fw_*_saving).
 Tensor fw_impl(const Tensor& twiddle, const Tensor& input, bool increasing_stride,
@@ -383,9 +388,10 @@ class ButterflyLayer : public torch::autograd::Function<ButterflyLayer> {
 Tensor butterfly_layer(const Tensor& twiddle, const c10::optional<Tensor>& twiddle2, const Tensor& input,
                        const c10::optional<Tensor>& bias, bool increasing_stride, int64_t out_size) {
   auto needs = [](const c10::optional<Tensor>& t) { return t.has_value() && t->defined() && t->requires_grad(); };
-  if (!at::GradMode::is_enabled() || !(twiddle.requires_grad() || input.requires_grad() || needs(twiddle2) || needs(bias)))
+  const bool wants_grad = at::GradMode::is_enabled() && (twiddle.requires_grad() || input.requires_grad() || needs(twiddle2) || needs(bias));
+  if (!wants_grad && !has_tangent(twiddle) && !has_tangent(input) && !has_tangent(twiddle2) && !has_tangent(bias))
     return layer_fw(twiddle, twiddle2.has_value() ? *twiddle2 : Tensor(), input, bias, increasing_stride, out_size, nullptr);
-  return ButterflyLayer::apply(twiddle, twiddle2, input, bias, increasing_stride, out_size, true);
+  return ButterflyLayer::apply(twiddle, twiddle2, input, bias, increasing_stride, out_size, wants_grad);
 }
 
 // The float32 layer on (batch, in_size) rows as stateless operators and as a differentiable one.
@@ -544,6 +550,9 @@ c10::optional<Tensor> butterfly_multiply_glue_fw(const Tensor& twiddle, const Te
   TORCH_CHECK(twiddle.sizes() == torch::IntArrayRef({nstacks, nblocks, log_n, n / 2, 2, 2}),
               "twiddle must have shape (nstacks, nblocks, log_n, n / 2, 2, 2)");
   TORCH_CHECK(input_size <= n, "butterfly_multiply_glue_fw: input_size must be <= n");
+  // (inside the autograd node of glue.py forward mode is off, and the node refuses tangents itself)
+  TORCH_CHECK(!c10::AutogradState::get_tls_state().get_fw_grad_mode() || !(has_tangent(twiddle) || has_tangent(input) || has_tangent(out_diag)),
+              "butterfly_multiply_glue_fw: forward-mode differentiation is not implemented");
   const bool cplx = twiddle.scalar_type() == at::kComplexFloat;
   TORCH_CHECK(cplx || twiddle.scalar_type() == at::kFloat, "butterfly_multiply_glue_fw: float32 or complex64 twiddle expected");
   const bool x_real = cplx && input.scalar_type() == at::kFloat;
