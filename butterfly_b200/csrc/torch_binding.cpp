@@ -323,6 +323,9 @@ Tensor layer_fw(const Tensor& twiddle, const Tensor& twiddle2, const Tensor& inp
                                scratch > 0 ? ws.data_ptr() : nullptr, (size_t)std::max<int64_t>(scratch, 0),
                                at::cuda::getCurrentCUDAStream().stream());
   check_status(rc, "butterfly_layer");
+  // A view that autograd knows as one, made inside the node, would refuse every in-place operator behind the layer
+  // (ReLU(inplace=True)); below its dispatch keys the same view is a tensor of its own, and nothing else sees its base.
+  at::AutoDispatchBelowADInplaceOrView no_view_tracking;
   if (input.dim() == 2) return out_size < c.width ? output.narrow(1, 0, out_size) : output;
   auto shape = input.sizes().vec();
   shape.back() = c.width;

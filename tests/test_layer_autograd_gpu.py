@@ -48,3 +48,22 @@ def test_pipelines_refuse_forward_mode(dev, what):
             bb.butterfly_multiply_glue(dual("twiddle", tw), dual("input", x), True, out_diag=dual("diagonal", diag))
         with pytest.raises(RuntimeError, match="forward.mode|jvp"):  # with a gradient asked for as well
             bb.butterfly_multiply_glue(dual("twiddle", tw), dual("input", x), True, out_diag=dual("diagonal", diag.requires_grad_(True)))
+
+
+@pytest.mark.parametrize("kind,in_size,out_size,lead,bias", [
+    ("f32", 64, 64, (3, 5), True), ("f32", 64, 64, (7,), True), ("f32", 64, 100, (7,), True), ("f32", 64, 50, (2, 7), False), ("c64", 64, 50, (7,), True),
+    ("c64", 64, 64, (3, 4), True), ("base4", 64, 50, (7,), True), ("base4", 64, 64, (), True)])
+def test_layer_outputs_take_in_place_operators(dev, kind, in_size, out_size, lead, bias):
+    """nn.ReLU(inplace=True) behind a layer: whatever the rank and the cut, the output is a tensor of its own."""
+    torch.manual_seed(3)
+    layer = _layer(kind, in_size, out_size, dev, bias=bias)
+    x = torch.randn(*lead, in_size, dtype=torch.complex64 if kind == "c64" else torch.float32, device=dev, requires_grad=True)
+    scale = torch.randn(*lead, out_size, dtype=x.dtype, device=dev)
+
+    def grads(in_place):
+        y = layer(x)
+        assert y.shape == scale.shape and not y._is_view()
+        z = y.mul_(scale) if in_place else y * scale
+        return [z.detach().clone()] + list(torch.autograd.grad(z.abs().sum(), [x] + list(p for p in layer.parameters() if p.numel())))
+    for a, b in zip(grads(True), grads(False)):
+        assert a.shape == b.shape and (a - b).abs().max() <= 1e-5 * b.abs().max()
