@@ -139,10 +139,9 @@ BFLY_HD int gather_column(int at, int i, const uint8_t* colbit, int logC, int nt
 // source << 16 | its own place); then, a few wide rows at a time, all threads read their sources (times diag[source]
 // when a diagonal is given), and after a barrier write their own places.  `total`: elements of the tile from wide row
 // r on.
-template <typename T, int SLOTS = kGlueSlots>
+template <typename T, int SLOTS>
 BFLY_HD int tile_permute_plan(int logC, const int32_t* __restrict__ perm, const uint8_t* colbit, int tid, int nthr, uint32_t* plan,
-                              int mask = 0xffff, int logW = 0) {
-  if (logW == 0) logW = logC;
+                              int mask, int logW) {
   const int W = 1 << logW, in_row = (1 << logC) - 1, at = deposit_unit(tid, colbit, logW);
   int cnt = 0;
 #pragma unroll
@@ -155,10 +154,9 @@ BFLY_HD int tile_permute_plan(int logC, const int32_t* __restrict__ perm, const 
   }
   return cnt;
 }
-template <typename T, int SLOTS = kGlueSlots, int ROWS = 1>
+template <typename T, int SLOTS, int ROWS>
 BFLY_HD void tile_permute_read(const T* __restrict__ sm, int r, int logC, const T* __restrict__ diag, const uint32_t* plan, int cnt, T* v,
-                               int mask = 0xffff, int logW = 0, int total = 1 << 30) {
-  if (logW == 0) logW = logC;
+                               int mask, int logW, int total) {
   const T* row = sm + ((size_t)r << logW);
 #pragma unroll
   for (int k = 0; k < SLOTS; ++k) {  // fixed bound: plan and v stay in registers
@@ -174,10 +172,8 @@ BFLY_HD void tile_permute_read(const T* __restrict__ sm, int r, int logC, const 
     }
   }
 }
-template <typename T, int SLOTS = kGlueSlots, int ROWS = 1>
-BFLY_HD void tile_permute_write(T* __restrict__ sm, int r, int logC, const uint32_t* plan, int cnt, const T* v, int logW = 0,
-                                int total = 1 << 30) {
-  if (logW == 0) logW = logC;
+template <typename T, int SLOTS, int ROWS>
+BFLY_HD void tile_permute_write(T* __restrict__ sm, int r, const uint32_t* plan, int cnt, const T* v, int logW, int total) {
   T* row = sm + ((size_t)r << logW);
 #pragma unroll
   for (int k = 0; k < SLOTS; ++k) {
@@ -186,45 +182,6 @@ BFLY_HD void tile_permute_write(T* __restrict__ sm, int r, int logC, const uint3
 #pragma unroll
     for (int j = 0; j < ROWS; ++j)
       if ((j << logW) + own < total) row[(j << logW) + own] = v[j * SLOTS + k];
-  }
-}
-
-// Diagonal without a gather: y[c] *= diag[c] in place, 16 bytes at a time; a thread keeps its
-// columns' diagonal entries in registers over the rows of the tile.  No barrier needed inside.  (The host model of the
-// kernel; on the device the diagonal goes with the store, tile_store_scaled.)
-template <typename T>
-BFLY_HD void tile_scale_rows(T* __restrict__ sm, int R, int logC, const T* __restrict__ diag, int tid, int nthr) {
-  constexpr int V = Vec16<T>::N, VL = Vec16<T>::LOG;
-  const int C = 1 << logC;
-  if (logC < VL) {
-    for (int e = tid; e < R * C; e += nthr) {
-      const int l = e & (C - 1);
-      T* q = sm + (e >> logC) * C + swzT<T>(l);
-      *q = Ops<T>::mul(*q, diag[l]);
-    }
-    return;
-  }
-  constexpr int kChunks = kGlueSlots / V;  // chunks per thread and row when C / nthr == kGlueSlots
-  T d[kChunks][V];
-#pragma unroll
-  for (int k = 0; k < kChunks; ++k) {
-    const int l = (tid + k * nthr) << VL;
-    if (l >= C) break;
-#pragma unroll
-    for (int i = 0; i < V; ++i) d[k][i] = diag[l + i];
-  }
-  for (int r = 0; r < R; ++r) {
-#pragma unroll
-    for (int k = 0; k < kChunks; ++k) {
-      const int l = (tid + k * nthr) << VL;
-      if (l >= C) break;
-      T* q = sm + r * C + swzT<T>(l);  // the swizzle moves whole 16-byte chunks
-      T v[V];
-      sm_ld16<0>(sm_addr(q), v);
-#pragma unroll
-      for (int i = 0; i < V; ++i) v[i] = Ops<T>::mul(v[i], d[k][i]);
-      sm_st16<0>(sm_addr(q), v);
-    }
   }
 }
 

@@ -98,7 +98,7 @@ __device__ __noinline__ void permute_tile(T* sm, int R, int logC, const int32_t*
   for (int left = R << logC, r = 0; left > 0; left -= RB << kWide, r += RB) {
     tile_permute_read<T, SL, RB>(sm, r, logC, diag, plan, cnt, v, mask, kWide, left);
     __syncthreads();
-    tile_permute_write<T, SL, RB>(sm, r, logC, plan, cnt, v, kWide, left);
+    tile_permute_write<T, SL, RB>(sm, r, plan, cnt, v, kWide, left);
   }
   __syncthreads();
 }

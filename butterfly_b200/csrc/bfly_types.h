@@ -190,7 +190,6 @@ template <typename T> struct FwGlue {
   // gathers: bit j of (thread + k * threads) becomes bit colbit[j] of the column a thread owns (glue_column_bits)
   uint8_t colbit[16];
   BFLY_HD bool any_in() const { return in_perm != nullptr; }
-  BFLY_HD bool any_out() const { return out_perm != nullptr || out_diag != nullptr; }
 };
 
 template <typename T> struct FwParams {

@@ -85,6 +85,8 @@ struct EmulExec {
     // what the TMA descriptors would refuse: widths that are not whole 32-column blocks, and, for
     // panels made of strided segments, rows that are not whole groups of segments
     if (!bw3 || !q.vec_x || !q.vec_g || !q.vec_o || q.xin_cols % 32 || q.gin_cols % 32 || q.gout_cols % 32) return false;
+    if (q.xin_cols < 32 || q.gin_cols < 32 || q.gout_cols < 32 || (q.gin_flat > 0 && q.gin_flat != q.S << q.log_n)) return false;
+    if (q.vr > 0) return q.log_n >= 5 && (kBw3Rows << q.vr) <= 256;  // whole rows, as many as a box takes
     if (q.panel.lseg != q.panel.logC) {
       const int grp = 1 << q.panel.pb;
       for (int cols : {q.xin_cols, q.gin_cols, q.gout_cols})
@@ -115,27 +117,28 @@ struct EmulExec {
       }
       for (int row0 = rb; row0 < re; row0 += kBw3Rows) {
         for (int tid = 0; tid < nthr; ++tid) {
-          tile_load_auto<float>(q.xin, q.xin_sB, q.xin_sS, q.xin_cols, q.B, stack, row0, kBw3Rows, q.panel, pbase, true, smX, tid, nthr);
-          tile_load_auto<float>(q.gin, q.gin_sB, q.gin_sS, q.gin_cols, q.B, stack, row0, kBw3Rows, q.panel, pbase, true, smG, tid, nthr);
+          tile_load_v<float>(q.xin, q.xin_sB, q.xin_sS, q.xin_cols, q.B_rows, stack, row0, kBw3Rows, q.panel, pbase, true, q.log_n, q.vr, smX, tid, nthr);
+          tile_load_v<float>(q.gin, q.gin_sB, q.gin_sS, q.gin_cols, q.B_rows, stack, row0, kBw3Rows, q.panel, pbase, true, q.log_n, q.vr, smG, tid, nthr);
         }
         if (q.dbias)  // column sums of the gradient tile as it arrived
           for (int r = 0; r < kBw3Rows; ++r)
             for (int l = 0; l < C; ++l) {
-              const int flat = stack * (1 << q.log_n) + q.panel.col(pbase, l);
+              const int flat = stack * (1 << q.log_n) + (q.panel.col(pbase, l) & ((1 << q.log_n) - 1));
               if (flat < q.dbias_len) q.dbias[flat] += smG[r * C + swz<2>(l)];
             }
         for (int step = 0; step < bw3_num_steps(q.nsg); ++step)
           for (int tid = 0; tid < nthr; ++tid)
             bw3_step(p, accs[tid], meta.data(), step, smem.data(), tid, pf.data() + (size_t)tid * 64, pf.data() + (size_t)tid * 64 + 32);
         if (q.gout_reduce) {  // the device kernel's reduce-add store
-          for (int r = 0; r < kBw3Rows && row0 + r < q.B; ++r)
+          for (int r = 0; r < kBw3Rows; ++r)
             for (int l = 0; l < C; ++l) {
-              const int col = q.panel.col(pbase, l);
-              if (col < q.gout_cols) q.gout[(int64_t)(row0 + r) * q.gout_sB + (int64_t)stack * q.gout_sS + col] += smG[r * C + swz<2>(l)];
+              const int at = q.panel.col(pbase, l), col = at & ((1 << q.log_n) - 1);
+              const int64_t row = ((int64_t)(row0 + r) << q.vr) + (at >> q.log_n);
+              if (row < q.B_rows && col < q.gout_cols) q.gout[row * q.gout_sB + (int64_t)stack * q.gout_sS + col] += smG[r * C + swz<2>(l)];
             }
         } else {
           for (int tid = 0; tid < nthr; ++tid)
-            tile_store_auto<float>(q.gout, q.gout_sB, q.gout_sS, q.gout_cols, q.B, stack, row0, kBw3Rows, q.panel, pbase, true, smG, tid, nthr);
+            tile_store_v<float>(q.gout, q.gout_sB, q.gout_sS, q.gout_cols, q.B_rows, stack, row0, kBw3Rows, q.panel, pbase, true, q.log_n, q.vr, smG, tid, nthr);
         }
       }
       for (int tid = 0; tid < nthr; ++tid) bw3_flush(p, accs[tid], stack, pbase, tid);
@@ -154,22 +157,24 @@ struct EmulExec {
       int row0, stack, pbase;
       fw_tile_coords(p, tile, row0, stack, pbase);
       for (int tid = 0; tid < threads_; ++tid) {
-        if (p.glue.x_real) tile_load_real(p.glue.x_real, p.x_sB, p.x_sS, p.x_cols, p.B, stack, row0, p.R, p.panel.logC, sm.data(), tid, threads_);
-        else tile_load_auto<T>(p.x, p.x_sB, p.x_sS, p.x_cols, p.B, stack, row0, p.R, p.panel, pbase, p.vec_in != 0, sm.data(), tid, threads_);
+        if (p.glue.x_real) tile_load_real(p.glue.x_real, p.x_sB, p.x_sS, p.x_cols, p.B_rows, stack, row0, p.R, p.panel.logC, sm.data(), tid, threads_, p.vr);
+        else tile_load_v<T>(p.x, p.x_sB, p.x_sS, p.x_cols, p.B_rows, stack, row0, p.R, p.panel, pbase, p.vec_in != 0, p.log_n, p.vr, sm.data(), tid, threads_);
       }
-      // the kernel's gather pass: every thread reads, barrier, every thread writes
+      // the kernel's gather pass: wide rows of the same width, three at a time: every thread reads, barrier, every thread writes
       auto permute_rows = [&](const int32_t* perm, const T* diag) {
-        const int slots = (C + threads_ - 1) / threads_;
-        std::vector<T> v((size_t)threads_ * slots);
-        std::vector<uint32_t> plan((size_t)threads_ * slots);
+        constexpr int kWide = sizeof(T) == 8 ? 11 : 12, kSlots = 64, RB = 3;
+        if ((1 << kWide) > kSlots * threads_) { std::fprintf(stderr, "emulated gathers need %d threads\n", (1 << kWide) / kSlots); std::abort(); }
+        std::vector<T> v((size_t)threads_ * RB * kSlots);
+        std::vector<uint32_t> plan((size_t)threads_ * kSlots);
         std::vector<int> cnt(threads_);
+        const int mask = (int)n - 1;
         for (int tid = 0; tid < threads_; ++tid)
-          cnt[tid] = tile_permute_plan<T>(p.panel.logC, perm, p.glue.colbit, tid, threads_, plan.data() + (size_t)tid * slots);
-        for (int r = 0; r < p.R; ++r) {
+          cnt[tid] = tile_permute_plan<T, kSlots>(p.panel.logC, perm, p.glue.colbit, tid, threads_, plan.data() + (size_t)tid * kSlots, mask, kWide);
+        for (int left = p.R << p.panel.logC, r = 0; left > 0; left -= RB << kWide, r += RB) {
           for (int tid = 0; tid < threads_; ++tid)
-            tile_permute_read<T>(sm.data(), r, p.panel.logC, diag, plan.data() + (size_t)tid * slots, cnt[tid], v.data() + (size_t)tid * slots);
+            tile_permute_read<T, kSlots, RB>(sm.data(), r, p.panel.logC, diag, plan.data() + (size_t)tid * kSlots, cnt[tid], v.data() + (size_t)tid * RB * kSlots, mask, kWide, left);
           for (int tid = 0; tid < threads_; ++tid)
-            tile_permute_write<T>(sm.data(), r, p.panel.logC, plan.data() + (size_t)tid * slots, cnt[tid], v.data() + (size_t)tid * slots);
+            tile_permute_write<T, kSlots, RB>(sm.data(), r, plan.data() + (size_t)tid * kSlots, cnt[tid], v.data() + (size_t)tid * RB * kSlots, kWide, left);
         }
       };
       if (p.glue.any_in()) permute_rows(p.glue.in_perm, nullptr);
@@ -178,18 +183,25 @@ struct EmulExec {
           fw_group_dispatch<T, 4, 0, 0>(p, g, sm.data(), tab.data(), p.R, stack, pbase, tid, threads_);
         if (p.g[g].emit)
           for (int tid = 0; tid < threads_; ++tid)
-            tile_store_auto<T>(p.snap[p.g[g].emit - 1], (int64_t)p.S * n, n, (int)n, p.B, stack, row0, p.R, p.panel, pbase, true, sm.data(), tid, threads_);
+            tile_store_v<T>(p.snap[p.g[g].emit - 1], (int64_t)p.S * n, n, (int)n, p.B_rows, stack, row0, p.R, p.panel, pbase, true, p.log_n, p.vr, sm.data(), tid, threads_);
       }
-      if (p.glue.any_out()) {
-        if (p.glue.out_perm) permute_rows(p.glue.out_perm, p.glue.out_diag);
-        else for (int tid = 0; tid < threads_; ++tid) tile_scale_rows<T>(sm.data(), p.R, p.panel.logC, p.glue.out_diag, tid, threads_);
+      if (p.bias)
+        for (int tid = 0; tid < threads_; ++tid)
+          tile_add_bias<T>(sm.data(), p.R, p.panel, pbase, p.bias, stack * (int)n, p.bias_len, (int)n - 1, tid, threads_);
+      if (p.glue.out_perm) permute_rows(p.glue.out_perm, p.glue.out_diag);
+      const bool scaled = p.glue.out_diag && !p.glue.out_perm;  // a diagonal alone goes with the store
+      for (int tid = 0; tid < threads_; ++tid) {
+        if (scaled && p.glue.out_real)
+          tile_store_scaled<T>(p.glue.out_real, p.out_sB, p.out_sS, p.out_cols, p.B_rows, stack, row0, p.R, p.panel.logC, p.log_n, p.vr,
+                               p.glue.out_diag, sm.data(), tid, threads_);
+        else if (scaled)
+          tile_store_scaled<T>(p.out, p.out_sB, p.out_sS, p.out_cols, p.B_rows, stack, row0, p.R, p.panel.logC, p.log_n, p.vr,
+                               p.glue.out_diag, sm.data(), tid, threads_);
+        else if (p.glue.out_real)
+          tile_store_real(p.glue.out_real, p.out_sB, p.out_sS, p.out_cols, p.B_rows, stack, row0, p.R, p.panel.logC, sm.data(), tid, threads_, p.vr);
+        else if (p.out)
+          tile_store_v<T>(p.out, p.out_sB, p.out_sS, p.out_cols, p.B_rows, stack, row0, p.R, p.panel, pbase, p.vec_out != 0, p.log_n, p.vr, sm.data(), tid, threads_);
       }
-      if (p.glue.out_real)
-        for (int tid = 0; tid < threads_; ++tid)
-          tile_store_real(p.glue.out_real, p.out_sB, p.out_sS, p.out_cols, p.B, stack, row0, p.R, p.panel.logC, sm.data(), tid, threads_);
-      else if (p.out)
-        for (int tid = 0; tid < threads_; ++tid)
-          tile_store_auto<T>(p.out, p.out_sB, p.out_sS, p.out_cols, p.B, stack, row0, p.R, p.panel, pbase, p.vec_out != 0, sm.data(), tid, threads_);
     }
     return BFLY_OK;
   }
@@ -217,8 +229,8 @@ struct EmulExec {
       for (int tid = 0; tid < nthr; ++tid) bw2_init<T, KW>(p, accs[tid], meta.data(), stack, tid, nthr);
       for (int row0 = rb; row0 < re; row0 += kBw2Rows) {
         for (int tid = 0; tid < nthr; ++tid) {
-          tile_load_auto<T>(p.xin, p.xin_sB, p.xin_sS, p.xin_cols, re, stack, row0, kBw2Rows, p.panel, pbase, p.vec_x != 0, smX.data(), tid, nthr);
-          tile_load_auto<T>(p.gin, p.gin_sB, p.gin_sS, p.gin_cols, re, stack, row0, kBw2Rows, p.panel, pbase, p.vec_g != 0, smG.data(), tid, nthr);
+          tile_load_v<T>(p.xin, p.xin_sB, p.xin_sS, p.xin_cols, bw_row_limit(p, re), stack, row0, kBw2Rows, p.panel, pbase, p.vec_x != 0, p.log_n, p.vr, smX.data(), tid, nthr);
+          tile_load_v<T>(p.gin, p.gin_sB, p.gin_sS, bw_gin_cols(p, stack), bw_row_limit(p, re), stack, row0, kBw2Rows, p.panel, pbase, p.vec_g != 0, p.log_n, p.vr, smG.data(), tid, nthr);
         }
         for (int j = 0; j + 1 < p.nsg; ++j)
           for (int tid = 0; tid < nthr; ++tid)
@@ -227,7 +239,7 @@ struct EmulExec {
           for (int tid = 0; tid < nthr; ++tid)
             bw2_bw_step<T, KW, 0>(p, accs[tid], meta.data(), j, smX.data(), smG.data(), tid, nthr);
         for (int tid = 0; tid < nthr; ++tid)
-          tile_store_auto<T>(p.gout, p.gout_sB, p.gout_sS, p.gout_cols, re, stack, row0, kBw2Rows, p.panel, pbase, p.vec_o != 0, smG.data(), tid, nthr);
+          tile_store_v<T>(p.gout, p.gout_sB, p.gout_sS, p.gout_cols, bw_row_limit(p, re), stack, row0, kBw2Rows, p.panel, pbase, p.vec_o != 0, p.log_n, p.vr, smG.data(), tid, nthr);
       }
       for (int tid = 0; tid < nthr; ++tid) bw2_flush<T, KW>(p, accs[tid], meta.data(), stack, tid, nthr);
     }
@@ -252,15 +264,15 @@ struct EmulExec {
       for (int row0 = rb; row0 < re; row0 += p.Rb) {
         const int R = p.Rb;
         for (int tid = 0; tid < nthr; ++tid) {
-          tile_load_auto<T>(p.xin, p.xin_sB, p.xin_sS, p.xin_cols, re, stack, row0, R, p.panel, pbase, p.vec_x != 0, smX.data(), tid, nthr);
-          tile_load_auto<T>(p.gin, p.gin_sB, p.gin_sS, p.gin_cols, re, stack, row0, R, p.panel, pbase, p.vec_g != 0, smG.data(), tid, nthr);
+          tile_load_v<T>(p.xin, p.xin_sB, p.xin_sS, p.xin_cols, bw_row_limit(p, re), stack, row0, R, p.panel, pbase, p.vec_x != 0, p.log_n, p.vr, smX.data(), tid, nthr);
+          tile_load_v<T>(p.gin, p.gin_sB, p.gin_sS, bw_gin_cols(p, stack), bw_row_limit(p, re), stack, row0, R, p.panel, pbase, p.vec_g != 0, p.log_n, p.vr, smG.data(), tid, nthr);
         }
         for (int j = 0; j + 1 < p.nsg; ++j)
           for (int tid = 0; tid < nthr; ++tid) bw_sg_step<T, KW, NSG, 0, 0, true>(p, st[tid], j, stack, smX.data(), smG.data(), R, tid, nthr);
         for (int j = p.nsg - 1; j >= 0; --j)
           for (int tid = 0; tid < nthr; ++tid) bw_sg_step<T, KW, NSG, 0, 0, false>(p, st[tid], j, stack, smX.data(), smG.data(), R, tid, nthr);
         for (int tid = 0; tid < nthr; ++tid)
-          tile_store_auto<T>(p.gout, p.gout_sB, p.gout_sS, p.gout_cols, re, stack, row0, R, p.panel, pbase, p.vec_o != 0, smG.data(), tid, nthr);
+          tile_store_v<T>(p.gout, p.gout_sB, p.gout_sS, p.gout_cols, bw_row_limit(p, re), stack, row0, R, p.panel, pbase, p.vec_o != 0, p.log_n, p.vr, smG.data(), tid, nthr);
       }
       for (int tid = 0; tid < nthr; ++tid) bw_flush_state<T, KW, NSG>(p, st[tid], stack, pbase, tid, nthr);
     }
@@ -272,6 +284,23 @@ struct EmulExec {
   int add_bias(float* out, const float* bias, int64_t B, int len, int64_t pitch) {
     for (int64_t b = 0; b < B; ++b)
       for (int f = 0; f < len; ++f) out[b * pitch + f] += bias[f];
+    return BFLY_OK;
+  }
+  static constexpr bool kFusedBias = true;  // run_fw adds FwParams::bias
+  // layers: the sums of the small kernels
+  template <typename T> int column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out) {
+    for (int c = 0; c < cols; ++c) out[c] = Ops<T>::zero();
+    for (int64_t b = 0; b < B; ++b)
+      for (int c = 0; c < cols; ++c) out[c] = add1(out[c], g[b * pitch + c]);
+    return BFLY_OK;
+  }
+  template <typename T> int stack_sums(const T* g, int64_t B, int S, int64_t n, int cols, T* out) {
+    for (int64_t b = 0; b < B; ++b)
+      for (int c = 0; c < cols; ++c) {
+        T acc = Ops<T>::zero();
+        for (int s = 0; s < S; ++s) acc = add1(acc, g[(b * S + s) * n + c]);
+        out[b * cols + c] = acc;
+      }
     return BFLY_OK;
   }
   int zero(void* ptr, size_t bytes) { std::memset(ptr, 0, bytes); return BFLY_OK; }
@@ -458,6 +487,40 @@ int bfly_emul_fw_glue(int dtype, const void* tw, const void* x, int x_is_real, i
   if (x_is_real) g.x_real = (const float*)x;
   if (out_is_real) g.out_real = (float*)out;
   return drive_fw_glue<cf>(ex, q, (const cf*)tw, x_is_real ? nullptr : (const cf*)x, x_sB, x_sS, out_is_real ? nullptr : (cf*)out, g);
+}
+// A whole layer: the forward (with the snapshots of the backward when `save`), then the backward that starts from them
+// or recomputes.  dtype 0 float32, 1 complex64; tw2 / tw4 and their gradients as in bfly_emul_fw.
+}
+template <typename T>
+static int emul_layer(const void* tw2, const void* tw4, const void* x, int64_t x_sB, const void* bias, void* out, const void* g, int64_t g_sB,
+                      void* d2, void* d4, void* d_in, void* d_bias, Problem q, int out_total, int save, int threads, int sms) {
+  EmulExec ex; ex.threads_ = threads; ex.sms = sms;
+  BwLayout<T> lay;
+  int rc = check_problem(q);
+  if (rc) return rc;
+  rc = plan_bw<T>(q, lay);
+  if (rc) return rc;
+  auto aligned = [](std::vector<char>& v) { return (void*)(((uintptr_t)v.data() + 255) / 256 * 256); };
+  const size_t keep = save && !lay.chunked ? lay.ws_bytes : 0;
+  std::vector<char> snaps(keep + 256), fws(fw_workspace_bytes<T>(q) + 256);
+  void* sp = keep ? aligned(snaps) : nullptr;
+  rc = drive_layer_fw<T>(ex, q, (const T*)tw2, (const T*)tw4, (const T*)x, x_sB, (T*)out, (const T*)bias, out_total, sp, keep,
+                         sp ? nullptr : aligned(fws), sp ? 0 : fw_workspace_bytes<T>(q));
+  if (rc) return rc;
+  LayerBwLayout L;
+  rc = plan_layer_bw<T>(q, out_total, sp != nullptr, L);
+  if (rc) return rc;
+  std::vector<char> ws(L.ws_bytes + 256);
+  return drive_layer_bw<T>(ex, q, (const T*)tw2, (const T*)tw4, (const T*)x, x_sB, (const T*)g, g_sB, (T*)d2, (T*)d4, (T*)d_in, (T*)d_bias,
+                           out_total, sp, keep, L.ws_bytes ? aligned(ws) : nullptr, L.ws_bytes);
+}
+extern "C" {
+int bfly_emul_layer(int dtype, int base4, const void* tw2, const void* tw4, const void* x, int64_t x_sB, const void* bias, void* out,
+                    const void* g, int64_t g_sB, void* d2, void* d4, void* d_in, void* d_bias, int B, int S, int log_n, int nblocks,
+                    int in_size, int out_total, int inc, int save, int threads, int sms) {
+  Problem q{B, S, log_n, nblocks, in_size, 1 << (log_n & 31), inc != 0, base4 != 0};
+  return dtype == 0 ? emul_layer<float>(tw2, tw4, x, x_sB, bias, out, g, g_sB, d2, d4, d_in, d_bias, q, out_total, save, threads, sms)
+                    : emul_layer<cf>(tw2, tw4, x, x_sB, bias, out, g, g_sB, d2, d4, d_in, d_bias, q, out_total, save, threads, sms);
 }
 // number of backward phases and workspace bytes the planner chooses (for tests of the planner)
 int bfly_emul_bw_plan(int dtype, int base4, int B, int S, int log_n, int nblocks, int inc, int64_t* ws_bytes) {

@@ -487,3 +487,122 @@ def test_packed_pair_forward_on_wide_rows(emul, oracle_mod):
     y = emul_fw(emul, tw, None, x, True, n, 13, 1, False, 256)
     assert emul.bfly_emul_fw2_calls() == calls
     assert rel_err(y, oracle_mod.multiply_fw(tw, x, True, n)) < 2e-5
+
+
+@pytest.mark.parametrize("cplx,base4,log_n,S,nblocks,cut,extra", [
+    (0, 0, 2, 1, 2, 0, 1), (0, 0, 5, 2, 1, 0, 3), (0, 0, 6, 1, 2, 0, 5), (0, 0, 8, 1, 1, 3, 1), (0, 0, 9, 1, 2, 64, 1),
+    (0, 1, 6, 1, 1, 0, 5), (0, 1, 7, 2, 1, 1, 3), (0, 1, 10, 1, 1, 32, 3), (1, 0, 3, 1, 1, 0, 7), (1, 0, 8, 2, 1, 3, 5)])
+def test_several_rows_to_a_tile_row(emul, oracle_mod, cplx, base4, log_n, S, nblocks, cut, extra):
+    """Narrow rows of 2^21 values and more share a tile row.  A batch that does not fill the last one, cut and unaligned
+    widths: against the oracle, and outputs and input gradients bit by bit against the same product row by row."""
+    torch.manual_seed(log_n)
+    n, dt = 1 << log_n, torch.complex64 if cplx else torch.float32
+    B = (1 << 21) // n + extra
+    tw2 = torch.randn(S, nblocks, log_n % 2 if base4 else log_n, n // 2, 2, 2, dtype=dt) / 2 ** 0.5
+    tw4 = torch.randn(S, nblocks, log_n // 2, n // 4, 4, 4, dtype=dt) / 2 if base4 else None
+    x, g = torch.randn(B, S, n - cut, dtype=dt), torch.randn(B, S, n - cut // 2, dtype=dt)
+    run = lambda: (emul_fw(emul, tw2, tw4, x, True, g.shape[2], log_n, nblocks, base4, 256),
+                   *emul_bw(emul, tw2, tw4, x, g, True, log_n, nblocks, base4, 256))
+    y, d2, d4, dx = run()
+    with emul_option(emul, "virtual_rows", 0):
+        ys, _, _, dxs = run()
+    assert torch.equal(y, ys) and torch.equal(dx, dxs)
+    wide = torch.complex128 if cplx else torch.float64
+    w = lambda t: t.to(wide)
+    if base4:
+        d4r, d2r, dxr = oracle_mod.base4_bw(w(tw4), w(tw2), w(x), w(g), True)
+        yr = oracle_mod.base4_fw(w(tw4), w(tw2), w(x), True, g.shape[2])
+    else:
+        (d2r, dxr), d4r = oracle_mod.multiply_bw(w(tw2), w(x), w(g), True), None
+        yr = oracle_mod.multiply_fw(w(tw2), w(x), True, g.shape[2])
+    assert rel_err(y, yr.to(dt)) < 2e-5 and rel_err(dx, dxr.to(dt)) < 2e-5
+    for a, b in ((d2, d2r), (d4, d4r)):  # sums over up to 2^19 rows: the emulator adds them one by one, 2^-24 * sqrt(rows) each way
+        assert a is None or not a.numel() or rel_err(a, b.to(dt)) < 1e-4
+
+
+@pytest.mark.parametrize("cplx,log_n,S", [(1, 2, 1), (1, 5, 2), (1, 8, 1), (0, 6, 2), (0, 9, 1)])
+def test_glue_of_rows_that_share_a_tile_row(emul, oracle_mod, cplx, log_n, S):
+    torch.manual_seed(50 + log_n)
+    n, dt = 1 << log_n, torch.complex64 if cplx else torch.float32
+    B = (1 << 21) // n + 3
+    tw = torch.randn(S, 1, log_n, n // 2, 2, 2, dtype=dt) / 2 ** 0.5
+    for combo in (1, 2, 4, 6, 7, 15) if cplx else (1, 4, 7):
+        real_io = bool(combo & 8)
+        x = torch.randn(B, S, n, dtype=torch.float32 if real_io else dt)
+        in_perm, out_perm = (torch.randperm(n, dtype=torch.int32) if combo & bit else None for bit in (1, 2))
+        diag = torch.randn(n, dtype=dt) if combo & 4 else None
+        out = torch.full((B, S, n), float("nan"), dtype=x.dtype)
+        rc = emul.bfly_emul_fw_glue(int(cplx), P(tw), P(x), int(real_io), I64(x.stride(0)), I64(x.stride(1)), P(out), int(real_io),
+                                    P(in_perm), P(diag), P(out_perm), B, S, log_n, 1, n, n, 1, 256)
+        assert rc == 0
+        want = _glue_reference(oracle_mod, tw, x, True, in_perm, diag, out_perm, real_io)
+        assert_rtol_atol(out, want, "glue of narrow rows n=%d combo=%d" % (n, combo), rtol=1e-4, atol=1e-4)
+
+
+def test_glue_of_padded_rows(emul, oracle_mod):
+    """Rows narrower than n enter padded where nothing gathers them (circulants of any length), real and complex, with a
+    diagonal and a gather behind the product, at widths with and without 16-byte rows."""
+    torch.manual_seed(60)
+    for log_n, B in ((5, 9), (9, 7), (11, 4), (6, (1 << 21) // 64 + 3)):
+        n = 1 << log_n
+        tw = torch.randn(1, 1, log_n, n // 2, 2, 2, dtype=torch.complex64) / 2 ** 0.5
+        for width, real_in, use_diag, use_perm, real_out in ((n // 2 + 1, 1, 1, 0, 0), (n // 2 + 4, 1, 1, 0, 0), (n - 7, 0, 0, 1, 0), (n - 3, 1, 0, 0, 1),
+                                                             (n - 2, 0, 1, 0, 1)):
+            x = torch.randn(B, 1, width, dtype=torch.float32 if real_in else torch.complex64)
+            diag = torch.randn(n, dtype=torch.complex64) if use_diag else None
+            perm = torch.randperm(n, dtype=torch.int32) if use_perm else None
+            out = torch.full((B, 1, n), float("nan"), dtype=torch.float32 if real_out else torch.complex64)
+            rc = emul.bfly_emul_fw_glue(1, P(tw), P(x), real_in, I64(x.stride(0)), I64(x.stride(1)), P(out), real_out, None, P(diag), P(perm),
+                                        B, 1, log_n, 1, width, n, 1, 256)
+            assert rc == 0
+            xp = torch.zeros(B, 1, n, dtype=torch.complex64)
+            xp[..., :width] = x
+            want = _glue_reference(oracle_mod, tw, xp, True, None, diag, perm, bool(real_out))
+            assert_rtol_atol(out, want, "glue of padded rows n=%d width=%d" % (n, width), rtol=1e-4, atol=1e-4)
+
+
+def emul_layer(lib, kind, tws, x, bias, g, S, log_n, nblocks, inc, save, threads=256, sms=7):
+    """Output, d_input, d_bias and twiddle gradients of a layer through the driver's layer calls."""
+    base4, B, n = kind == "base4", x.shape[0], 1 << log_n
+    tw4, tw2 = tws if base4 else (None, tws[0])
+    out = torch.full((B, S * n), float("nan"), dtype=x.dtype)
+    d4, d2 = (None if t is None else torch.full_like(t, float("nan")) for t in (tw4, tw2))
+    d_in = torch.full((B, x.shape[1] if S > 1 else max(x.shape[1], n)), float("nan"), dtype=x.dtype)
+    d_b = None if bias is None else torch.full_like(bias, float("nan"))
+    rc = lib.bfly_emul_layer(int(x.is_complex()), int(base4), P(tw2), P(tw4), P(x), I64(x.stride(0)), P(bias), P(out), P(g), I64(g.stride(0)),
+                             P(d2), P(d4), P(d_in), P(d_b), B, S, log_n, nblocks, x.shape[1], g.shape[1], int(inc), int(save), threads, sms)
+    return rc, out[:, :g.shape[1]], d_in[:, :x.shape[1]], d_b, [d4, d2] if base4 else [d2]
+
+
+@pytest.mark.parametrize("save", [0, 1])
+@pytest.mark.parametrize("kind,in_size,S,out_size,nblocks,B", [
+    ("f32", 1000, 3, 3000, 1, 37), ("f32", 1024, 2, 2048, 2, 60), ("f32", 1023, 2, 1025, 2, 1), ("f32", 5, 1, 2, 1, 1), ("f32", 96, 1, 100, 2, 21),
+    ("f32", 8000, 1, 8192, 1, 3), ("f32", 70, 2, 200, 1, (1 << 21) // 128 + 3), ("f32", 64, 2, 128, 1, (1 << 21) // 64 + 3),
+    ("c64", 1000, 2, 1500, 2, 9), ("c64", 100, 1, 120, 1, (1 << 21) // 128 + 5), ("base4", 500, 1, 512, 2, 11), ("base4", 1024, 2, 2000, 1, 7),
+    ("base4", 100, 1, 120, 1, (1 << 21) // 128 + 5)])
+def test_layers(emul, oracle_mod, kind, in_size, S, out_size, nblocks, B, save):
+    """A whole layer: padded input shared by the stacks, cut last stack read as one matrix, bias on the tile, input
+    gradient summed over the stacks, with and without the forward's snapshots, rows that share a tile row."""
+    torch.manual_seed(in_size + nblocks)
+    log_n = max(1, (in_size - 1).bit_length())
+    n, dt = 1 << log_n, torch.complex64 if kind == "c64" else torch.float32
+    wide = torch.complex128 if kind == "c64" else torch.float64
+    x, g, bias = torch.randn(B, in_size, dtype=dt), torch.randn(B, out_size, dtype=dt), torch.randn(out_size, dtype=dt)
+    xe = x.to(wide).unsqueeze(1).expand(B, S, in_size).contiguous()
+    gp = torch.zeros(B, S * n, dtype=wide)
+    gp[:, :out_size] = g
+    if kind == "base4":
+        tws = [torch.randn(S, nblocks, log_n // 2, n // 4, 4, 4) / 2, torch.randn(S, nblocks, log_n % 2, n // 2, 2, 2) / 2 ** 0.5]
+        y = oracle_mod.base4_fw(*[t.to(wide) for t in tws], xe, True)
+        d4, d2, dx = oracle_mod.base4_bw(*[t.to(wide) for t in tws], xe, gp.view(B, S, n), True)
+        dtw = [d4, d2]
+    else:
+        tws = [torch.randn(S, nblocks, log_n, n // 2, 2, 2, dtype=dt) / 2 ** 0.5]
+        y = oracle_mod.multiply_fw(tws[0].to(wide), xe, True)
+        d, dx = oracle_mod.multiply_bw(tws[0].to(wide), xe, gp.view(B, S, n), True)
+        dtw = [d]
+    want = [y.reshape(B, S * n)[:, :out_size] + bias, dx.sum(1), g.to(wide).sum(0)] + dtw
+    rc, out, d_in, d_b, d_tw = emul_layer(emul, kind, tws, x, bias, g, S, log_n, nblocks, True, save)
+    assert rc == 0
+    for got, ref, what in zip([out, d_in, d_b] + d_tw, want, ("output", "d_input", "d_bias", "d_twiddle", "d_twiddle2")):
+        assert got.shape == ref.shape and (not got.numel() or rel_err(got, ref.to(dt)) < (2e-5 if B < 1000 else 1e-4)), what
