@@ -175,6 +175,13 @@ inline int check_problem(const Problem& q) {
   return BFLY_OK;
 }
 
+// Is a twiddle tensor missing that the product reads?  (Radix 4: twiddle2 holds the odd factor of each block, if there is one.)
+template <typename T> inline bool twiddle_missing(const Problem& q, const T* tw2, const T* tw4) {
+  int64_t per_stack[2];
+  twiddle_stack_sizes(q, per_stack);
+  return (per_stack[0] && !tw2) || (per_stack[1] && !tw4);
+}
+
 inline std::vector<Stage> problem_stages(const Problem& q) {
   return q.base4 ? make_stages_r4(q.log_n, q.nblocks, q.inc) : make_stages_r2(q.log_n, q.nblocks, q.inc);
 }
@@ -490,7 +497,7 @@ int drive_fw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T* x, in
   int rc = check_problem(q);
   if (rc != BFLY_OK) return rc;
   if (q.B == 0) return BFLY_OK;
-  if (!x || !out || (!tw2 && !tw4)) return BFLY_E_ARG;
+  if (!x || !out || twiddle_missing(q, tw2, tw4)) return BFLY_E_ARG;
   if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4))) return BFLY_E_ALIGN;
   const std::vector<Stage> st = problem_stages(q);
   const int64_t n = (int64_t)1 << q.log_n;
@@ -571,7 +578,7 @@ int drive_fw_saving(E& ex, const Problem& q, const T* tw2, const T* tw4, const T
   int rc = check_problem(q);
   if (rc != BFLY_OK) return rc;
   if (q.B == 0) return BFLY_OK;
-  if (!x || !out || (!tw2 && !tw4)) return BFLY_E_ARG;
+  if (!x || !out || twiddle_missing(q, tw2, tw4)) return BFLY_E_ARG;
   if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4))) return BFLY_E_ALIGN;
   BwLayout<T> lay;
   rc = plan_bw<T>(q, lay);
@@ -765,7 +772,7 @@ int drive_layer_fw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T*
   if (rc != BFLY_OK) return rc;
   if (out_total < 0 || out_total > ((int64_t)q.S << q.log_n)) return BFLY_E_ARG;
   if (q.B == 0) return BFLY_OK;
-  if (!x || !out || (!tw2 && !tw4)) return BFLY_E_ARG;
+  if (!x || !out || twiddle_missing(q, tw2, tw4)) return BFLY_E_ARG;
   if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4))) return BFLY_E_ALIGN;
   const std::vector<Stage> st = problem_stages(q);
   const int64_t n = (int64_t)1 << q.log_n;
@@ -949,10 +956,19 @@ int drive_layer_bw(E& ex, const Problem& q_in, const T* tw2, const T* tw4, const
   if (rc != BFLY_OK) return rc;
   const int64_t n = (int64_t)1 << q.log_n, DX = std::max<int64_t>(q.in_size, n);
   if (out_total < 0 || out_total > q.S * n) return BFLY_E_ARG;
+  if (q.B > 0 && (!x || !d_in || (out_total > 0 && !grad))) return BFLY_E_ARG;
   LayerBwLayout L;
   rc = plan_layer_bw<T>(q, out_total, saved != nullptr, L);
   if (rc != BFLY_OK) return rc;
   if (ws_bytes < L.ws_bytes || (L.ws_bytes > 0 && (!ws || !aligned16(ws)))) return BFLY_E_WORKSPACE;
+  if (out_total == 0) {  // no output, no gradient: a (B, 0) matrix has no column to read
+    int64_t stk[2];
+    twiddle_stack_sizes(q, stk);
+    if ((stk[0] && !d_tw2) || (stk[1] && !d_tw4)) return BFLY_E_ARG;
+    if (stk[0] && (rc = ex.zero(d_tw2, (size_t)q.S * stk[0] * sizeof(T)))) return rc;
+    if (stk[1] && (rc = ex.zero(d_tw4, (size_t)q.S * stk[1] * sizeof(T)))) return rc;
+    return q.B > 0 ? ex.zero(d_in, (size_t)q.B * (q.S > 1 ? q.in_size : DX) * sizeof(T)) : BFLY_OK;
+  }
   if constexpr (sizeof(T) == 4) {
     if (L.fused_bytes) {
       rc = drive_linear_bw(ex, q, tw2, x, x_sB, grad, g_sB, d_tw2, d_in, q.S > 1 ? (int64_t)q.in_size : DX, d_bias, out_total, ws,
@@ -968,7 +984,7 @@ int drive_layer_bw(E& ex, const Problem& q_in, const T* tw2, const T* tw4, const
   const bool ready = saved && !lay.chunked;
   void* planes = ready ? saved : ws;
   rc = drive_bw<T>(ex, q, tw2, tw4, x, x_sB, 0, grad, g_sB, n, d_tw2, d_tw4, dx, lay.ws_bytes ? planes : nullptr, lay.ws_bytes, ready,
-                   out_total == q.S * n ? 0 : std::max(out_total, 1));
+                   out_total == q.S * n ? 0 : out_total);
   if (rc != BFLY_OK) return rc;
   if (q.S > 1) {
     rc = ex.stack_sums(dx, q.B, q.S, DX, q.in_size, d_in);

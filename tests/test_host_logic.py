@@ -606,3 +606,29 @@ def test_layers(emul, oracle_mod, kind, in_size, S, out_size, nblocks, B, save):
     assert rc == 0
     for got, ref, what in zip([out, d_in, d_b] + d_tw, want, ("output", "d_input", "d_bias", "d_twiddle", "d_twiddle2")):
         assert got.shape == ref.shape and (not got.numel() or rel_err(got, ref.to(dt)) < (2e-5 if B < 1000 else 1e-4)), what
+
+
+def test_missing_tensors_are_refused(emul):
+    """A NULL where the kernels would read or write is an argument error: the odd factors' twiddle2 of a radix-4 product,
+    and every tensor of a layer's backward."""
+    n, log_n = 32, 5
+    tw4, tw2 = torch.randn(1, 1, 2, 8, 4, 4), torch.randn(1, 1, 1, 16, 2, 2)
+    x, out = torch.randn(3, 1, n), torch.empty(3, 1, n)
+    fw = lambda a, b: emul.bfly_emul_fw(0, 1, P(a), P(b), P(x), I64(n), I64(n), P(out), 3, 1, log_n, 1, n, n, 1, 64)
+    assert fw(tw2, tw4) == 0 and fw(None, tw4) == -1 and fw(tw2, None) == -1
+    tw = torch.randn(2, 1, log_n, 16, 2, 2)
+    x, g, bias = torch.randn(3, n), torch.randn(3, 50), torch.randn(50)
+    full = dict(d2=torch.empty_like(tw), d_in=torch.empty(3, n), x=x, g=g, out=torch.empty(3, 2 * n))
+    for missing in (None, "d_in", "g", "d2", "x", "out"):
+        t = {k: None if k == missing else v for k, v in full.items()}
+        rc = emul.bfly_emul_layer(0, 0, P(tw), None, P(t["x"]), I64(n), P(bias), P(t["out"]), P(t["g"]), I64(50), P(t["d2"]), None, P(t["d_in"]),
+                                  None, 3, 2, log_n, 1, n, 50, 1, 0, 64, 7)
+        assert rc == (-1 if missing else 0), missing
+
+
+@pytest.mark.parametrize("S", [1, 2])
+def test_layer_without_output_columns(emul, S):
+    """out_size 0: the gradient matrix has no column, and every gradient is zero."""
+    tw, x, g = torch.randn(S, 1, 5, 16, 2, 2), torch.randn(4, 30), torch.full((4, 0), float("nan"))
+    rc, out, d_in, _, (d_tw,) = emul_layer(emul, "f32", [tw], x, None, g, S, 5, 1, True, 0)
+    assert rc == 0 and out.shape == (4, 0) and (d_in == 0).all() and (d_tw == 0).all()
