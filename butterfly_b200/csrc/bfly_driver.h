@@ -152,6 +152,9 @@ inline bool fw2_enabled() {
   return o.fw2 != 0 && o.tma != 0 && o.fw_logcmax < 0 && o.fw_kmax < 0 && o.fw_rows < 0;
 }
 
+// Rows move element by element with one access each where 16-byte accesses do not apply (tile_copy_in): a row tensor
+// starts on a whole element, 8 bytes for complex64.
+template <typename T> inline bool rows_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & (sizeof(T) - 1)) == 0; }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 template <typename T> inline bool vec_ok(const void* p, int64_t sB, int64_t sS) {
   return aligned16(p) && (sB * (int64_t)sizeof(T)) % 16 == 0 && (sS * (int64_t)sizeof(T)) % 16 == 0;
@@ -499,6 +502,7 @@ int drive_fw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T* x, in
   if (q.B == 0) return BFLY_OK;
   if (!x || !out || twiddle_missing(q, tw2, tw4)) return BFLY_E_ARG;
   if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4))) return BFLY_E_ALIGN;
+  if (!rows_aligned<T>(x) || !rows_aligned<T>(out)) return BFLY_E_ALIGN;
   const std::vector<Stage> st = problem_stages(q);
   const int64_t n = (int64_t)1 << q.log_n;
   if (ws && !aligned16(ws)) ws = nullptr;  // optional scratch: without it the generic kernel runs
@@ -519,7 +523,8 @@ int drive_fw_glue(E& ex, const Problem& q, const T* tw2, const T* x, int64_t x_s
   if (q.B == 0) return BFLY_OK;
   if ((!x && !glue.x_real) || (!out && !glue.out_real) || !tw2) return BFLY_E_ARG;
   if ((x && glue.x_real) || (out && glue.out_real)) return BFLY_E_ARG;
-  if (!aligned16(tw2)) return BFLY_E_ALIGN;
+  if (!aligned16(tw2) || !rows_aligned<T>(x) || !rows_aligned<T>(out) || !rows_aligned<float>(glue.x_real) || !rows_aligned<float>(glue.out_real))
+    return BFLY_E_ALIGN;
   if (glue.in_perm && q.in_size != (1 << q.log_n)) return BFLY_E_ARG;  // the gather addresses whole rows
   if ((glue.out_perm || glue.out_diag) && q.out_size != (1 << q.log_n)) return BFLY_E_ARG;
   const std::vector<Stage> st = problem_stages(q);
@@ -580,6 +585,7 @@ int drive_fw_saving(E& ex, const Problem& q, const T* tw2, const T* tw4, const T
   if (q.B == 0) return BFLY_OK;
   if (!x || !out || twiddle_missing(q, tw2, tw4)) return BFLY_E_ARG;
   if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4))) return BFLY_E_ALIGN;
+  if (!rows_aligned<T>(x) || !rows_aligned<T>(out)) return BFLY_E_ALIGN;
   BwLayout<T> lay;
   rc = plan_bw<T>(q, lay);
   if (rc != BFLY_OK) return rc;
@@ -619,6 +625,7 @@ int drive_bw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T* x, in
   if (stk[1]) { rc = ex.zero(d_tw4, (size_t)q.S * stk[1] * sizeof(T)); if (rc) return rc; }
   if (q.B == 0) return BFLY_OK;
   if (!x || !grad || !d_x) return BFLY_E_ARG;
+  if (!rows_aligned<T>(x) || !rows_aligned<T>(grad) || !rows_aligned<T>(d_x)) return BFLY_E_ALIGN;
   BwLayout<T> lay;
   rc = plan_bw<T>(q, lay);
   if (rc != BFLY_OK) return rc;
@@ -774,6 +781,7 @@ int drive_layer_fw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T*
   if (q.B == 0) return BFLY_OK;
   if (!x || !out || twiddle_missing(q, tw2, tw4)) return BFLY_E_ARG;
   if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4))) return BFLY_E_ALIGN;
+  if (!rows_aligned<T>(x) || !rows_aligned<T>(out)) return BFLY_E_ALIGN;
   const std::vector<Stage> st = problem_stages(q);
   const int64_t n = (int64_t)1 << q.log_n;
   if (ws && !aligned16(ws)) ws = nullptr;
@@ -957,6 +965,7 @@ int drive_layer_bw(E& ex, const Problem& q_in, const T* tw2, const T* tw4, const
   const int64_t n = (int64_t)1 << q.log_n, DX = std::max<int64_t>(q.in_size, n);
   if (out_total < 0 || out_total > q.S * n) return BFLY_E_ARG;
   if (q.B > 0 && (!x || !d_in || (out_total > 0 && !grad))) return BFLY_E_ARG;
+  if (!rows_aligned<T>(x) || !rows_aligned<T>(grad) || !rows_aligned<T>(d_in)) return BFLY_E_ALIGN;
   LayerBwLayout L;
   rc = plan_layer_bw<T>(q, out_total, saved != nullptr, L);
   if (rc != BFLY_OK) return rc;

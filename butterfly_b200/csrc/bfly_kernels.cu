@@ -896,7 +896,7 @@ const char* bfly_strerror(int status) {
     case BFLY_OK: return "success";
     case BFLY_E_ARG: return "invalid argument (sizes inconsistent or null pointer)";
     case BFLY_E_UNSUPPORTED: return "shape not supported by the B200 butterfly kernels";
-    case BFLY_E_ALIGN: return "twiddle pointer must be 16-byte aligned";
+    case BFLY_E_ALIGN: return "misaligned pointer (twiddles: 16 bytes; rows: one element, 8 bytes for complex64)";
     case BFLY_E_WORKSPACE: return "workspace missing, misaligned or too small";
     case BFLY_E_CUDA: return "CUDA runtime call or kernel launch failed";
     case BFLY_E_NODEVICE: return "no usable CUDA device";

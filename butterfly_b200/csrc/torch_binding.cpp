@@ -41,8 +41,16 @@ int dtype_code(const Tensor& t, const char* what) {
 
 // Borrowed tensors are never mutated; lazily-conjugated or strided views are materialised.
 Tensor dense_twiddle(const Tensor& t) { return t.resolve_conj().contiguous(); }
+// The kernels take complex rows from 8-byte boundaries (bfly.h).  Tensors over foreign memory may start in between; they
+// are copied as floats (PyTorch's own complex copies assume the alignment too).
+Tensor on_element(const Tensor& t) {
+  if (!t.numel() || reinterpret_cast<uintptr_t>(t.const_data_ptr()) % t.element_size() == 0) return t;
+  const bool conj = t.is_conj();
+  Tensor r = at::view_as_complex(at::view_as_real(conj ? t.conj() : t).clone(at::MemoryFormat::Contiguous));
+  return conj ? r.conj() : r;
+}
 Tensor rows_view(const Tensor& t) {
-  Tensor r = t.resolve_conj();
+  Tensor r = on_element(t).resolve_conj();
   if (r.size(2) > 1 && r.stride(2) != 1) r = r.contiguous();
   if (r.size(2) <= 1 && r.stride(2) != 1) r = r.contiguous();
   return r;
@@ -249,7 +257,8 @@ struct LayerCall {
 };
 
 Tensor rows_2d(const Tensor& t) {
-  Tensor r = t.dim() == 2 ? t : t.reshape({-1, t.size(-1)});
+  Tensor r = on_element(t);
+  if (r.dim() != 2) r = r.reshape({-1, r.size(-1)});
   r = r.resolve_conj();
   return r.stride(1) == 1 ? r : r.contiguous();
 }

@@ -26,6 +26,8 @@
  *   d_twiddle (d_twiddle4, d_twiddle2): like the twiddle they belong to, 16-byte aligned
  *   d_x       (batch, nstacks, max(input_size, n)) contiguous; columns < input_size
  *             hold the input gradient (columns >= n of them are zero)
+ * Row tensors (x, out, grad, d_x, d_input) start on a whole element: 8 bytes for complex64 (BFLY_E_ALIGN otherwise).
+ * Rows of 16-byte aligned pitch move fastest.
  * Input columns >= n are ignored, missing ones (input_size < n) read as zero, exactly as
  * the reference pads (csrc/cpu/butterfly_cpu.cpp:47-49, csrc/cuda/butterfly_cuda.cu:148-149).
  */
@@ -42,7 +44,7 @@ extern "C" {
 #define BFLY_OK 0
 #define BFLY_E_ARG (-1)          /* inconsistent sizes or a null pointer */
 #define BFLY_E_UNSUPPORTED (-2)  /* shape outside what the kernels cover */
-#define BFLY_E_ALIGN (-3)        /* twiddle or d_twiddle pointer not 16-byte aligned */
+#define BFLY_E_ALIGN (-3)        /* twiddle or d_twiddle not 16-byte aligned, or rows not aligned to their element */
 #define BFLY_E_WORKSPACE (-4)    /* workspace missing, misaligned or too small */
 #define BFLY_E_CUDA (-5)         /* a CUDA runtime call or launch failed */
 #define BFLY_E_NODEVICE (-6)     /* no usable CUDA device */

@@ -632,3 +632,24 @@ def test_layer_without_output_columns(emul, S):
     tw, x, g = torch.randn(S, 1, 5, 16, 2, 2), torch.randn(4, 30), torch.full((4, 0), float("nan"))
     rc, out, d_in, _, (d_tw,) = emul_layer(emul, "f32", [tw], x, None, g, S, 5, 1, True, 0)
     assert rc == 0 and out.shape == (4, 0) and (d_in == 0).all() and (d_tw == 0).all()
+
+
+def test_rows_between_elements_are_refused(emul):
+    """Rows that cannot move in 16-byte accesses move one element at a time, complex ones 8 bytes: every complex row tensor
+    that starts four bytes off is refused."""
+    n, log_n, c64 = 8, 3, torch.complex64
+    tw = torch.randn(1, 1, log_n, n // 2, 2, 2, dtype=c64)
+    off = lambda t, by: ctypes.c_void_p(t.data_ptr() + by)
+    for which in ("none", "x", "out", "g", "dx"):
+        t = {k: torch.zeros(3, 1, n + 1, dtype=c64) for k in ("x", "out", "g", "dx")}
+        p = {k: off(v, 4 if k == which else 0) for k, v in t.items()}
+        d_tw = torch.empty_like(tw)
+        s = (I64(n), I64(n))
+        fw = emul.bfly_emul_fw(1, 0, P(tw), None, p["x"], *s, p["out"], 3, 1, log_n, 1, n, n, 1, 64)
+        bw = emul.bfly_emul_bw(1, 0, P(tw), None, p["x"], *s, p["g"], *s, P(d_tw), None, p["dx"], 3, 1, log_n, 1, n, n, 1, 64, 7)
+        both = emul.bfly_emul_fw_bw_saved(1, P(tw), p["x"], *s, p["out"], p["g"], *s, P(d_tw), p["dx"], 3, 1, log_n, 1, n, n, 1, 64, 7)
+        layer = emul.bfly_emul_layer(1, 0, P(tw), None, p["x"], I64(n), None, p["out"], p["g"], I64(n), P(d_tw), None, p["dx"], None, 3, 1, log_n, 1,
+                                     n, n, 1, 0, 64, 7)
+        glue = emul.bfly_emul_fw_glue(1, P(tw), p["x"], 0, *s, p["out"], 0, None, None, None, 3, 1, log_n, 1, n, n, 1, 64)
+        bad = lambda *names: -3 if which in names else 0
+        assert (fw, bw, both, layer, glue) == (bad("x", "out"), bad("x", "g", "dx"), bad(*p), bad(*p), bad("x", "out")), which

@@ -613,3 +613,32 @@ def test_operators_capture_into_a_cuda_graph(dev, oracle_mod):
         yr = oracle_mod.multiply_fw(tw.cpu(), x.cpu(), True)
         dtr, dxr = oracle_mod.multiply_bw(tw.cpu(), x.cpu(), g.cpu(), True)
         assert rel_err(y, yr) < TOL and rel_err(d_x, dxr) < TOL and rel_err(d_tw, dtr) < TOL
+
+
+def test_complex_rows_between_elements(dev):
+    """Complex tensors over foreign memory that start four bytes off an element (a kernel element copy would be misaligned):
+    the operators work on an aligned copy."""
+    import butterfly_b200 as bb
+    torch.manual_seed(6)
+
+    class Foreign:  # the CUDA array interface takes any address
+        def __init__(self, owner, shape):
+            self.owner = owner
+            self.__cuda_array_interface__ = dict(shape=shape, typestr="<c8", data=(owner.data_ptr() + 4, False), strides=None, version=3)
+
+    def pair(*shape):
+        count = 2
+        for s in shape:
+            count *= s
+        floats = torch.randn(count + 1, device=dev)
+        return torch.as_tensor(Foreign(floats, shape), device=dev), torch.view_as_complex(floats[1:].clone().view(*shape, 2)), floats
+    x, xa, _keep_x = pair(9, 1, 61)
+    g, ga, _keep_g = pair(9, 1, 64)
+    assert x.data_ptr() % 8 == 4
+    tw = torch.randn(1, 1, 6, 32, 2, 2, dtype=torch.complex64, device=dev)
+    assert torch.equal(bb.butterfly_multiply_fw(tw, x, True), bb.butterfly_multiply_fw(tw, xa, True))
+    for a, b in zip(bb.butterfly_multiply_bw(tw, x, g, True), bb.butterfly_multiply_bw(tw, xa, ga, True)):
+        assert (a - b).abs().max() < 1e-5 * b.abs().max()
+    layer = bb.Butterfly(61, 64, complex=True).to(dev)
+    with torch.no_grad():
+        assert torch.equal(layer(x), layer(xa)) and torch.equal(layer(x.conj()), layer(xa.conj()))
