@@ -16,7 +16,7 @@
 //   int  zero2d(void* ptr, size_t pitch_bytes, size_t width_bytes, size_t rows);
 //   int  add_bias(float* out, const float* bias, int64_t B, int len, int64_t pitch);   // out[b, f] += bias[f], f < len
 //   static constexpr bool kFusedBias;                      // optional: run_fw adds FwParams::bias itself
-//   int  column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out);           // layers: bias gradient
+//   int  column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out, float* partial);   // layers: bias gradient
 //   int  stack_sums(const T* g, int64_t B, int S, int64_t n, int cols, T* out);         // layers: sum over the stacks
 #pragma once
 #include <cstdlib>
@@ -934,8 +934,24 @@ int drive_linear_bw(E& ex, const Problem& q, const float* tw, const float* x, in
 // input with the gradient read as one (B, out_total) matrix, sums the stacks in one pass and the bias in another.
 struct LayerBwLayout {
   size_t fused_bytes;                 // 0: the fused route does not apply
-  size_t planes_off, dx_off, ws_bytes;  // unfused: snapshots when not saved, then the stacks' input gradients
+  size_t planes_off, dx_off, sums_off, ws_bytes;  // unfused: snapshots when not saved, the stacks' input gradients, partial bias gradients
 };
+
+// Row slices of a column sum over a (B, cols) float matrix: up to 2048 rows one slice, which writes the sums (a second
+// launch costs about 2 us: 2047 rows of 3000 columns 8.6 us this way, 11 in twelve slices); more rows in slices of 128 and
+// up, at most 256 and as many as give 1184 blocks of 32 columns (eight per SM of a B200), whose sums a second launch adds.
+// Only the shape decides, so that results do not depend on the device or its load.
+struct SumSlices { int64_t count, rows; size_t floats; };
+inline SumSlices column_sum_slices(int64_t B, int cols) {
+  const int64_t gx = std::max<int64_t>(1, ((int64_t)cols + 31) / 32);
+  SumSlices s;
+  s.count = B <= 2048 ? 1 : std::min<int64_t>(std::min<int64_t>((B + 127) / 128, 256), std::max<int64_t>(1, 1184 / gx));
+  s.rows = std::max<int64_t>(1, (B + s.count - 1) / s.count);
+  s.count = std::max<int64_t>(1, (B + s.rows - 1) / s.rows);
+  s.floats = s.count > 1 ? (size_t)s.count * cols : 0;
+  return s;
+}
+
 template <typename T>
 int plan_layer_bw(const Problem& q, int out_total, bool saved, LayerBwLayout& L) {
   BwLayout<T> lay;
@@ -950,7 +966,8 @@ int plan_layer_bw(const Problem& q, int out_total, bool saved, LayerBwLayout& L)
     L.fused_bytes = (saved ? 0 : lay.ws_bytes) + plane;
   L.planes_off = 0;
   L.dx_off = saved && !lay.chunked ? 0 : (lay.ws_bytes + 255) / 256 * 256;
-  L.ws_bytes = L.dx_off + (q.S > 1 ? (size_t)q.B * q.S * DX * sizeof(T) : 0);
+  L.sums_off = L.dx_off + (q.S > 1 ? ((size_t)q.B * q.S * DX * sizeof(T) + 255) / 256 * 256 : 0);
+  L.ws_bytes = L.sums_off + column_sum_slices(q.B, out_total * (int)(sizeof(T) / 4)).floats * sizeof(float);
   L.ws_bytes = std::max(L.ws_bytes, L.fused_bytes);
   return BFLY_OK;
 }
@@ -999,7 +1016,7 @@ int drive_layer_bw(E& ex, const Problem& q_in, const T* tw2, const T* tw4, const
     rc = ex.stack_sums(dx, q.B, q.S, DX, q.in_size, d_in);
     if (rc != BFLY_OK) return rc;
   }
-  return d_bias ? ex.column_sums(grad, g_sB, q.B, out_total, d_bias) : BFLY_OK;
+  return d_bias ? ex.column_sums(grad, g_sB, q.B, out_total, d_bias, reinterpret_cast<float*>(static_cast<char*>(ws) + L.sums_off)) : BFLY_OK;
 }
 
 }  // namespace bfly

@@ -20,8 +20,9 @@ int fw2_launch(const Fw2Params& p, int ctas_per_sm, int sms, cudaStream_t stream
 // out[b, f] += bias[f], f < len, on a (B, width) matrix with row pitch `pitch` (elements).
 int bias_add_launch(float* out, const float* bias, int64_t B, int len, int64_t pitch, int sms, cudaStream_t stream);
 
-// out[c] = sum of g[b, c] over the rows of a (B, cols) matrix with row pitch `pitch`.
-int column_sums_launch(const float* g, int64_t pitch, int64_t B, int cols, float* out, int sms, cudaStream_t stream);
+// out[c] = sum of g[b, c] over the rows of a (B, cols) matrix with row pitch `pitch`, in an order that B and cols fix.
+// `partial`: column_sum_slices(B, cols).floats floats of scratch (bfly_driver.h).  `launches`: kernels launched.
+int column_sums_launch(const float* g, int64_t pitch, int64_t B, int cols, float* out, float* partial, cudaStream_t stream, int* launches);
 // out[b, c] = sum of g[b, s, c] over s; g (B, S, n), out (B, cols), cols <= n.
 int stack_sums_launch(const float* g, int64_t B, int S, int64_t n, int cols, float* out, int sms, cudaStream_t stream);
 

@@ -8,6 +8,7 @@
 #include <mutex>
 
 #include "bfly_fw2.h"
+#include "bfly_driver.h"
 #include "bfly_fast.h"
 #include "bfly_tma.h"
 
@@ -251,42 +252,49 @@ int bias_add_launch(float* out, const float* bias, int64_t B, int len, int64_t p
   return cudaGetLastError() == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
 }
 
-// Bias gradient: 32 columns x 8 row lanes per block, eight rows in flight per thread; the row lanes meet in shared
-// memory.  One row slice writes its sums directly (up to 512 rows: no clearing pass), more add them up.
-__global__ void __launch_bounds__(256) bfly_column_sums_kernel(const float* __restrict__ g, int64_t pitch, int64_t B, int cols,
-                                                                float* __restrict__ out, int64_t rows_per_slice) {
-  __shared__ float part[8][33];
+// Column sums of a (B, cols) matrix, the bias gradient: 32 columns x LANES row lanes per block, eight rows in flight per
+// thread; the row lanes meet in shared memory.  Slice y of the rows writes row y of `out`: the sums themselves where there
+// is one slice, else a matrix whose columns a second launch sums, so that every sum has one order whatever the schedule.
+template <int LANES>
+__global__ void __launch_bounds__(32 * LANES) bfly_column_sums_kernel(const float* __restrict__ g, int64_t pitch, int64_t B, int cols,
+                                                                       float* __restrict__ out, int64_t rows_per_slice) {
+  __shared__ float part[LANES][33];
   const int c = blockIdx.x * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
   const int64_t r0 = blockIdx.y * rows_per_slice, r1 = r0 + rows_per_slice < B ? r0 + rows_per_slice : B;
   float acc = 0.f;
   if (c < cols) {
     const float* q = g + c;
     int64_t r = r0 + lane;
-    for (; r + 56 < r1; r += 64) {
+    for (; r + 7 * LANES < r1; r += 8 * LANES) {
       float v[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) v[k] = __ldg(q + (r + 8 * k) * pitch);
+      for (int k = 0; k < 8; ++k) v[k] = __ldg(q + (r + LANES * k) * pitch);
 #pragma unroll
       for (int k = 0; k < 8; ++k) acc += v[k];
     }
-    for (; r < r1; r += 8) acc += __ldg(q + r * pitch);
+    for (; r < r1; r += LANES) acc += __ldg(q + r * pitch);
   }
   part[lane][threadIdx.x & 31] = acc;
   __syncthreads();
   if (lane == 0 && c < cols) {
-    for (int k = 1; k < 8; ++k) acc += part[k][threadIdx.x & 31];
-    if (gridDim.y == 1) out[c] = acc;
-    else atomicAdd(out + c, acc);
+    for (int k = 1; k < LANES; ++k) acc += part[k][threadIdx.x & 31];
+    out[(int64_t)blockIdx.y * cols + c] = acc;
   }
 }
-int column_sums_launch(const float* g, int64_t pitch, int64_t B, int cols, float* out, int sms, cudaStream_t stream) {
+int column_sums_launch(const float* g, int64_t pitch, int64_t B, int cols, float* out, float* partial, cudaStream_t stream, int* launches) {
+  *launches = 0;
   if (cols <= 0) return BFLY_OK;
   const int gx = (cols + 31) / 32;
-  int64_t slices = B <= 512 ? 1 : std::min<int64_t>((B + 127) / 128, std::max(1, 8 * sms / gx));
-  const int64_t rows = std::max<int64_t>(1, (B + slices - 1) / slices);
-  slices = std::max<int64_t>(1, (B + rows - 1) / rows);
-  if (slices > 1 && cudaMemsetAsync(out, 0, (size_t)cols * 4, stream) != cudaSuccess) return BFLY_E_CUDA;
-  bfly_column_sums_kernel<<<dim3(gx, (unsigned)slices), 256, 0, stream>>>(g, pitch, B, cols, out, rows);
+  const SumSlices s = column_sum_slices(B, cols);
+  if (s.count > 1 && !partial) return BFLY_E_WORKSPACE;
+  auto launch = [&](const float* src, int64_t row_pitch, int64_t rows, float* dst, int64_t slices, int64_t per_slice) {
+    const dim3 grid(gx, (unsigned)slices);
+    if (slices == 1 && rows > 64) bfly_column_sums_kernel<32><<<grid, 1024, 0, stream>>>(src, row_pitch, rows, cols, dst, per_slice);
+    else bfly_column_sums_kernel<8><<<grid, 256, 0, stream>>>(src, row_pitch, rows, cols, dst, per_slice);
+    ++*launches;
+  };
+  launch(g, pitch, B, s.count > 1 ? partial : out, s.count, s.rows);
+  if (s.count > 1) launch(partial, cols, s.count, out, 1, s.count);
   return cudaGetLastError() == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
 }
 // Input gradient of a layer whose stacks share their input.

@@ -741,10 +741,11 @@ struct CudaExec {
     return rc;
   }
   // column sums of a (B, cols) matrix
-  template <typename T> int column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out) {
+  template <typename T> int column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out, float* partial) {
+    int launches = 0;
     const int rc = column_sums_launch(reinterpret_cast<const float*>(g), pitch * (int)(sizeof(T) / 4), B, cols * (int)(sizeof(T) / 4),
-                                      reinterpret_cast<float*>(out), dev.sms, stream);
-    if (rc == BFLY_OK) g_launches.fetch_add(1);
+                                      reinterpret_cast<float*>(out), partial, stream, &launches);
+    if (rc == BFLY_OK) g_launches.fetch_add(launches);
     return rc;
   }
   // out[b, c] = sum over s of g[b, s, c], c < cols; g is (B, S, n)

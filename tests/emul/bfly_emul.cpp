@@ -288,10 +288,21 @@ struct EmulExec {
   }
   static constexpr bool kFusedBias = true;  // run_fw adds FwParams::bias
   // layers: the sums of the small kernels
-  template <typename T> int column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out) {
-    for (int c = 0; c < cols; ++c) out[c] = Ops<T>::zero();
-    for (int64_t b = 0; b < B; ++b)
-      for (int c = 0; c < cols; ++c) out[c] = add1(out[c], g[b * pitch + c]);
+  template <typename T> int column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out, float* partial) {
+    constexpr int F = (int)(sizeof(T) / 4);
+    auto sums = [](const float* src, int64_t p, int64_t rows, int n, float* dst) {
+      for (int c = 0; c < n; ++c) {
+        dst[c] = 0.f;
+        for (int64_t r = 0; r < rows; ++r) dst[c] += src[r * p + c];
+      }
+    };
+    const SumSlices s = column_sum_slices(B, cols * F);
+    const float* gf = reinterpret_cast<const float*>(g);
+    float* of = reinterpret_cast<float*>(out);
+    if (s.count == 1) { sums(gf, pitch * F, B, cols * F, of); return BFLY_OK; }
+    for (int64_t y = 0; y < s.count; ++y)
+      sums(gf + y * s.rows * pitch * F, pitch * F, std::min(s.rows, B - y * s.rows), cols * F, partial + y * cols * F);
+    sums(partial, cols * F, s.count, cols * F, of);
     return BFLY_OK;
   }
   template <typename T> int stack_sums(const T* g, int64_t B, int S, int64_t n, int cols, T* out) {

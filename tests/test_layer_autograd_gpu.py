@@ -67,3 +67,20 @@ def test_layer_outputs_take_in_place_operators(dev, kind, in_size, out_size, lea
         return [z.detach().clone()] + list(torch.autograd.grad(z.abs().sum(), [x] + list(p for p in layer.parameters() if p.numel())))
     for a, b in zip(grads(True), grads(False)):
         assert a.shape == b.shape and (a - b).abs().max() <= 1e-5 * b.abs().max()
+
+
+@pytest.mark.parametrize("kind,in_size,out_size", [("f32", 100, 70), ("f32", 40, 3000), ("c64", 60, 50), ("base4", 100, 128)])
+@pytest.mark.parametrize("batch", [64, 65, 700, 2048, 2049, 40011])
+def test_bias_gradients_have_one_order(dev, kind, in_size, out_size, batch):
+    """The bias gradient of a layer off the fused route sums its rows in an order that the shape fixes: the same bits on
+    every call, the float64 sum within what float32 sums of that many rows may be off (terms that grow like the square root of the rows, 2^-24 of the sum so far each)."""
+    torch.manual_seed(batch)
+    layer = _layer(kind, in_size, out_size, dev)
+    x = torch.randn(batch, in_size, dtype=layer.bias.dtype, device=dev)
+    g = torch.randn(batch, out_size, dtype=layer.bias.dtype, device=dev)
+    first = torch.autograd.grad(layer(x), [layer.bias], g)[0]
+    for _ in range(10):
+        assert torch.equal(torch.autograd.grad(layer(x), [layer.bias], g)[0], first)
+    wide = torch.complex128 if kind == "c64" else torch.float64
+    want = g.to(wide).sum(0)
+    assert (first.to(wide) - want).abs().max() <= 2e-6 * want.abs().max()
