@@ -697,10 +697,25 @@ class KroneckerTwiddle : public torch::autograd::Function<KroneckerTwiddle> {
     return out;
   }
 };
+// The same from views and one cat per block, which every transform has rules for; the node above has none for forward
+// mode and functorch.
+Tensor kronecker_composed(const Tensor& t1, const Tensor& t2, bool inc) {
+  const int64_t S = t1.size(0), nb = t1.size(1), l1 = t1.size(2), h1 = t1.size(3), l2 = t2.size(2), h2 = t2.size(3);
+  const Tensor a = t1.unsqueeze(3).expand({S, nb, l1, 2 * h2, h1, 2, 2}).reshape({S, nb, l1, 2 * h2 * h1, 2, 2});
+  const Tensor b = t2.unsqueeze(4).expand({S, nb, l2, h2, 2 * h1, 2, 2}).reshape({S, nb, l2, h2 * 2 * h1, 2, 2});
+  std::vector<Tensor> blocks;
+  for (int64_t j = 0; j < nb; ++j) {
+    const bool up = inc != (j % 2 == 1);
+    blocks.push_back(torch::cat({(up ? a : b).select(1, j), (up ? b : a).select(1, j)}, 1));
+  }
+  return torch::stack(blocks, 1);
+}
 Tensor kronecker_twiddle(const Tensor& twiddle1, const Tensor& twiddle2, bool increasing_stride) {
-  BFLY_CHECK_DIM(twiddle1, 6); BFLY_CHECK_DIM(twiddle2, 6);
+  BFLY_CHECK_DIM(twiddle1, 6); BFLY_CHECK_DIM(twiddle2, 6); BFLY_CHECK_SAME_DEVICE(twiddle1, twiddle2);
   TORCH_CHECK(twiddle1.size(0) == twiddle2.size(0) && twiddle1.size(1) == twiddle2.size(1) && twiddle1.scalar_type() == twiddle2.scalar_type(),
               "kronecker_twiddle: the two maps must have the same stacks, blocks and dtype");
+  if (has_tangent(twiddle1) || has_tangent(twiddle2) || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+    return kronecker_composed(twiddle1, twiddle2, increasing_stride);
   return KroneckerTwiddle::apply(twiddle1, twiddle2, increasing_stride);
 }
 

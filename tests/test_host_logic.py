@@ -653,3 +653,28 @@ def test_rows_between_elements_are_refused(emul):
         glue = emul.bfly_emul_fw_glue(1, P(tw), p["x"], 0, *s, p["out"], 0, None, None, None, 3, 1, log_n, 1, n, n, 1, 64)
         bad = lambda *names: -3 if which in names else 0
         assert (fw, bw, both, layer, glue) == (bad("x", "out"), bad("x", "g", "dx"), bad(*p), bad(*p), bad("x", "out")), which
+
+
+def test_kronecker_twiddle_as_transforms_see_it():
+    """The twiddle of a 2-D map is index work, the same on any device: gradients, forward mode and functorch transforms go
+    through it, tensors of two devices do not."""
+    import butterfly_b200 as bb
+    from torch.autograd import forward_ad
+    torch.manual_seed(4)
+    t1, t2 = (torch.randn(1, 2, l, 1 << (l - 1), 2, 2, dtype=torch.float64) for l in (3, 2))
+    v = torch.randn_like(t1)
+    for inc in (True, False):
+        k = lambda a, b=t2: bb.combine.kronecker_twiddle(a, b, inc)
+        want = k(v, torch.zeros_like(t2))  # linear in the pair
+        with forward_ad.dual_level():
+            assert torch.equal(forward_ad.unpack_dual(k(forward_ad.make_dual(t1, v))).tangent, want)
+        assert torch.equal(torch.func.jvp(k, (t1,), (v,))[1], want)
+        assert torch.equal(torch.func.vmap(k)(torch.stack([t1, v])), torch.stack([k(t1), k(v)]))
+        g = torch.randn_like(want)
+        leaf = t1.clone().requires_grad_(True)
+        d, = torch.autograd.grad(k(leaf), leaf, g)
+        assert torch.allclose(torch.func.vjp(k, t1)[1](g)[0], d)
+        assert abs(((d * v).sum() - (want * g).sum()).item()) < 1e-9  # the adjoint of the forward
+        assert torch.autograd.gradgradcheck(k, (leaf,))
+    with pytest.raises(RuntimeError, match="same device"):
+        bb.combine.kronecker_twiddle(t1.to("meta"), t2, True)
