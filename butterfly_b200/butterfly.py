@@ -17,9 +17,13 @@ from .multiply_base4 import butterfly_multiply_base4, twiddle_base2_to_base4
 _COMPLEX = {torch.float32: torch.complex64, torch.float64: torch.complex128}
 
 
-def _native(twiddle, x):
-    """Can the native layer operator take these?  (Everything else goes through the multiply operators, which say what is wrong.)"""
-    return x.is_cuda and x.dtype == twiddle.dtype and (x.dtype == torch.float32 or x.dtype == torch.complex64)
+def _native(layer, twiddle, x):
+    """Can the native layer operator run the whole layer?  Everything else goes through pre_process, the multiply operators
+    and post_process, which say what is wrong: glue of the class's own (asked at every call), other types."""
+    cls, dt = type(layer), x.dtype
+    if cls.pre_process is not Butterfly.pre_process or cls.post_process is not Butterfly.post_process:
+        return False
+    return x.is_cuda and dt == twiddle.dtype and (dt == torch.float32 or dt == torch.complex64)
 
 
 def _as_rows(x, width):
@@ -60,13 +64,6 @@ class Butterfly(nn.Module):
         shape = (self.nstacks, nblocks, self.log_n, self.n // 2, 2, 2)
         self._make_params(shape, dtype, init, (out_size,) if bias else None)
         self.reset_parameters()
-
-    # ---- one native operator for the whole layer, unless a subclass has glue of its own
-    _native_glue = True
-
-    def __init_subclass__(cls, **kwargs):
-        super().__init_subclass__(**kwargs)
-        cls._native_glue = cls.pre_process is Butterfly.pre_process and cls.post_process is Butterfly.post_process
 
     # ---- construction helpers shared by the subclasses
     def _configure(self, in_size, out_size, complex, increasing_stride, nblocks):
@@ -131,7 +128,7 @@ class Butterfly(nn.Module):
         leading part of the parameters for a shorter input (the output then has the n' columns of
         the first stack, as in the reference: torch_butterfly/butterfly.py:147-150)."""
         twiddle = self._effective_twiddle()
-        if self._native_glue and not subtwiddle and _native(twiddle, input):
+        if not subtwiddle and _native(self, twiddle, input):
             inc = self.increasing_stride
             if conjugate and self.complex:
                 twiddle = twiddle.conj()
@@ -309,7 +306,7 @@ class ButterflyBase4(Butterfly):
         self.twiddle2._is_structured = True
 
     def forward(self, input):
-        if self._native_glue and _native(self.twiddle4, input):
+        if _native(self, self.twiddle4, input):
             return butterfly_layer(self.twiddle4, self.twiddle2, input, self.bias, self.increasing_stride, self.out_size)
         rows = self.pre_process(input)
         output_size = self.out_size if self.nstacks == 1 else None

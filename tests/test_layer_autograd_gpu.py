@@ -84,3 +84,21 @@ def test_bias_gradients_have_one_order(dev, kind, in_size, out_size, batch):
     wide = torch.complex128 if kind == "c64" else torch.float64
     want = g.to(wide).sum(0)
     assert (first.to(wide) - want).abs().max() <= 2e-6 * want.abs().max()
+
+
+@pytest.mark.parametrize("kind", ["f32", "c64", "base4"])
+def test_glue_given_to_a_class_later_runs(dev, kind, monkeypatch):
+    """pre_process / post_process are looked up at the call, as methods are."""
+    import butterfly_b200 as bb
+    layer = _layer(kind, 60, 50, dev)
+    x = torch.randn(7, 60, dtype=layer.bias.dtype, device=dev)
+    plain, bias = layer(x).detach(), layer.bias.detach()
+    pre, post = bb.Butterfly.pre_process, bb.Butterfly.post_process
+    cls = type("Own", (type(layer),), {})
+    layer.__class__ = cls
+    assert torch.equal(layer(x), plain)
+    cls.pre_process = lambda self, rows: pre(self, 2 * rows)
+    assert torch.allclose(layer(x), 2 * (plain - bias) + bias, rtol=1e-4, atol=1e-4)
+    del cls.pre_process
+    cls.post_process = lambda self, rows, out, out_size=None: 3 * post(self, rows, out, out_size)
+    assert torch.allclose(layer(x), 3 * plain, rtol=1e-4, atol=1e-4)
