@@ -19,11 +19,17 @@ _COMPLEX = {torch.float32: torch.complex64, torch.float64: torch.complex128}
 
 def _native(layer, twiddle, x):
     """Can the native layer operator run the whole layer?  Everything else goes through pre_process, the multiply operators
-    and post_process, which say what is wrong: glue of the class's own (asked at every call), other types."""
+    and post_process, which say what is wrong: glue of the class's own (asked at every call), other types, and biases that
+    only broadcasting or promotion adds (real radix-2 layers never took those)."""
     cls, dt = type(layer), x.dtype
     if cls.pre_process is not Butterfly.pre_process or cls.post_process is not Butterfly.post_process:
         return False
-    return x.is_cuda and dt == twiddle.dtype and (dt == torch.float32 or dt == torch.complex64)
+    if not x.is_cuda or dt != twiddle.dtype or (dt != torch.float32 and dt != torch.complex64):
+        return False
+    if dt == torch.float32 and not isinstance(layer, ButterflyBase4):
+        return True
+    b = layer.bias
+    return b is None or (b.dtype == dt and b.dim() == 1 and b.shape[0] >= layer.out_size)
 
 
 def _as_rows(x, width):

@@ -102,3 +102,19 @@ def test_glue_given_to_a_class_later_runs(dev, kind, monkeypatch):
     del cls.pre_process
     cls.post_process = lambda self, rows, out, out_size=None: 3 * post(self, rows, out, out_size)
     assert torch.allclose(layer(x), 3 * plain, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("kind", ["c64", "base4"])
+@pytest.mark.parametrize("bias", ["promoted", "broadcast"])
+def test_biases_that_promote_or_broadcast(dev, kind, bias):
+    """Complex and radix-4 layers add whatever bias PyTorch adds to their output."""
+    layer = _layer(kind, 60, 50, dev)
+    x = torch.randn(7, 60, dtype=layer.bias.dtype, device=dev)
+    own = layer.bias.detach().clone()
+    base = layer(x).detach() - own
+    new = torch.randn(50, dtype=torch.float32 if kind == "c64" else torch.float64, device=dev) if bias == "promoted" else own[:1].clone()
+    layer.bias = torch.nn.Parameter(new)
+    y = layer(x)
+    assert y.dtype == (base + new).dtype and torch.allclose(y, base + new, rtol=1e-4, atol=1e-4)
+    y.abs().sum().backward()
+    assert layer.bias.grad.shape == new.shape
