@@ -106,12 +106,58 @@ def test_fused_transforms_against_torch_fft(dev):
     launches = abi.launch_count()
     assert_rtol_atol(one(x), want, "circulant as one butterfly", rtol=1e-4, atol=2e-4 * n ** 0.5)
     assert abi.launch_count() - launches == 1
-    # a length that is not a power of two runs link by link
+    # a length that is no power of two: padded rows in, cut rows out, two launches as well
     m = 12
     colm = torch.randn(m, dtype=torch.complex64)
     xm = torch.randn(4, m, dtype=torch.complex64, device=dev)
     idx = (torch.arange(m).unsqueeze(1) - torch.arange(m).unsqueeze(0)) % m
-    assert_rtol_atol(special.circulant(colm).to(dev)(xm), xm @ colm.to(dev)[idx.to(dev)].t(), "circulant n=12", rtol=1e-4, atol=1e-4)
+    ragged = special.circulant(colm).to(dev)
+    launches = abi.launch_count()
+    assert_rtol_atol(ragged(xm), xm @ colm.to(dev)[idx.to(dev)].t(), "circulant n=12", rtol=1e-4, atol=1e-4)
+    assert abi.launch_count() - launches == 2
+
+
+@pytest.mark.parametrize("n", [12, 100, 1000])
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("separate_diagonal", [False, True])
+def test_training_circulants_of_ragged_lengths(dev, oracle_mod, n, cplx, separate_diagonal):
+    """Gradients through pipelines whose rows enter padded and leave cut: input and parameters against autograd through the
+    dense matrices the double-precision oracle gives for the same factors."""
+    from butterfly_b200 import special
+    torch.manual_seed(n)
+    dt = torch.complex64 if cplx else torch.float32
+    f = special.circulant(torch.randn(n, dtype=dt), separate_diagonal=separate_diagonal)
+    params = [p.detach().clone() for p in f.parameters()]
+    f = f.to(dev)
+    x = torch.randn(3, 5, n, dtype=dt, device=dev, requires_grad=True)
+    g = torch.randn(3, 5, n, dtype=dt, device=dev)
+    y = f(x)
+    assert y.shape == g.shape and y.dtype == dt
+    grads = torch.autograd.grad(y, [x] + list(f.parameters()), g)
+    # the same chain in double precision: forward links, then their adjoints
+    w = lambda t: t.detach().cpu().to(torch.complex128)
+    rows, gr = w(x).reshape(-1, 1, n), w(g).reshape(-1, 1, n)
+    tws = [w(p) for p in params if p.dim() == 6]
+    N = 2 * tws[0].shape[3]
+    pad = lambda t: torch.nn.functional.pad(t, (0, N - n))
+    if separate_diagonal:
+        diag = w(next(p for p in params if p.dim() == 1))
+        a = oracle_mod.multiply_fw(tws[0], pad(rows), False)
+        out = oracle_mod.multiply_fw(tws[1], a * diag, True)
+        d2, d_mid = oracle_mod.multiply_bw(tws[1], a * diag, pad(gr), True)
+        d_diag = (d_mid * a.conj()).sum((0, 1))
+        d1, d_x = oracle_mod.multiply_bw(tws[0], pad(rows), d_mid * diag.conj(), False)
+        by_shape = [d1, d_diag, d2]
+    else:
+        out = oracle_mod.multiply_fw(tws[0], pad(rows), False)
+        d1, d_x = oracle_mod.multiply_bw(tws[0], pad(rows), pad(gr), False)
+        by_shape = [d1]
+    real = lambda t: t if cplx else t.real
+    want = [real(out[..., :n]).reshape(y.shape), real(d_x[..., :n]).reshape(x.shape)] + by_shape
+    assert len(grads) == len(want) - 1
+    for got, ref in zip([y.detach(), *grads], want):
+        assert got.shape == ref.shape
+        assert (got.cpu().to(ref.dtype) - ref).abs().max() <= 2e-5 * ref.abs().max()
 
 
 @pytest.mark.parametrize("cplx", [False, True])

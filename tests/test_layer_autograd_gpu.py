@@ -118,3 +118,22 @@ def test_biases_that_promote_or_broadcast(dev, kind, bias):
     assert y.dtype == (base + new).dtype and torch.allclose(y, base + new, rtol=1e-4, atol=1e-4)
     y.abs().sum().backward()
     assert layer.bias.grad.shape == new.shape
+
+
+@pytest.mark.parametrize("kind,planes", [("f32", 2), ("c64", 5), ("base4", 2)])
+@pytest.mark.parametrize("save", [0, -1])
+def test_what_a_layer_holds_for_its_backward(dev, kind, planes, save):
+    """Between forward and backward a layer holds its input and, under the option's default, one plane per phase boundary
+    (24 stages: three phases of 8 for floats, six of 4 for complex values) next to the re-ordered twiddles."""
+    from conftest import abi_option
+    layer = _layer(kind, 4096, 4096, dev, bias=False, nblocks=2)
+    x = torch.randn(1024, 4096, dtype=torch.complex64 if kind == "c64" else torch.float32, device=dev)
+    plane = x.numel() * x.element_size()
+    with abi_option("autograd_save", save):
+        layer(x)
+        before = torch.cuda.memory_allocated()
+        y = layer(x)
+        held = torch.cuda.memory_allocated() - before - plane
+        del y
+        assert torch.cuda.memory_allocated() == before
+    assert held < 4096 if save == 0 else planes * plane <= held < (planes + 0.5) * plane
