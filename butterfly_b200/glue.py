@@ -88,7 +88,8 @@ def butterfly_multiply_glue(twiddle: torch.Tensor, input: torch.Tensor, increasi
     width = input.shape[-1]
     if in_perm is not None and width < n:  # the gather would read past the row, which a GPU answers with a lost context
         raise RuntimeError("butterfly_multiply_glue: in_perm needs rows of %d entries, got %d" % (n, width))
-    if n > limit or width > n or not input.is_cuda:
+    # (a tracer and functorch's transforms see through the links, not through the fused operator's optional result)
+    if n > limit or width > n or not input.is_cuda or torch.jit.is_tracing() or torch._C._functorch.peek_interpreter_stack() is not None:
         return _unfused(twiddle, input, increasing_stride, in_perm, out_diag, out_perm, out_real)
     if not (torch.is_grad_enabled() and (input.requires_grad or twiddle.requires_grad
                                          or (out_diag is not None and out_diag.requires_grad))):

@@ -137,3 +137,21 @@ def test_what_a_layer_holds_for_its_backward(dev, kind, planes, save):
         del y
         assert torch.cuda.memory_allocated() == before
     assert held < 4096 if save == 0 else planes * plane <= held < (planes + 0.5) * plane
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("make", [lambda s: s.circulant(torch.randn(12)), lambda s: s.circulant(torch.randn(16)), lambda s: s.fft(16),
+                                  lambda s: s.ifft(16, br_first=False)], ids=["circulant12", "circulant16", "fft", "ifft"])
+def test_pipelines_trace_and_vmap(dev, make):
+    """Under a tracer or a functorch transform a pipeline runs its links, which have rules there."""
+    from butterfly_b200 import special
+    torch.manual_seed(8)
+    f = make(special).to(dev)
+    b = f[0].butterfly
+    x = torch.randn(2, 5, b.in_size, dtype=torch.float32 if f[0].real_in else torch.complex64, device=dev)
+    traced = torch.jit.trace(f, x, check_trace=False)
+    other = torch.randn_like(x)
+    close = lambda a, c: (a - c).abs().max() <= 1e-5 * c.abs().max()
+    assert close(traced(other), f(other)) and close(torch.func.vmap(f)(x), f(x))
+    with torch.no_grad():
+        assert close(torch.func.vmap(f)(x), f(x))
