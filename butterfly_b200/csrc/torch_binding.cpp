@@ -187,7 +187,7 @@ std::tuple<Tensor, Tensor> butterfly_multiply_bw(const Tensor& twiddle, const Te
   return bw_impl(twiddle, input, grad, increasing_stride, nullptr);
 }
 
-// The autograd node may keep the forward's phase-boundary activations for its backward (the
+// The autograd nodes (the operator's and the layers') may keep the forward's phase-boundary activations for the backward (the
 // reference recomputes them, csrc/butterfly.cpp:99-118): that removes one forward-sized pass from
 // every training step at the price of holding (phases - 1) activation-sized buffers per call
 // between forward and backward.  On by default while those buffers stay under 1 GiB per call;

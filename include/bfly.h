@@ -185,7 +185,8 @@ int bfly_bw_c64_saved(const void* twiddle, const void* x, int64_t x_sB, int64_t 
  * launch path never reads the environment.  Names (environment variable): "tma" (BFLY_TMA: 0 =
  * per-thread tile copies instead of the TMA unit), "fw2" (BFLY_FW2: 0 = generic forward kernel
  * only), "bw_v2" (BFLY_BW_V2), "fw_kmax", "fw_rows", "fw_logcmax", "bw_rows", "bw_maxsg" (planner
- * overrides; -1 = default), "autograd_save" (BFLY_AUTOGRAD_SAVE: the torch autograd operator keeps
+ * overrides; -1 = default), "fw_spread" (BFLY_FW_SPREAD), "virtual_rows" (BFLY_VIRTUAL_ROWS: 0 = rows one by
+ * one), "autograd_save" (BFLY_AUTOGRAD_SAVE: the torch autograd operators, butterfly_multiply and the layers, keep
  * the forward's snapshots: 0 never, 1 always, -1 by size).  Returns BFLY_E_ARG for an unknown name. */
 int bfly_set_option(const char* name, int value);
 int bfly_get_option(const char* name, int* value);
@@ -225,6 +226,8 @@ int bfly_linear_bw_f32(const float* twiddle, const float* x, int64_t x_sB, const
  *   snapshots  NULL, or bfly_layer_snapshot_bytes bytes that the matching bfly_layer_bw takes as `snapshots`
  * bfly_layer_bw: grad (batch, output_size) rows with pitch g_sB; d_input is (batch, input_size) contiguous when
  * nstacks > 1, else (batch, max(input_size, n)) of which the first input_size columns are the result; d_bias may be NULL.
+ * Where bfly_linear_bw_f32 would run, it does (sums over stacks and rows in no fixed order); elsewhere both sums have one
+ * order, which the shape fixes.
  * Work space: bfly_fw_workspace_bytes (forward; not needed with snapshots) and bfly_layer_bw_workspace_bytes. */
 typedef struct {
   int dtype, base4, batch, nstacks, log_n, nblocks, input_size, output_size, increasing_stride;
