@@ -329,14 +329,16 @@ BFLY_HD void bw2_init(const BwParams<T>& p, const AccStore<T, KW>& accs, const u
 }
 
 // Add this thread's accumulators to d_twiddle.
-template <typename T, int KW>
+// (fold: as for the packed-pair kernel, bfly_bw3.h)
+template <typename T, int KW, typename FOLD>
 BFLY_HD void bw2_flush(const BwParams<T>& p, const AccStore<T, KW>& accs, const uint32_t* meta, int stack, int tid,
-                       int nthr) {
+                       int nthr, FOLD&& fold) {
   constexpr int N = BwTwn<KW>::value;
   for (int j = 0; j < p.nsg; ++j) {
     const BwSg& sg = p.sg[j];
     T acc[N];
     accs.ld(j, acc);
+    if (!fold(j, acc)) continue;
     T* dtw = p.dtw[sg.which] + (int64_t)stack * p.tw_stack[sg.which];
     const uint32_t* tws = meta + (size_t)p.nsg * nthr * 4;
     const uint32_t t0 = tws[(j * 2 + 0) * nthr + tid];

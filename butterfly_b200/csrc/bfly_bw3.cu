@@ -133,7 +133,16 @@ bfly_bw3_kernel(const __grid_constant__ Bw3Params p, const __grid_constant__ CUt
   }
   if (tid == 0) tma_store_wait_all();
   if (kBw3Prefetch || kBw3PrefetchTw) acc.wait_ld();  // the fetch issued by the last step
-  if (!gave_up) bw3_flush(p, acc, stack, pbase, tid);
+  // Rows that share a tile row leave 2^vr threads with sums for the same twiddles.  They meet in the CTA before one of them
+  // adds to d_twiddle, in the tiles' shared memory (thread 0 has waited for its stores).  Added one by one they made
+  // chains of float32 additions 2^vr times as long, which also queue at the same addresses (n = 64, 2^21 values: 1.1e-6
+  // off the float64 sum and 104 us, now 3.3e-7 and 27 us; row by row 8.7e-7; 2^25 values 233 and 132 us).
+  auto fold = [&](int j, float* ar) -> bool {
+    const int mask = bw_row_threads(q, p.sg[j].ubit, 7);
+    if (mask) fold_threads<32, kBw3Threads>(ar, mask, sm, tid);
+    return !(tid & mask);
+  };
+  if (!gave_up) bw3_flush(p, acc, stack, pbase, tid, fold);
   if (!gave_up && q.dbias) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {

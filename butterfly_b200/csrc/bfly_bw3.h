@@ -523,9 +523,10 @@ BFLY_HD void bw3_init(const Bw3Params& p, const ACC& acc, uint32_t* meta, int st
   acc.wait_st();
 }
 
-// Add this thread's accumulators to d_twiddle (one 16-byte vector reduction per 2x2 block).
-template <typename ACC>
-BFLY_HD void bw3_flush(const Bw3Params& p, const ACC& acc, int stack, int pbase, int tid) {
+// Add this thread's accumulators to d_twiddle (one 16-byte vector reduction per 2x2 block).  fold(j, accumulators) sums
+// those of sub-group j over the threads that hold the same twiddles and says whether this thread adds the result.
+template <typename ACC, typename FOLD>
+BFLY_HD void bw3_flush(const Bw3Params& p, const ACC& acc, int stack, int pbase, int tid, FOLD&& fold) {
   float* dtw = p.b.dtw[0] + (int64_t)stack * p.b.tw_stack[0];
   for (int j = 0; j < p.b.nsg; ++j) {
     const Bw3Sg& s = p.sg[j];
@@ -534,6 +535,7 @@ BFLY_HD void bw3_flush(const Bw3Params& p, const ACC& acc, int stack, int pbase,
     acc.wait_st();
     acc.ld32(j * 64 + 32, ar);
     acc.wait_ld();
+    if (!fold(j, ar)) continue;
     for (int k = 0; k < s.nst; ++k) {
       uint32_t off[16];
       bw3_tw_offsets(s, k, col0, off);

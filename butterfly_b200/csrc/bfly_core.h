@@ -68,6 +68,30 @@ template <int IMM, typename T> inline void sm_st16(smaddr_t a, const T* v) {
 }
 #endif
 
+#if defined(__CUDACC__)
+// Sums w[0 .. N) over the threads of a CTA of NT whose indices differ in the bits of `mask` alone (uniform; every thread
+// calls): lanes by shuffles, warps through `buf` (N * NT floats of shared memory that nothing else uses), two by two, so
+// that all of them end with the same sums.
+template <int N, int NT>
+__device__ __forceinline__ void fold_threads(float* w, int mask, float* buf, int tid) {
+#pragma unroll 1
+  for (int b = 1; b < 32; b <<= 1) {
+    if (!(mask & b)) continue;
+#pragma unroll
+    for (int k = 0; k < N; ++k) w[k] += __shfl_xor_sync(0xffffffffu, w[k], b);
+  }
+#pragma unroll 1
+  for (int b = 32; b < NT; b <<= 1) {
+    if (!(mask & b)) continue;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) buf[k * NT + tid] = w[k];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) w[k] += buf[k * NT + (tid ^ b)];
+  }
+}
+#endif
 #if defined(__CUDA_ARCH__)
 __device__ __forceinline__ void unpack16(const float4& q, float* v) { v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w; }
 __device__ __forceinline__ void unpack16(const float4& q, cf* v) { v[0] = cf{q.x, q.y}; v[1] = cf{q.z, q.w}; }

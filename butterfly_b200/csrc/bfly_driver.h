@@ -203,7 +203,7 @@ inline void twiddle_stack_sizes(const Problem& q, int64_t out[2]) {
 // Narrow rows of a large problem run several to a tile row of 2^target columns (log2 of their number; 0 = one by one):
 // with one row of 64 columns per tile row, half of the 256 threads share a row's few units and the shared-memory
 // round trips are short and many.  2^25 floats, microseconds one by one and this way: n = 64 forward 505 and 83, backward
-// 963 and 231; n = 256 201 and 93, 409 and 167; radix 4 n = 64 forward 1094 and 118; n = 512 backward 482 and 328.
+// 963 and 132; n = 256 201 and 93, 409 and 167; radix 4 n = 64 forward 1094 and 118; n = 512 backward 482 and 324.
 // Below 2^21 elements the tiles would no longer cover the chip.
 inline int virtual_rows(const Problem& q, int target) {
   const Options& o = options();

@@ -456,7 +456,15 @@ bfly_bw2_kernel(const __grid_constant__ BwParams<T> p, const __grid_constant__ C
     }
   }
   if (p.tma && tid == 0) tma_store_wait_all();
-  if (!gave_up) bw2_flush<T, KW>(p, accs, meta, stack, tid, kThreads);
+  auto fold = [&](int j, T* a) -> bool {  // rows that share a tile row: as in bfly_bw3_kernel
+    if constexpr (sizeof(T) == 4) {
+      const int mask = bw_row_threads(p, p.sg[j].ubit, p.sg[j].nubits);
+      if (mask) fold_threads<AccStore<T, KW>::N, kThreads>(a, mask, smX, tid);
+      return !(tid & mask);
+    }
+    return true;
+  };
+  if (!gave_up) bw2_flush<T, KW>(p, accs, meta, stack, tid, kThreads, fold);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {

@@ -279,4 +279,12 @@ template <typename T> BFLY_HD int bw_gin_cols(const BwParams<T>& p, int stack) {
   return left < p.gin_cols ? left : p.gin_cols;
 }
 
+// Several rows to a tile row: the bits of a thread index that tell rows apart when unit bit j sits at tile column bit
+// ubit[j].  Threads that differ in these bits alone hold sums for the same twiddles.
+template <typename T> BFLY_HD int bw_row_threads(const BwParams<T>& p, const uint8_t* ubit, int nubits) {
+  int mask = 0;
+  for (int j = 0; j < nubits; ++j) mask |= (p.vr > 0 && ubit[j] >= p.log_n ? 1 : 0) << j;
+  return mask;
+}
+
 }  // namespace bfly

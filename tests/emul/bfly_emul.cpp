@@ -21,6 +21,23 @@ namespace {
 long g_fw2_calls = 0;  // launches the emulator ran through the packed-pair forward path
 long g_bw3_calls = 0;  // ... and through the packed-pair backward phase path
 
+// The accumulators of every sub-group and thread, summed two by two over the thread bits of mask(j) (fold_threads).
+template <int N, typename T = float, typename MASK, typename LD>
+std::vector<T> fold_rows(int nsg, int nthr, MASK mask, LD ld) {
+  std::vector<T> w((size_t)nsg * nthr * N);
+  for (int j = 0; j < nsg; ++j) {
+    T* a = &w[(size_t)j * nthr * N];
+    for (int tid = 0; tid < nthr; ++tid) ld(j, tid, a + (size_t)tid * N);
+    for (int b = 1; b < nthr; b <<= 1)
+      if (mask(j) & b)
+        for (int tid = 0; tid < nthr; ++tid)
+          if (!(tid & b))
+            for (int k = 0; k < N; ++k)
+              a[(size_t)tid * N + k] = a[(size_t)(tid ^ b) * N + k] = add1(a[(size_t)tid * N + k], a[(size_t)(tid ^ b) * N + k]);
+  }
+  return w;
+}
+
 struct EmulExec {
   int sms = 7;       // odd on purpose: exercises ragged row slices
   int threads_ = 64;  // simulated block size (any power of two)
@@ -141,7 +158,13 @@ struct EmulExec {
             tile_store_v<float>(q.gout, q.gout_sB, q.gout_sS, q.gout_cols, q.B_rows, stack, row0, kBw3Rows, q.panel, pbase, true, q.log_n, q.vr, smG, tid, nthr);
         }
       }
-      for (int tid = 0; tid < nthr; ++tid) bw3_flush(p, accs[tid], stack, pbase, tid);
+      const std::vector<float> folded = fold_rows<32>(q.nsg, nthr, [&](int j) { return bw_row_threads(q, p.sg[j].ubit, 7); },
+                                                      [&](int j, int tid, float* w) { accs[tid].ld32(j * 64 + 32, w); });
+      for (int tid = 0; tid < nthr; ++tid)
+        bw3_flush(p, accs[tid], stack, pbase, tid, [&](int j, float* w) {
+          std::copy_n(&folded[(size_t)(j * nthr + tid) * 32], 32, w);
+          return !(tid & bw_row_threads(q, p.sg[j].ubit, 7));
+        });
     }
     return BFLY_OK;
   }
@@ -241,7 +264,13 @@ struct EmulExec {
         for (int tid = 0; tid < nthr; ++tid)
           tile_store_v<T>(p.gout, p.gout_sB, p.gout_sS, p.gout_cols, bw_row_limit(p, re), stack, row0, kBw2Rows, p.panel, pbase, p.vec_o != 0, p.log_n, p.vr, smG.data(), tid, nthr);
       }
-      for (int tid = 0; tid < nthr; ++tid) bw2_flush<T, KW>(p, accs[tid], meta.data(), stack, tid, nthr);
+      auto mask = [&](int j) { return sizeof(T) == 4 ? bw_row_threads(p, p.sg[j].ubit, p.sg[j].nubits) : 0; };
+      const std::vector<T> folded = fold_rows<N, T>(p.nsg, nthr, mask, [&](int j, int tid, T* w) { accs[tid].ld(j, w); });
+      for (int tid = 0; tid < nthr; ++tid)
+        bw2_flush<T, KW>(p, accs[tid], meta.data(), stack, tid, nthr, [&](int j, T* w) {
+          std::copy_n(&folded[(size_t)(j * nthr + tid) * N], N, w);
+          return !(tid & mask(j));
+        });
     }
     return BFLY_OK;
   }
