@@ -146,7 +146,7 @@ bfly_bw3_kernel(const __grid_constant__ Bw3Params p, const __grid_constant__ CUt
   if (!gave_up && q.dbias) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const int flat = stack * (1 << q.log_n) + (q.panel.col(pbase, 8 * tid + e) & ((1 << q.log_n) - 1));
+      const int flat = stack * (1 << q.log_n) + q.panel.col(pbase, 8 * tid + e);
       if (flat < q.dbias_len) atomicAdd(q.dbias + flat, db[e]);
     }
   }

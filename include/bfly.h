@@ -226,8 +226,8 @@ int bfly_linear_bw_f32(const float* twiddle, const float* x, int64_t x_sB, const
  *   snapshots  NULL, or bfly_layer_snapshot_bytes bytes that the matching bfly_layer_bw takes as `snapshots`
  * bfly_layer_bw: grad (batch, output_size) rows with pitch g_sB; d_input is (batch, input_size) contiguous when
  * nstacks > 1, else (batch, max(input_size, n)) of which the first input_size columns are the result; d_bias may be NULL.
- * Where bfly_linear_bw_f32 would run, it does (sums over stacks and rows in no fixed order); elsewhere both sums have one
- * order, which the shape fixes.
+ * Where bfly_linear_bw_f32 would run, it does (d_input of several stacks, and d_bias from n = 1024 on, in no fixed order);
+ * elsewhere both sums have one order, which the shape fixes.
  * Work space: bfly_fw_workspace_bytes (forward; not needed with snapshots) and bfly_layer_bw_workspace_bytes. */
 typedef struct {
   int dtype, base4, batch, nstacks, log_n, nblocks, input_size, output_size, increasing_stride;

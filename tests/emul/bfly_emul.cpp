@@ -140,7 +140,7 @@ struct EmulExec {
         if (q.dbias)  // column sums of the gradient tile as it arrived
           for (int r = 0; r < kBw3Rows; ++r)
             for (int l = 0; l < C; ++l) {
-              const int flat = stack * (1 << q.log_n) + (q.panel.col(pbase, l) & ((1 << q.log_n) - 1));
+              const int flat = stack * (1 << q.log_n) + q.panel.col(pbase, l);
               if (flat < q.dbias_len) q.dbias[flat] += smG[r * C + swz<2>(l)];
             }
         for (int step = 0; step < bw3_num_steps(q.nsg); ++step)

@@ -155,3 +155,17 @@ def test_pipelines_trace_and_vmap(dev, make):
     assert close(traced(other), f(other)) and close(torch.func.vmap(f)(x), f(x))
     with torch.no_grad():
         assert close(torch.func.vmap(f)(x), f(x))
+
+
+@pytest.mark.parametrize("in_size,out_size", [(64, 64), (64, 128), (256, 256), (512, 1024)])
+def test_bias_gradients_of_narrow_rows(dev, in_size, out_size):
+    """Rows that share a tile row, stacks full: the bias gradient has one order there too, and is as close to the float64 sum
+    as PyTorch's own (1.5 for another order of as many additions)."""
+    torch.manual_seed(in_size)
+    layer = _layer("f32", in_size, out_size, dev)
+    batch = (1 << 21) // in_size + 3
+    x, g = torch.randn(batch, in_size, device=dev), torch.randn(batch, out_size, device=dev)
+    first, again = (torch.autograd.grad(layer(x), layer.bias, g)[0] for _ in range(2))
+    want = g.double().sum(0)
+    off = lambda s: ((s.double() - want).norm() / want.norm()).item()
+    assert torch.equal(first, again) and off(first) <= 1.5 * off(g.sum(0))
