@@ -27,6 +27,7 @@ from .permutation import FixedPermutation
 
 
 _glue_fw = torch.ops.torch_butterfly.butterfly_multiply_glue_fw.default
+_is_tracing, _transforms = torch._C._is_tracing, torch._C._functorch.peek_interpreter_stack
 
 
 def _unfused(twiddle, input, increasing_stride, in_perm, out_diag, out_perm, out_real):
@@ -89,7 +90,7 @@ def butterfly_multiply_glue(twiddle: torch.Tensor, input: torch.Tensor, increasi
     if in_perm is not None and width < n:  # the gather would read past the row, which a GPU answers with a lost context
         raise RuntimeError("butterfly_multiply_glue: in_perm needs rows of %d entries, got %d" % (n, width))
     # (a tracer and functorch's transforms see through the links, not through the fused operator's optional result)
-    if n > limit or width > n or not input.is_cuda or torch.jit.is_tracing() or torch._C._functorch.peek_interpreter_stack() is not None:
+    if n > limit or width > n or not input.is_cuda or _is_tracing() or _transforms() is not None:
         return _unfused(twiddle, input, increasing_stride, in_perm, out_diag, out_perm, out_real)
     if not (torch.is_grad_enabled() and (input.requires_grad or twiddle.requires_grad
                                          or (out_diag is not None and out_diag.requires_grad))):
@@ -151,7 +152,7 @@ class ButterflyPipeline(nn.Module):
     def forward(self, input):
         b = self.butterfly
         width = input.shape[-1]
-        if b.in_size == b.n and width != b.n:  # (a narrower layer pads or trims its rows, whole ones take none but their own)
+        if width != b.n and b.in_size == b.n:  # (a narrower layer pads or trims its rows, whole ones take none but their own)
             raise RuntimeError("ButterflyPipeline: rows of %d entries expected, got %d" % (b.n, width))
         rows = input.unsqueeze(1) if input.dim() == 2 else input.reshape(-1, 1, width)
         if not self.real_in and b.complex and not rows.is_complex():
