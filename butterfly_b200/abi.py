@@ -20,6 +20,7 @@ SYMBOLS = (
     "bfly_strerror", "bfly_version", "bfly_cuda_version", "bfly_fw_f32", "bfly_fw_c64", "bfly_fw_workspace_bytes",
     "bfly_bw_workspace_bytes", "bfly_bw_f32", "bfly_bw_c64", "bfly4_fw_f32", "bfly4_bw_workspace_bytes",
     "bfly4_bw_f32", "bfly_launch_count", "bfly_profile_enable", "bfly_profile_collect", "bfly_layer_snapshot_bytes", "bfly_layer_fw",
+    "bfly_bw_snapshot_bytes", "bfly_fw_saving_ws", "bfly_bw_saved_workspace_bytes", "bfly_bw_saved_ws",
     "bfly_layer_bw_workspace_bytes", "bfly_layer_bw", "bfly_bw_f32_noalloc",
     "bfly_linear_fw_f32", "bfly_linear_bw_f32", "bfly_linear_bw_workspace_bytes", "bfly_device_error", "bfly_set_option", "bfly_get_option", "bfly4_fw_c64", "bfly4_bw_c64", "bfly_fw_f32_saving", "bfly_fw_c64_saving", "bfly_bw_f32_saved", "bfly_bw_c64_saved",
     "bfly_unitary_twiddle_fw", "bfly_unitary_twiddle_bw", "bfly_fw_glue_f32", "bfly_fw_glue_c64",
@@ -394,7 +395,8 @@ def device_error():
     return rc
 
 
-KERNEL_NAMES = ("bfly_fw_kernel", "bfly_bw_kernel", "bfly_fw2_kernel", "bfly_bw2_kernel", "bfly_bw3_kernel")
+KERNEL_NAMES = ("bfly_fw_kernel", "bfly_bw_kernel", "bfly_fw2_kernel", "bfly_bw2_kernel", "bfly_bw3_kernel", "bfly_mma_fw_kernel",
+                "bfly_mma_bw_kernel", "bfly_mma_operator_kernels")
 
 
 def profile_enable(on=True):

@@ -18,19 +18,23 @@
 //   static constexpr bool kFusedBias;                      // optional: run_fw adds FwParams::bias itself
 //   int  column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out, float* partial);   // layers: bias gradient
 //   int  stack_sums(const T* g, int64_t B, int S, int64_t n, int cols, T* out);         // layers: sum over the stacks
+//   static constexpr bool kMma;                            // optional: the tensor-core passes (bfly_mma.h) are available:
+//   int  mma_prep(const MmaPrep&, bool cplx); int mma_fw(const MmaPass&); int mma_bw(const MmaPass&, int ctas);
+//   int  mma_post(const MmaPost&, bool cplx);
 #pragma once
 #include <cstdlib>
 #include <cstring>
 
 #include "bfly_bw3.h"
 #include "bfly_fw2.h"
+#include "bfly_mma.h"
 #include "bfly_plan.h"
 
 namespace bfly {
 
 // Development and test switches.  They are read from the environment once, when first used
 // (BFLY_TMA, BFLY_BW_V2, BFLY_FW2, BFLY_FW_KMAX, BFLY_FW_ROWS, BFLY_FW_LOGCMAX, BFLY_BW_ROWS,
-// BFLY_BW_MAXSG, BFLY_AUTOGRAD_SAVE), and can be changed afterwards with set_option() (C ABI: bfly_set_option); the
+// BFLY_BW_MAXSG, BFLY_MMA, BFLY_AUTOGRAD_SAVE), and can be changed afterwards with set_option() (C ABI: bfly_set_option); the
 // launch path itself never touches the environment.  -1 = not set (planner's default).
 struct Options {
   int tma = 1;          // tile traffic through the TMA unit where tensors qualify
@@ -47,6 +51,7 @@ struct Options {
   int bw3_min_rows = 100;  // fewest rows per CTA for which a plain backward phase takes the packed-pair kernel
   int fw_spread = 1;       // few wide rows: narrower panels, so that several CTAs share a row
   int virtual_rows = 1;    // narrow rows of large problems several to a tile row
+  int mma = -1;            // tensor-core passes: 0 never, 1 wherever they can run, -1 by size
   int autograd_save = -1;  // torch autograd operator: keep the forward's snapshots for the backward
 };
 struct OptionName { const char* name; const char* env; int Options::*field; };
@@ -62,6 +67,7 @@ inline const OptionName* option_names(int* count) {
       {"bw3_min_rows", "BFLY_BW3_MIN_ROWS", &Options::bw3_min_rows},
       {"fw_spread", "BFLY_FW_SPREAD", &Options::fw_spread},
       {"virtual_rows", "BFLY_VIRTUAL_ROWS", &Options::virtual_rows},
+      {"mma", "BFLY_MMA", &Options::mma},
       {"autograd_save", "BFLY_AUTOGRAD_SAVE", &Options::autograd_save},
   };
   *count = (int)(sizeof(names) / sizeof(names[0]));
@@ -163,6 +169,7 @@ template <typename T> inline bool vec_ok(const void* p, int64_t sB, int64_t sS) 
 struct Problem {
   int B, S, log_n, nblocks, in_size, out_size;
   bool inc, base4;
+  bool phases = false;  // stay on the phase kernels (bfly_mma.h is not asked)
 };
 
 inline void twiddle_stack_sizes(const Problem& q, int64_t out[2]);
@@ -373,6 +380,178 @@ int drive_fw2_view(E& ex, const Problem& q, const std::vector<Stage>& st, int t0
     if (rc != BFLY_OK) return rc;
   }
   return BFLY_OK;
+}
+
+// ------------------------------------------------------------------ products on the tensor cores (bfly_mma.h)
+
+template <typename E, typename = void> struct has_mma : std::false_type {};
+template <typename E> struct has_mma<E, decltype((void)E::kMma)> : std::true_type {};
+
+// Microseconds of a training step, passes against phases, fitted to measurements of 2^20 to 2^25 floats (f = 1: 2^25).
+// A group costs a forward and a backward pass, an operator its block in the kernels before and after them.  A stage of the
+// phases costs more where rows are complex, wide or (complex) narrow and where factors are radix 4.  Measured, us, phases
+// against passes, in short runs: float 4096 two blocks 2^25 669 : 532, 2^24 371 : 333; float 1024 two blocks 2^25 576 : 510, 2^24
+// 323 : 326; float 4096 one block 383 : 493; float 8192 two blocks (five groups) 815 : 859; radix 4, 16384, 642 : 549;
+// complex 2048 514 : 482, 1024 two blocks 845 : 497, 256 two blocks 1180 : 495, 512 one block with 2^21 123 : 131.
+// Radix-2 floats below 0.75 2^25 stay on the phases altogether: little to gain, and a forward that records keeps the bits
+// of one that does not.  The margin: under the power cap (runs above 0.1 s) the clock falls to 1.65 GHz with the passes and
+// stays at 1.96 with the phases (complex 2048: 535 against 514 then).  (Forward-only calls stay there at any size: the packed-pair kernel keeps rows on chip.)
+inline bool mma_pays(const Problem& q, int F, int ng) {
+  if (q.B < 512) return false;  // an operator meets too few rows
+  const double f = (double)((int64_t)q.B * q.S << (q.log_n + F)) / (1 << 25), w = (double)q.nblocks * q.log_n;
+  const double passes = 35 + 0.08 * ng * (double)((int64_t)q.S << (q.log_n + F - kMmaWin)) + ng * (17 + 128 * f);
+  double phases;
+  if (F) phases = q.log_n <= 9 ? 60 + 70 * w * f : 90 + 38.5 * w * f;
+  else if (q.base4) phases = q.log_n <= 12 ? 75 + 30 * w * f : 65 + 38 * w * f;
+  else phases = f < 0.75 ? 0 : 45 + 25 * w * f;
+  return passes * 1.12 < phases;
+}
+
+// Does a training step of this shape run as tensor-core passes, and how?  Only shapes and the option decide, so that a
+// backward finds the planes its forward left.
+template <typename T> inline bool mma_layout(const Problem& q, MmaLayout& L) {
+  const int opt = options().mma;
+  if (opt == 0 || q.phases || q.B < 1 || q.log_n > 15) return false;
+  L.F = sizeof(T) == 8 ? 1 : 0;
+  L.log_nf = q.log_n + L.F;
+  if (L.log_nf < kMmaWin) return false;
+  // products that the backward runs as one phase need no planes there
+  if ((int64_t)q.nblocks * q.log_n <= 8) return false;
+  // (the fewest groups there can be: most small calls need no plan to be turned away)
+  if (opt < 0 && !mma_pays(q, L.F, (q.nblocks * q.log_n + kMmaMaxStages - 1) / kMmaMaxStages)) return false;
+  if (!mma_groups(problem_stages(q), L.F, q.log_n, L.g)) return false;
+  L.nq = 1 << (L.log_nf - kMmaWin);
+  L.nt = ((int64_t)q.B + kMmaRows - 1) / kMmaRows;
+  if (L.nt * L.nq * q.S >= ((int64_t)1 << 30)) return false;
+  // ends in pieces below a sector: 2 to 4 times a pass
+  if (opt < 0 && (std::min(L.g.front().geo.ib, L.g.back().geo.ib) < 3 || !mma_pays(q, L.F, (int)L.g.size()))) return false;
+  const size_t ng = L.g.size(), slots = (size_t)q.S * L.nq + kMmaBwMaxCtas;
+  L.plane = (((size_t)q.S * kMmaRows * sizeof(float)) << L.log_nf) * L.nt;
+  L.images = ng * q.S * L.nq * kMmaImageBytes;
+  L.slots = ng * slots * kMmaSlotFloats * sizeof(float);
+  L.bias_slots = slots * kMmaCols * sizeof(float);
+  return true;
+}
+// The layout of either direction of a problem, for queries that do not name one: the larger need.
+template <typename T, typename F> inline int64_t mma_either(Problem q, F&& bytes) {
+  int64_t best = 0;
+  for (int inc = 0; inc < 2; ++inc) {
+    q.inc = inc != 0;
+    MmaLayout L;
+    if (mma_layout<T>(q, L)) best = std::max<int64_t>(best, (int64_t)bytes(L));
+  }
+  return best;
+}
+
+// The caller's rows as the passes see them (floats).
+template <typename T> inline MmaRowsIO mma_rows(const T* p, int64_t sB, int64_t sS, int cols, int S, int flat = 0) {
+  constexpr int F = (int)(sizeof(T) / 4);
+  MmaRowsIO r;
+  r.p = const_cast<float*>(reinterpret_cast<const float*>(p));
+  r.sB = sB * F; r.sS = S > 1 ? sS * F : 0; r.cols = cols * F; r.flat = flat * F;
+  const uint64_t bits = (uint64_t)reinterpret_cast<uintptr_t>(p) | (uint64_t)(r.sB * 4) | (uint64_t)(r.sS * 4);
+  r.align = bits % 32 == 0 ? 32 : bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : 4;
+  return r;
+}
+
+// Planes are read 32 bytes at a time; buffers of 16-byte alignment, which the phases ask for, have 16 bytes to spare.
+constexpr size_t kMmaSpare = 16;
+inline char* mma_align(void* p, size_t& bytes) {
+  const size_t skip = (32 - (reinterpret_cast<uintptr_t>(p) & 31)) & 31;
+  if (!p || skip > bytes || !aligned16(p)) return nullptr;
+  bytes -= skip;
+  return static_cast<char*>(p) + skip;
+}
+
+template <typename T, typename E>
+int mma_run_prep(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, const T* tw4, uint8_t* images) {
+  MmaPrep p;
+  std::memset(&p, 0, sizeof(p));
+  p.tw[0] = tw2; p.tw[1] = tw4;
+  twiddle_stack_sizes(q, p.tw_stack);
+  p.S = q.S; p.nq = L.nq; p.ng = (int)L.g.size();
+  p.images = images;
+  for (int i = 0; i < p.ng; ++i) p.g[i] = L.g[i];
+  return ex.mma_prep(p, sizeof(T) == 8);
+}
+
+inline MmaPass mma_pass(const Problem& q, const MmaLayout& L, int g, const uint8_t* images) {
+  MmaPass p;
+  std::memset(&p, 0, sizeof(p));
+  p.geo = L.g[g].geo;
+  p.S = q.S; p.B = q.B; p.nq = L.nq; p.nt = (int)L.nt;
+  p.images = images + (size_t)g * q.S * L.nq * kMmaImageBytes;
+  return p;
+}
+
+// Forward; the activations between the groups stay in `kept`, then the operators.  Groups [0, last_group) only when the
+// output is not wanted.
+template <typename T, typename E>
+int drive_mma_fw(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, const T* tw4, const T* x, int64_t x_sB, int64_t x_sS, T* out, int out_cols,
+                 const T* bias, int bias_len, char* kept) {
+  constexpr int F = (int)(sizeof(T) / 4);
+  const int64_t n = (int64_t)1 << q.log_n;
+  const int ng = (int)L.g.size();
+  uint8_t* images = reinterpret_cast<uint8_t*>(kept) + (ng - 1) * L.plane;
+  if (int rc = mma_run_prep(ex, q, L, tw2, tw4, images)) return rc;
+  for (int g = 0; g < (out ? ng : ng - 1); ++g) {
+    MmaPass p = mma_pass(q, L, g, images);
+    if (g == 0) p.in = mma_rows<T>(x, x_sB, x_sS, q.in_size, q.S);
+    else p.in_t = reinterpret_cast<const float*>(kept + (g - 1) * L.plane);
+    if (g + 1 < ng) {
+      p.out_t = reinterpret_cast<float*>(kept + g * L.plane);
+    } else {
+      p.out = mma_rows<T>(out, (int64_t)q.S * n, n, out_cols, q.S);
+      p.bias = reinterpret_cast<const float*>(bias); p.bias_len = bias ? bias_len * F : 0;
+    }
+    if (int rc = ex.mma_fw(p)) return rc;
+  }
+  return BFLY_OK;
+}
+
+// Backward.  dx: rows of the input gradient, added to when `reduce`; d_bias (column sums of the gradient) may be null.
+// `kept`: what the forward left, untouched here, or null.
+template <typename T, typename E>
+int drive_mma_bw(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, const T* tw4, const T* x, int64_t x_sB, int64_t x_sS, const MmaRowsIO& grad,
+                 const MmaRowsIO& dx, bool reduce, T* d_tw2, T* d_tw4, T* d_bias, int bias_len, const char* kept, char* ws, size_t ws_bytes) {
+  constexpr int F = (int)(sizeof(T) / 4);
+  if (ws_bytes < L.bw_bytes(kept != nullptr)) return BFLY_E_WORKSPACE;
+  const int ng = (int)L.g.size();
+  const size_t slots_per_group = (size_t)q.S * L.nq + kMmaBwMaxCtas;
+  char* gplane = ws;
+  float* slots = reinterpret_cast<float*>(ws + (kept ? (ng > 1 ? L.plane : 0) : L.kept()));
+  float* bias_slots = reinterpret_cast<float*>(reinterpret_cast<char*>(slots) + L.slots);
+  if (!kept) {
+    if (int rc = drive_mma_fw<T>(ex, q, L, tw2, tw4, x, x_sB, x_sS, (T*)nullptr, 0, (const T*)nullptr, 0, ws)) return rc;
+    kept = ws;
+    if (ng > 1) gplane = ws + (ng - 2) * L.plane;  // a tile's activations are read before its gradient is written
+  }
+  const uint8_t* images = reinterpret_cast<const uint8_t*>(kept) + (ng - 1) * L.plane;
+  const int ctas = (int)std::min<int64_t>(std::min(ex.num_sms(), kMmaBwMaxCtas), (int64_t)q.S * L.nq * L.nt);
+  for (int g = ng - 1; g >= 0; --g) {
+    MmaPass p = mma_pass(q, L, g, images);
+    if (g == ng - 1) {
+      p.in = grad;
+      if (d_bias) p.bias_slots = bias_slots;
+    } else {
+      p.in_t = reinterpret_cast<const float*>(gplane);
+    }
+    if (g == 0) p.x = mma_rows<T>(x, x_sB, x_sS, q.in_size, q.S);
+    else p.x_t = reinterpret_cast<const float*>(kept + (g - 1) * L.plane);
+    if (g == 0) { p.out = dx; p.reduce = reduce; }
+    else p.out_t = reinterpret_cast<float*>(gplane);
+    p.slots = slots + (size_t)g * slots_per_group * kMmaSlotFloats;
+    if (int rc = ex.mma_bw(p, ctas)) return rc;
+  }
+  MmaPost p;
+  std::memset(&p, 0, sizeof(p));
+  p.tw[0] = tw2; p.tw[1] = tw4; p.dtw[0] = d_tw2; p.dtw[1] = d_tw4;
+  twiddle_stack_sizes(q, p.tw_stack);
+  p.S = q.S; p.nq = L.nq; p.nt = (int)L.nt; p.ng = ng; p.ctas = ctas; p.last_group = ng - 1;
+  p.slots = slots; p.slots_group = (int64_t)slots_per_group * kMmaSlotFloats;
+  if (d_bias) { p.bias_slots = bias_slots; p.dbias = reinterpret_cast<float*>(d_bias); p.dbias_len = bias_len * F; }
+  for (int i = 0; i < ng; ++i) p.g[i] = L.g[i];
+  return ex.mma_post(p, sizeof(T) == 8);
 }
 
 // Run stages [t0, t1) of the product with the row-owner forward kernel.  `cuts` lists the
@@ -587,6 +766,14 @@ int drive_fw_saving(E& ex, const Problem& q, const T* tw2, const T* tw4, const T
   if (!x || !out || twiddle_missing(q, tw2, tw4)) return BFLY_E_ARG;
   if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4))) return BFLY_E_ALIGN;
   if (!rows_aligned<T>(x) || !rows_aligned<T>(out)) return BFLY_E_ALIGN;
+  if constexpr (has_mma<E>::value) {
+    MmaLayout L;
+    if (mma_layout<T>(q, L)) {
+      char* kept = mma_align(ws, ws_bytes);
+      if (!kept || ws_bytes < L.kept()) return BFLY_E_WORKSPACE;
+      return drive_mma_fw<T>(ex, q, L, tw2, tw4, x, x_sB, x_sS, out, q.out_size, (const T*)nullptr, 0, kept);
+    }
+  }
   BwLayout<T> lay;
   rc = plan_bw<T>(q, lay);
   if (rc != BFLY_OK) return rc;
@@ -610,11 +797,12 @@ int drive_fw_saving(E& ex, const Problem& q, const T* tw2, const T* tw4, const T
 }
 
 // Backward of the whole product.  d_x is (B, S, max(in_size, n)) contiguous and doubles as
-// the gradient buffer between phases; d_tw2 / d_tw4 are overwritten.
+// the gradient buffer between phases; d_tw2 / d_tw4 are overwritten.  `extra`: work space next to saved snapshots, which
+// the tensor-core passes need.
 template <typename T, typename E>
 int drive_bw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T* x, int64_t x_sB, int64_t x_sS,
              const T* grad, int64_t g_sB, int64_t g_sS, T* d_tw2, T* d_tw4, T* d_x, void* ws,
-             size_t ws_bytes, bool snapshots_ready = false, int gin_flat = 0) {
+             size_t ws_bytes, bool snapshots_ready = false, int gin_flat = 0, void* extra = nullptr, size_t extra_bytes = 0) {
   int rc = check_problem(q);
   if (rc != BFLY_OK) return rc;
   int64_t stk[2];
@@ -622,6 +810,23 @@ int drive_bw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T* x, in
   if ((stk[0] && (!tw2 || !d_tw2)) || (stk[1] && (!tw4 || !d_tw4))) return BFLY_E_ARG;
   if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4))) return BFLY_E_ALIGN;
   if ((d_tw2 && !aligned16(d_tw2)) || (d_tw4 && !aligned16(d_tw4))) return BFLY_E_ALIGN;  // 16-byte vector reductions
+  if constexpr (has_mma<E>::value) {
+    MmaLayout L;
+    if (mma_layout<T>(q, L)) {
+      if (!x || !grad || !d_x) return BFLY_E_ARG;
+      if (!rows_aligned<T>(x) || !rows_aligned<T>(grad) || !rows_aligned<T>(d_x)) return BFLY_E_ALIGN;
+      size_t work_bytes = snapshots_ready ? extra_bytes : ws_bytes;
+      char* work = mma_align(snapshots_ready ? extra : ws, work_bytes);
+      const char* kept = snapshots_ready ? mma_align(ws, ws_bytes) : nullptr;
+      if (!work || (snapshots_ready && (!kept || ws_bytes < L.kept()))) return BFLY_E_WORKSPACE;
+      const int64_t n = (int64_t)1 << q.log_n, DX = std::max<int64_t>(q.in_size, n);
+      rc = drive_mma_bw<T>(ex, q, L, tw2, tw4, x, x_sB, x_sS, mma_rows<T>(grad, g_sB, g_sS, q.out_size, q.S, gin_flat),
+                           mma_rows<T>(d_x, (int64_t)q.S * DX, DX, (int)std::min<int64_t>(q.in_size, n), q.S), false, d_tw2, d_tw4, (T*)nullptr, 0,
+                           kept, work, work_bytes);
+      if (rc != BFLY_OK || q.in_size <= n) return rc;
+      return ex.zero2d(d_x + n, (size_t)DX * sizeof(T), (size_t)(q.in_size - n) * sizeof(T), (size_t)q.B * q.S);
+    }
+  }
   if (stk[0]) { rc = ex.zero(d_tw2, (size_t)q.S * stk[0] * sizeof(T)); if (rc) return rc; }
   if (stk[1]) { rc = ex.zero(d_tw4, (size_t)q.S * stk[1] * sizeof(T)); if (rc) return rc; }
   if (q.B == 0) return BFLY_OK;
@@ -786,6 +991,14 @@ int drive_layer_fw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T*
   const std::vector<Stage> st = problem_stages(q);
   const int64_t n = (int64_t)1 << q.log_n;
   if (ws && !aligned16(ws)) ws = nullptr;
+  if constexpr (has_mma<E>::value) {
+    MmaLayout M;
+    if (snapshots && out_total > 0 && mma_layout<T>(q, M)) {
+      char* kept = mma_align(snapshots, snapshot_bytes);
+      if (!kept || snapshot_bytes < M.kept()) return BFLY_E_WORKSPACE;
+      return drive_mma_fw<T>(ex, q, M, tw2, tw4, x, x_sB, 0, out, (int)n, bias, out_total, kept);
+    }
+  }
   T* snaps[kMaxSnap] = {nullptr};
   std::vector<int> cuts;
   if (snapshots) {
@@ -977,6 +1190,40 @@ int plan_layer_bw(const Problem& q, int out_total, bool saved, LayerBwLayout& L)
   return BFLY_OK;
 }
 
+// The tensor-core route of a layer's backward: like the fused one it adds the stacks' input gradients up in the last
+// pass where the layer is one of full-width stacks; elsewhere they go through rows of their own and one pass more.
+template <typename T> inline bool mma_layer_adds(const Problem& q, int out_total) {
+  return sizeof(T) == 4 && !q.base4 && q.S > 1 && out_total == ((int64_t)q.S << q.log_n) && q.in_size <= 1 << q.log_n && q.in_size % 32 == 0;
+}
+template <typename T> inline size_t mma_layer_bw_bytes(const Problem& q, int out_total, const MmaLayout& M, bool saved) {
+  const int64_t DX = std::max<int64_t>(q.in_size, (int64_t)1 << q.log_n);
+  return M.bw_bytes(saved) + (q.S > 1 && !mma_layer_adds<T>(q, out_total) ? (size_t)q.B * q.S * DX * sizeof(T) : 0);
+}
+template <typename T, typename E>
+int drive_mma_layer_bw(E& ex, const Problem& q, const MmaLayout& M, const T* tw2, const T* tw4, const T* x, int64_t x_sB, const T* grad, int64_t g_sB,
+                       T* d_tw2, T* d_tw4, T* d_in, T* d_bias, int out_total, void* saved, size_t saved_bytes, void* ws, size_t ws_bytes) {
+  char* work = mma_align(ws, ws_bytes);
+  if (!work || ws_bytes < mma_layer_bw_bytes<T>(q, out_total, M, saved != nullptr)) return BFLY_E_WORKSPACE;
+  const char* kept = saved ? mma_align(saved, saved_bytes) : nullptr;
+  if (saved && (!kept || saved_bytes < M.kept())) return BFLY_E_WORKSPACE;
+  const int64_t n = (int64_t)1 << q.log_n, DX = std::max<int64_t>(q.in_size, n);
+  const int cols = (int)std::min<int64_t>(q.in_size, n);
+  const bool adds = mma_layer_adds<T>(q, out_total);
+  const size_t own = M.bw_bytes(saved != nullptr);
+  T* rows = q.S > 1 && !adds ? reinterpret_cast<T*>(work + own) : d_in;
+  MmaRowsIO dx = adds ? mma_rows<T>(d_in, q.in_size, 0, cols, 1) : mma_rows<T>(rows, (int64_t)q.S * DX, DX, cols, q.S);
+  if (adds)
+    if (int rc = ex.zero(d_in, (size_t)q.B * q.in_size * sizeof(T))) return rc;
+  int rc = drive_mma_bw<T>(ex, q, M, tw2, tw4, x, x_sB, 0, mma_rows<T>(grad, g_sB, n, (int)n, q.S, out_total), dx, adds, d_tw2, d_tw4, d_bias, out_total,
+                           kept, work, own);
+  if (rc != BFLY_OK) return rc;
+  if (q.in_size > n) {  // columns beyond n have no gradient
+    rc = ex.zero2d(rows + n, (size_t)DX * sizeof(T), (size_t)(q.in_size - n) * sizeof(T), (size_t)q.B * q.S);
+    if (rc != BFLY_OK) return rc;
+  }
+  return q.S > 1 && !adds ? ex.stack_sums(rows, q.B, q.S, DX, q.in_size, d_in) : BFLY_OK;
+}
+
 template <typename T, typename E>
 int drive_layer_bw(E& ex, const Problem& q_in, const T* tw2, const T* tw4, const T* x, int64_t x_sB, const T* grad, int64_t g_sB,
                    T* d_tw2, T* d_tw4, T* d_in, T* d_bias, int out_total, void* saved, size_t saved_bytes, void* ws, size_t ws_bytes) {
@@ -988,6 +1235,17 @@ int drive_layer_bw(E& ex, const Problem& q_in, const T* tw2, const T* tw4, const
   if (out_total < 0 || out_total > q.S * n) return BFLY_E_ARG;
   if (q.B > 0 && (!x || !d_in || (out_total > 0 && !grad))) return BFLY_E_ARG;
   if (!rows_aligned<T>(x) || !rows_aligned<T>(grad) || !rows_aligned<T>(d_in)) return BFLY_E_ALIGN;
+  if constexpr (has_mma<E>::value) {
+    MmaLayout M;
+    if (out_total > 0 && mma_layout<T>(q, M)) {
+      int64_t stk[2];
+      twiddle_stack_sizes(q, stk);
+      if (twiddle_missing(q, tw2, tw4) || (stk[0] && !d_tw2) || (stk[1] && !d_tw4)) return BFLY_E_ARG;
+      if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4)) || (d_tw2 && !aligned16(d_tw2)) || (d_tw4 && !aligned16(d_tw4))) return BFLY_E_ALIGN;
+      return drive_mma_layer_bw<T>(ex, q, M, tw2, tw4, x, x_sB, grad, g_sB, d_tw2, d_tw4, d_in, d_bias, out_total, saved, saved_bytes, ws, ws_bytes);
+    }
+  }
+  q.phases = true;  // as the forward went, and as the work space is laid out
   LayerBwLayout L;
   rc = plan_layer_bw<T>(q, out_total, saved != nullptr, L);
   if (rc != BFLY_OK) return rc;

@@ -7,6 +7,7 @@
 
 #include "bfly_bw3.h"
 #include "bfly_fw2.h"
+#include "bfly_mma.h"
 
 namespace bfly {
 
@@ -30,6 +31,12 @@ int stack_sums_launch(const float* g, int64_t B, int S, int64_t n, int cols, flo
 // in, gradient out) describe boxes of kBw3Rows rows of the phase's panel (bfly_tma.h).
 int bw3_launch(const Bw3Params& p, const CUtensorMap& mx, const CUtensorMap& mg, const CUtensorMap& mo, cudaStream_t stream,
                int* err);
+
+// The kernels of bfly_mma.h.  `err` as for fw2_launch.
+int mma_prep_launch(const MmaPrep& p, bool cplx, cudaStream_t stream);
+int mma_fw_launch(const MmaPass& p, int sms, cudaStream_t stream, int* err);
+int mma_bw_launch(const MmaPass& p, int ctas, cudaStream_t stream, int* err);
+int mma_post_launch(const MmaPost& p, bool cplx, cudaStream_t stream, int* launches);
 
 // Adds to the count that bfly_launch_count reports (kernels launched by the other translation units).
 void count_launches(int n);

@@ -479,7 +479,7 @@ void count_launches(int n) { g_launches.fetch_add(n); }
 
 // Optional per-launch timing (bfly_profile_*): while enabled, every kernel launch is
 // bracketed by a pair of CUDA events on the launching stream.
-enum KernelId : int { kKernFw = 0, kKernBw = 1, kKernFw2 = 2, kKernBw2 = 3, kKernBw3 = 4, kNumKernelIds = 5 };
+enum KernelId : int { kKernFw = 0, kKernBw = 1, kKernFw2 = 2, kKernBw2 = 3, kKernBw3 = 4, kKernMmaFw = 5, kKernMmaBw = 6, kKernMmaOps = 7, kNumKernelIds = 8 };
 struct ProfileRec { int id; cudaEvent_t a, b; };
 static std::mutex g_prof_mu;
 static bool g_prof_on = false;
@@ -763,6 +763,27 @@ struct CudaExec {
     if (rc == BFLY_OK) g_launches.fetch_add(1);
     return rc;
   }
+  static constexpr bool kMma = true;
+  template <typename F> int mma_launch(int id, F&& launch) {
+    int* err = nullptr;
+    int rc = device_error_ptr(&err);
+    if (rc) return rc;
+    {
+      ProfileScope prof(id, stream);
+      rc = launch(err);
+    }
+    if (rc == BFLY_OK) g_launches.fetch_add(1);
+    return rc;
+  }
+  int mma_prep(const MmaPrep& p, bool cplx) { return mma_launch(kKernMmaOps, [&](int*) { return mma_prep_launch(p, cplx, stream); }); }
+  int mma_fw(const MmaPass& p) { return mma_launch(kKernMmaFw, [&](int* err) { return mma_fw_launch(p, dev.sms, stream, err); }); }
+  int mma_bw(const MmaPass& p, int ctas) { return mma_launch(kKernMmaBw, [&](int* err) { return mma_bw_launch(p, ctas, stream, err); }); }
+  int mma_post(const MmaPost& p, bool cplx) {
+    int launches = 0;
+    const int rc = mma_launch(kKernMmaOps, [&](int*) { return mma_post_launch(p, cplx, stream, &launches); });
+    g_launches.fetch_add(std::max(launches - 1, 0));
+    return rc;
+  }
   int zero(void* ptr, size_t bytes) {
     if (bytes == 0) return BFLY_OK;
     return cudaMemsetAsync(ptr, 0, bytes, stream) == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
@@ -812,11 +833,11 @@ static int fw_glue_entry(const void* tw, const void* x, int x_is_real, int64_t x
 template <typename T>
 static int fw_saving_entry(const void* tw2, const void* x, int64_t x_sB, int64_t x_sS, void* out, int B, int S,
                            int log_n, int nblocks, int in_size, int out_size, int inc, void* ws, size_t ws_bytes,
-                           void* stream) {
+                           void* stream, bool phases) {
   CudaExec ex;
   int rc = make_exec(stream, ex);
   if (rc) return rc;
-  Problem q{B, S, log_n, nblocks, in_size, out_size, inc != 0, false};
+  Problem q{B, S, log_n, nblocks, in_size, out_size, inc != 0, false, phases};
   return drive_fw_saving<T>(ex, q, static_cast<const T*>(tw2), static_cast<const T*>(nullptr),
                             static_cast<const T*>(x), x_sB, x_sS, static_cast<T*>(out), ws, ws_bytes);
 }
@@ -825,14 +846,14 @@ template <typename T>
 static int bw_entry(bool base4, const void* tw2, const void* tw4, const void* x, int64_t x_sB, int64_t x_sS,
                     const void* grad, int64_t g_sB, int64_t g_sS, void* d2, void* d4, void* dx, int B, int S,
                     int log_n, int nblocks, int in_size, int out_size, int inc, void* ws, size_t ws_bytes,
-                    void* stream, bool snapshots_ready = false) {
+                    void* stream, bool snapshots_ready = false, void* extra = nullptr, size_t extra_bytes = 0, bool phases = false) {
   CudaExec ex;
   int rc = make_exec(stream, ex);
   if (rc) return rc;
-  Problem q{B, S, log_n, nblocks, in_size, out_size, inc != 0, base4};
+  Problem q{B, S, log_n, nblocks, in_size, out_size, inc != 0, base4, phases};
   return drive_bw<T>(ex, q, static_cast<const T*>(tw2), static_cast<const T*>(tw4), static_cast<const T*>(x),
                      x_sB, x_sS, static_cast<const T*>(grad), g_sB, g_sS, static_cast<T*>(d2),
-                     static_cast<T*>(d4), static_cast<T*>(dx), ws, ws_bytes, snapshots_ready);
+                     static_cast<T*>(d4), static_cast<T*>(dx), ws, ws_bytes, snapshots_ready, 0, extra, extra_bytes);
 }
 
 template <typename T>
@@ -847,7 +868,18 @@ static int64_t ws_for(const Problem& q0) {
     if (rc) return rc;
     best = std::max<int64_t>(best, (int64_t)lay.ws_bytes);
   }
-  return best;
+  // tensor-core passes: at least a plane per group, like the phases with the forward's scratch behind it
+  return std::max(best, mma_either<T>(q0, [&](const MmaLayout& L) {
+    return std::max(L.bw_bytes(false) + kMmaSpare, L.g.size() * L.plane) + (q0.base4 ? 0 : fw_workspace_bytes<T>(q0));
+  }));
+}
+// What a saving forward has to leave for the backward.
+template <typename T>
+static int64_t kept_for(const Problem& q0) {
+  const int64_t kept = mma_either<T>(q0, [](const MmaLayout& L) { return L.kept() + kMmaSpare; });
+  Problem q = q0;
+  q.phases = true;
+  return kept > 0 ? kept : ws_for<T>(q);
 }
 
 // f(element of the layer's type, problem)
@@ -1058,6 +1090,8 @@ int bfly_linear_bw_f32(const float* twiddle, const float* x, int64_t x_sB, const
 int64_t bfly_layer_snapshot_bytes(const bfly_layer_t* l) {
   if (!l) return BFLY_E_ARG;
   return layer_call(l, [&](auto t, const Problem& q) -> int64_t {
+    MmaLayout M;
+    if (l->output_size > 0 && mma_layout<decltype(t)>(q, M)) return (int64_t)(M.kept() + kMmaSpare);
     BwLayout<decltype(t)> lay;
     const int rc = plan_bw<decltype(t)>(q, lay);
     return rc ? rc : (lay.chunked ? 0 : (int64_t)lay.ws_bytes);
@@ -1078,6 +1112,8 @@ int bfly_layer_fw(const bfly_layer_t* l, const void* twiddle2, const void* twidd
 int64_t bfly_layer_bw_workspace_bytes(const bfly_layer_t* l, int with_snapshots) {
   if (!l) return BFLY_E_ARG;
   return layer_call(l, [&](auto t, const Problem& q) -> int64_t {
+    MmaLayout M;
+    if (l->output_size > 0 && mma_layout<decltype(t)>(q, M)) return (int64_t)(mma_layer_bw_bytes<decltype(t)>(q, l->output_size, M, with_snapshots != 0) + kMmaSpare);
     LayerBwLayout L;
     const int rc = plan_layer_bw<decltype(t)>(q, l->output_size, with_snapshots != 0, L);
     return rc ? rc : (int64_t)L.ws_bytes;
@@ -1101,13 +1137,13 @@ int bfly_fw_f32_saving(const float* twiddle, const float* x, int64_t x_sB, int64
                        int nstacks, int log_n, int nblocks, int input_size, int output_size, int increasing_stride,
                        void* snapshots, size_t snapshot_bytes, void* stream) {
   return fw_saving_entry<float>(twiddle, x, x_sB, x_sS, out, batch, nstacks, log_n, nblocks, input_size, output_size,
-                                increasing_stride, snapshots, snapshot_bytes, stream);
+                                increasing_stride, snapshots, snapshot_bytes, stream, true);
 }
 int bfly_fw_c64_saving(const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, void* out, int batch,
                        int nstacks, int log_n, int nblocks, int input_size, int output_size, int increasing_stride,
                        void* snapshots, size_t snapshot_bytes, void* stream) {
   return fw_saving_entry<cf>(twiddle, x, x_sB, x_sS, out, batch, nstacks, log_n, nblocks, input_size, output_size,
-                             increasing_stride, snapshots, snapshot_bytes, stream);
+                             increasing_stride, snapshots, snapshot_bytes, stream, true);
 }
 int bfly_bw_f32_saved(const float* twiddle, const float* x, int64_t x_sB, int64_t x_sS, const float* grad,
                       int64_t g_sB, int64_t g_sS, float* d_twiddle, float* d_x, int batch, int nstacks, int log_n,
@@ -1124,6 +1160,44 @@ int bfly_bw_c64_saved(const void* twiddle, const void* x, int64_t x_sB, int64_t 
   return bw_entry<cf>(false, twiddle, nullptr, x, x_sB, x_sS, grad, g_sB, g_sS, d_twiddle, nullptr, d_x, batch,
                       nstacks, log_n, nblocks, input_size, output_size, increasing_stride, snapshots, snapshot_bytes,
                       stream, true);
+}
+int64_t bfly_bw_snapshot_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks) {
+  Problem q{batch, nstacks, log_n, nblocks, 1, 1, true, false};
+  const int rc = check_problem(q);
+  if (rc) return rc;
+  if (dtype == BFLY_F32) return kept_for<float>(q);
+  if (dtype == BFLY_C64) return kept_for<cf>(q);
+  return BFLY_E_UNSUPPORTED;
+}
+int bfly_fw_saving_ws(int dtype, const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, void* out, int batch, int nstacks, int log_n,
+                      int nblocks, int input_size, int output_size, int increasing_stride, void* snapshots, size_t snapshot_bytes, void* stream) {
+  if (dtype == BFLY_F32)
+    return fw_saving_entry<float>(twiddle, x, x_sB, x_sS, out, batch, nstacks, log_n, nblocks, input_size, output_size, increasing_stride, snapshots,
+                                  snapshot_bytes, stream, false);
+  if (dtype == BFLY_C64)
+    return fw_saving_entry<cf>(twiddle, x, x_sB, x_sS, out, batch, nstacks, log_n, nblocks, input_size, output_size, increasing_stride, snapshots,
+                               snapshot_bytes, stream, false);
+  return BFLY_E_UNSUPPORTED;
+}
+int bfly_bw_saved_ws(int dtype, const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, const void* grad, int64_t g_sB, int64_t g_sS,
+                     void* d_twiddle, void* d_x, int batch, int nstacks, int log_n, int nblocks, int input_size, int output_size,
+                     int increasing_stride, void* snapshots, size_t snapshot_bytes, void* workspace, size_t workspace_bytes, void* stream) {
+  if (dtype == BFLY_F32)
+    return bw_entry<float>(false, twiddle, nullptr, x, x_sB, x_sS, grad, g_sB, g_sS, d_twiddle, nullptr, d_x, batch, nstacks, log_n, nblocks,
+                           input_size, output_size, increasing_stride, snapshots, snapshot_bytes, stream, true, workspace, workspace_bytes);
+  if (dtype == BFLY_C64)
+    return bw_entry<cf>(false, twiddle, nullptr, x, x_sB, x_sS, grad, g_sB, g_sS, d_twiddle, nullptr, d_x, batch, nstacks, log_n, nblocks,
+                        input_size, output_size, increasing_stride, snapshots, snapshot_bytes, stream, true, workspace, workspace_bytes);
+  return BFLY_E_UNSUPPORTED;
+}
+int64_t bfly_bw_saved_workspace_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks) {
+  Problem q{batch, nstacks, log_n, nblocks, 1, 1, true, false};
+  const int rc = check_problem(q);
+  if (rc) return rc;
+  auto bytes = [](const MmaLayout& L) { return L.bw_bytes(true) + kMmaSpare; };
+  if (dtype == BFLY_F32) return mma_either<float>(q, bytes);
+  if (dtype == BFLY_C64) return mma_either<cf>(q, bytes);
+  return BFLY_E_UNSUPPORTED;
 }
 int bfly_bw_f32_noalloc(const float* twiddle, const float* x, int64_t x_sB, int64_t x_sS, const float* grad,
                         int64_t g_sB, int64_t g_sS, float* d_twiddle, float* d_x, int batch, int nstacks, int log_n,
@@ -1143,7 +1217,7 @@ int bfly_bw_f32_noalloc(const float* twiddle, const float* x, int64_t x_sB, int6
   }
   return bw_entry<float>(false, twiddle, nullptr, x, x_sB, x_sS, grad, g_sB, g_sS, d_twiddle, nullptr, d_x,
                          batch, nstacks, log_n, nblocks, input_size, output_size, increasing_stride, scratch,
-                         lay.ws_bytes, stream);
+                         lay.ws_bytes, stream, false, nullptr, 0, true);
 }
 int bfly4_fw_f32(const float* twiddle4, const float* twiddle2, const float* x, int64_t x_sB, int64_t x_sS,
                  float* out, int batch, int nstacks, int log_n, int nblocks, int input_size, int output_size,

@@ -1,0 +1,187 @@
+// Butterfly products of large problems as matrix products on the tensor cores (tcgen05).
+//
+// The stages of a product are cut into groups whose column bits fit a window of six bits.  Inside a window the
+// stages of a group, twelve of them where two blocks meet at their turning point, are ONE dense 64 x 64 matrix per
+// block of 64 columns ("operator").  A pass multiplies tiles of 128 rows by these operators; the backward multiplies the
+// gradient by the transposed operator and accumulates the gradient of the whole operator, g^T x over the rows, which
+// a small kernel takes apart into the gradients of the stages afterwards.  Per pass a tile crosses shared memory once,
+// whatever the number of stages, and the operators' arithmetic costs a quarter of the tile's trip through HBM.
+//
+// Precision.  A float32 value is the exact sum of three bfloat16 values (8 + 8 + 8 bits); products are formed from the
+// six pairs above 2^-24 and summed in float32, the largest apart from the others.  Operators are multiplied out in
+// float64.  tcgen05 truncates its sums: the mean of that loss is added back (kMmaTrunc*).
+//
+// Columns are counted in floats here: complex rows are rows of 2n floats whose bit 0 tells real from imaginary parts,
+// always inside the window, and a complex operator of 32 x 32 is a real one of 64 x 64.
+//
+// Between passes rows live in planes of their own layout, (stack, row tile, column, 128 rows): every column of a tile
+// is 512 contiguous bytes, so that a window of any column bits is read and written in long runs.  Only the first read
+// and the last write of a product see the caller's rows; groups at the ends keep the low column bits in the window.
+//
+// This header: planning and parameter blocks, plain C++.  Kernels: bfly_mma.cu.
+#pragma once
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "bfly_plan.h"
+
+namespace bfly {
+
+constexpr int kMmaWin = 6;                    // bits of a window: operators are 64 x 64
+constexpr int kMmaCols = 1 << kMmaWin;
+constexpr int kMmaRows = 128;                 // rows of a tile (the lanes of tensor memory)
+constexpr int kMmaMaxStages = 12;             // radix-2 stages a group may hold (a radix-4 factor counts as two)
+constexpr int kMmaMaxGroups = 8;
+constexpr int kMmaImageBytes = 3 * kMmaCols * kMmaCols * 2;  // one operator: three bfloat16 slices, swizzled as tcgen05 reads them
+constexpr int kMmaBwMaxCtas = 160;            // most CTAs of a backward pass (one per SM)
+constexpr int kMmaSlotFloats = 2 * kMmaCols * kMmaCols;      // an operator gradient as a CTA leaves it: two halves to be added
+struct MmaStage {
+  uint32_t tw_off;       // element offset of the factor's twiddles inside one stack
+  uint8_t lbit, gbit;    // lowest bit the factor acts on: in the window, in the row (elements)
+  uint8_t radix, which;
+};
+// Window: float column bits [0, ib) and [b0, b0 + 6 - ib).
+struct MmaGeom {
+  int ib, b0, log_nf;
+  int sib;  // 2^sib CTAs walk the same row tiles of neighbouring blocks (mma_cta_of)
+  BFLY_HD int mid() const { return b0 - ib; }
+  // first column of block q of the row (the blocks are numbered by the bits outside the window)
+  BFLY_HD int base(int q) const { return ((q & ((1 << mid()) - 1)) << ib) | ((q >> mid()) << (b0 + kMmaWin - ib)); }
+  BFLY_HD int col(int j) const { return (j & ((1 << ib) - 1)) | ((j >> ib) << b0); }
+};
+struct MmaGroup {
+  int t0, t1;  // stages
+  MmaGeom geo;
+  int nst;
+  int passive; // element window bits no stage of the group acts on
+  MmaStage st[kMmaMaxStages];
+};
+
+// Rows of the caller: (row, stack, column) at p[row * sB + stack * sS + column], columns from `cols` on read as zero and
+// are not written.  flat > 0: the stacks are side by side in one matrix of `flat` columns, the last ones cut short.
+struct MmaRowsIO {
+  float* p;
+  int64_t sB, sS;
+  int cols, flat;
+  int align;  // bytes every row start is a multiple of (4, 8, 16 or 32)
+};
+BFLY_HD int mma_cols(const MmaRowsIO& r, int stack, int log_nf) {
+  if (r.flat <= 0) return r.cols;
+  const int left = r.flat - stack * (1 << log_nf);
+  return left < r.cols ? (left < 0 ? 0 : left) : r.cols;
+}
+
+struct MmaPass {
+  MmaGeom geo;
+  int S, B, nq, nt;       // stacks, rows, blocks of a row, row tiles
+  const uint8_t* images;  // operators of the group, (stack, block)
+  // forward: in -> out.  backward: gradient in -> out, x the activation that entered the group.  *_t: a plane instead of rows
+  const float* in_t;
+  float* out_t;
+  const float* x_t;
+  MmaRowsIO in, out, x;
+  int reduce;             // backward: add to the output rows (their stack stride is 0)
+  const float* bias;      // forward: bias[stack * nf + column] for flat positions below bias_len
+  int bias_len;
+  float* slots;           // backward: operator gradients, slot = block of (stack, q) + CTA
+  float* bias_slots;      // backward: column sums of the incoming gradient, 64 per slot; may be null
+};
+
+struct MmaPrep {
+  const void* tw[2];
+  int64_t tw_stack[2];
+  int S, nq, ng;
+  uint8_t* images;        // (group, stack, block)
+  MmaGroup g[kMmaMaxGroups];
+};
+struct MmaPost {
+  const void* tw[2];
+  void* dtw[2];
+  int64_t tw_stack[2];
+  int S, nq, nt, ng, ctas;
+  int last_group, group[kMmaMaxGroups];  // number of the product's last group, and of g[i] (by the launch)
+  const float* slots;     // (group, slot)
+  int64_t slots_group;    // floats from a group to the next
+  const float* bias_slots;
+  float* dbias;           // with bias_slots: column sums of the last group's incoming gradient
+  int dbias_len;
+  MmaGroup g[kMmaMaxGroups];
+};
+
+// Work of a pass: tiles numbered (stack, block, row tile); CTA c of G takes [W c / G, W (c + 1) / G), so that it keeps an
+// operator over many row tiles.  mma_cta_of: the CTA that takes tile w.  With geo.sib, CTAs and blocks count in groups of
+// 2^sib, one block to a CTA of the group.
+BFLY_HD int64_t mma_first_tile(int64_t W, int G, int c) { return W * c / G; }
+BFLY_HD int mma_cta_of(int64_t W, int G, int64_t w) { return (int)(((w + 1) * G + W - 1) / W) - 1; }
+// CTAs of a pass, and where group c of them leaves the sums of a block: both walk up, so that no two share a slot.
+BFLY_HD int mma_ctas(const MmaGeom& geo, int64_t tiles, int most) { return (int)(tiles < most ? tiles : most) >> geo.sib << geo.sib; }
+BFLY_HD int64_t mma_slot(const MmaGeom& geo, int64_t block, int c) { return block + ((int64_t)c << geo.sib); }
+
+// ------------------------------------------------------------------ host planning
+
+// Cut the stages into groups: fewest passes, and groups at the ends of the product that keep at least eight floats
+// (32 bytes, a sector) of a row together: pieces of 16 bytes cost a pass about a third more, shorter ones multiply it.
+inline bool mma_groups(const std::vector<Stage>& st, int F, int log_n, std::vector<MmaGroup>& out) {
+  const int ns = (int)st.size(), log_nf = log_n + F;
+  if (log_nf < kMmaWin) return false;
+  std::vector<double> best(ns + 1, 1e30);
+  std::vector<int> from(ns + 1, -1);
+  std::vector<MmaGeom> geo(ns + 1);
+  best[0] = 0;
+  for (int j = 0; j < ns; ++j) {
+    if (best[j] >= 1e29) continue;
+    int lo = 32, hi = 0, weight = 0;
+    for (int e = j + 1; e <= ns; ++e) {
+      const Stage& s = st[e - 1];
+      lo = std::min(lo, s.bit + F);
+      hi = std::max(hi, s.bit + F + (s.radix == 4 ? 2 : 1));
+      weight += s.radix == 4 ? 2 : 1;
+      MmaGeom g{kMmaWin, kMmaWin, log_nf, 0};
+      if (hi > kMmaWin) { g.ib = kMmaWin - (hi - lo); g.b0 = lo; }
+      if (g.ib < F || weight > kMmaMaxStages) break;
+      const double rough = g.ib >= 5 ? 0 : g.ib == 4 ? 0.1 : g.ib == 3 ? 0.2 : g.ib == 2 ? 1.5 : g.ib == 1 ? 3.0 : 6.0;
+      const double cost = best[j] + 1 + (j == 0 ? rough : 0) + (e == ns ? rough : 0);
+      if (cost < best[e] - 1e-9) { best[e] = cost; from[e] = j; geo[e] = g; }
+    }
+  }
+  if (from[ns] < 0) return false;
+  out.clear();
+  for (int e = ns; e > 0; e = from[e]) {
+    MmaGroup g;
+    std::memset(&g, 0, sizeof(g));
+    g.t0 = from[e]; g.t1 = e; g.geo = geo[e];
+    g.passive = (kMmaCols >> F) - 1;
+    for (int k = g.t0; k < e; ++k) {
+      MmaStage& m = g.st[g.nst++];
+      const int fb = st[k].bit + F;
+      m.tw_off = st[k].tw_off;
+      m.gbit = (uint8_t)st[k].bit;
+      m.lbit = (uint8_t)((fb < g.geo.ib ? fb : fb - g.geo.b0 + g.geo.ib) - F);
+      m.radix = (uint8_t)st[k].radix;
+      m.which = (uint8_t)st[k].which;
+      g.passive &= ~((st[k].radix == 4 ? 3 : 1) << m.lbit);
+    }
+    // Pieces of the caller's rows below a cache line: the CTAs that share lines keep together, so that L2 joins the pieces.
+    if ((g.t0 == 0 || g.t1 == ns) && g.geo.ib < 5 && g.geo.mid() >= 2) g.geo.sib = 2;
+    out.push_back(g);
+  }
+  std::reverse(out.begin(), out.end());
+  return (int)out.size() <= kMmaMaxGroups;
+}
+
+struct MmaLayout {
+  std::vector<MmaGroup> g;
+  int F, log_nf, nq;
+  int64_t nt;                   // row tiles
+  size_t plane;                 // bytes of a plane
+  size_t images;                // operators of all groups
+  size_t slots, bias_slots;     // backward: operator gradients of all groups, bias sums
+  // what a forward leaves: the activations between the groups, the operators
+  size_t kept() const { return (g.size() - 1) * plane + images; }
+  // work space of a backward that starts from that (a gradient plane), and of one that makes it itself (the gradient takes
+  // the place of the last activations)
+  size_t bw_bytes(bool from_kept) const { return slots + bias_slots + (from_kept ? (g.size() > 1 ? plane : 0) : kept()); }
+};
+
+}  // namespace bfly

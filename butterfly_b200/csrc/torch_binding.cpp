@@ -85,19 +85,12 @@ Tensor fw_impl(const Tensor& twiddle, const Tensor& input, bool increasing_strid
   auto stream = at::cuda::getCurrentCUDAStream();
   int rc;
   if (snapshots) {
-    const int64_t ws_bytes = bfly_bw_workspace_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks);
+    const int64_t ws_bytes = bfly_bw_snapshot_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks);
     TORCH_CHECK(ws_bytes >= 0, "butterfly_multiply failed: ", bfly_strerror((int)ws_bytes));
     *snapshots = torch::empty({ws_bytes}, input.options().dtype(at::kByte));
     void* sp = ws_bytes ? snapshots->data_ptr() : nullptr;
-    if (dt == BFLY_F32) {
-      rc = bfly_fw_f32_saving(tw.data_ptr<float>(), x.data_ptr<float>(), x.stride(0), x.stride(1),
-                              output.data_ptr<float>(), (int)batch, (int)nstacks, (int)log_n, (int)nblocks,
-                              (int)input_size, (int)out_size, increasing_stride, sp, (size_t)ws_bytes, stream.stream());
-    } else {
-      rc = bfly_fw_c64_saving(tw.data_ptr(), x.data_ptr(), x.stride(0), x.stride(1), output.data_ptr(), (int)batch,
-                              (int)nstacks, (int)log_n, (int)nblocks, (int)input_size, (int)out_size,
-                              increasing_stride, sp, (size_t)ws_bytes, stream.stream());
-    }
+    rc = bfly_fw_saving_ws(dt, tw.data_ptr(), x.data_ptr(), x.stride(0), x.stride(1), output.data_ptr(), (int)batch, (int)nstacks, (int)log_n,
+                           (int)nblocks, (int)input_size, (int)out_size, increasing_stride, sp, (size_t)ws_bytes, stream.stream());
   } else {
     // optional scratch of the forward (room for the re-ordered twiddles of its fastest kernel)
     const int64_t fws = bfly_fw_workspace_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks);
@@ -150,22 +143,19 @@ std::tuple<Tensor, Tensor> bw_impl(const Tensor& twiddle, const Tensor& input, c
   const Tensor g = rows_view(grad);
   Tensor d_twiddle = torch::empty_like(tw);
   Tensor d_input = torch::empty({batch, nstacks, std::max(input_size, n)}, input.options());
-  const int64_t ws_bytes = bfly_bw_workspace_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks);
+  const int64_t kept = snapshots && snapshots->defined() ? bfly_bw_snapshot_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks) : 0;
+  const bool saved = kept > 0 && snapshots->numel() >= kept;
+  const int64_t ws_bytes = saved ? bfly_bw_saved_workspace_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks)
+                                 : bfly_bw_workspace_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks);
   TORCH_CHECK(ws_bytes >= 0, "butterfly_multiply_bw failed: ", bfly_strerror((int)ws_bytes));
-  const bool saved = snapshots && snapshots->defined() && snapshots->numel() >= ws_bytes;
-  Tensor ws = saved ? *snapshots : torch::empty({ws_bytes}, input.options().dtype(at::kByte));
+  Tensor ws = torch::empty({ws_bytes}, input.options().dtype(at::kByte));
   auto stream = at::cuda::getCurrentCUDAStream();
   int rc;
-  if (saved && dt == BFLY_F32) {
-    rc = bfly_bw_f32_saved(tw.data_ptr<float>(), x.data_ptr<float>(), x.stride(0), x.stride(1), g.data_ptr<float>(),
-                           g.stride(0), g.stride(1), d_twiddle.data_ptr<float>(), d_input.data_ptr<float>(),
-                           (int)batch, (int)nstacks, (int)log_n, (int)nblocks, (int)input_size, (int)out_size,
-                           increasing_stride, ws_bytes ? ws.data_ptr() : nullptr, (size_t)ws_bytes, stream.stream());
-  } else if (saved) {
-    rc = bfly_bw_c64_saved(tw.data_ptr(), x.data_ptr(), x.stride(0), x.stride(1), g.data_ptr(), g.stride(0),
-                           g.stride(1), d_twiddle.data_ptr(), d_input.data_ptr(), (int)batch, (int)nstacks,
-                           (int)log_n, (int)nblocks, (int)input_size, (int)out_size, increasing_stride,
-                           ws_bytes ? ws.data_ptr() : nullptr, (size_t)ws_bytes, stream.stream());
+  if (saved) {
+    rc = bfly_bw_saved_ws(dt, tw.data_ptr(), x.data_ptr(), x.stride(0), x.stride(1), g.data_ptr(), g.stride(0), g.stride(1),
+                          d_twiddle.data_ptr(), d_input.data_ptr(), (int)batch, (int)nstacks, (int)log_n, (int)nblocks, (int)input_size,
+                          (int)out_size, increasing_stride, snapshots->data_ptr(), (size_t)kept, ws_bytes ? ws.data_ptr() : nullptr,
+                          (size_t)ws_bytes, stream.stream());
   } else if (dt == BFLY_F32) {
     rc = bfly_bw_f32(tw.data_ptr<float>(), x.data_ptr<float>(), x.stride(0), x.stride(1), g.data_ptr<float>(),
                      g.stride(0), g.stride(1), d_twiddle.data_ptr<float>(), d_input.data_ptr<float>(), (int)batch,
@@ -215,7 +205,7 @@ class ButterflyMultiply : public torch::autograd::Function<ButterflyMultiply> {
     bool save = false;
     if (wants_grad && twiddle.is_cuda() && input.is_cuda() && twiddle.dim() == 6 && input.dim() == 3 &&
         (input.scalar_type() == at::kFloat || input.scalar_type() == at::kComplexFloat)) {
-      const int64_t ws = bfly_bw_workspace_bytes(input.scalar_type() == at::kFloat ? BFLY_F32 : BFLY_C64,
+      const int64_t ws = bfly_bw_snapshot_bytes(input.scalar_type() == at::kFloat ? BFLY_F32 : BFLY_C64,
                                                  (int)input.size(0), (int)input.size(1), (int)twiddle.size(2),
                                                  (int)twiddle.size(1));
       save = ws > 0 && autograd_saves(ws);

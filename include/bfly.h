@@ -180,12 +180,26 @@ int bfly_bw_c64_saved(const void* twiddle, const void* x, int64_t x_sB, int64_t 
                       int output_size, int increasing_stride, void* snapshots,
                       size_t snapshot_bytes, void* stream);
 
+/* The same pair with the two kinds of scratch apart: what the saving forward leaves (bfly_bw_snapshot_bytes), and the
+ * backward's own work space (bfly_bw_saved_workspace_bytes, may be 0), so that nothing but the activations is held between
+ * the two.  Large products run as tensor-core passes here and in bfly_bw_*, whose planes need that; the pair above stays on the phase kernels.  dtype is BFLY_F32 or BFLY_C64. */
+int64_t bfly_bw_snapshot_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks);
+int64_t bfly_bw_saved_workspace_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks);
+int bfly_fw_saving_ws(int dtype, const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, void* out, int batch,
+                      int nstacks, int log_n, int nblocks, int input_size, int output_size, int increasing_stride,
+                      void* snapshots, size_t snapshot_bytes, void* stream);
+int bfly_bw_saved_ws(int dtype, const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, const void* grad,
+                     int64_t g_sB, int64_t g_sS, void* d_twiddle, void* d_x, int batch, int nstacks, int log_n,
+                     int nblocks, int input_size, int output_size, int increasing_stride, void* snapshots,
+                     size_t snapshot_bytes, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Development and test switches (no counterpart in the reference).  They are read from the
  * environment once, when the library first needs them, and can be changed at run time here; the
  * launch path never reads the environment.  Names (environment variable): "tma" (BFLY_TMA: 0 =
  * per-thread tile copies instead of the TMA unit), "fw2" (BFLY_FW2: 0 = generic forward kernel
  * only), "bw_v2" (BFLY_BW_V2), "fw_kmax", "fw_rows", "fw_logcmax", "bw_rows", "bw_maxsg" (planner
- * overrides; -1 = default), "fw_spread" (BFLY_FW_SPREAD), "virtual_rows" (BFLY_VIRTUAL_ROWS: 0 = rows one by
+ * overrides; -1 = default), "mma" (BFLY_MMA: tensor-core passes of large products; 0 never, 1 wherever they can run, -1 by
+ * size; not to be changed between a saving forward and its backward), "fw_spread" (BFLY_FW_SPREAD), "virtual_rows" (BFLY_VIRTUAL_ROWS: 0 = rows one by
  * one), "autograd_save" (BFLY_AUTOGRAD_SAVE: the torch autograd operators, butterfly_multiply and the layers, keep
  * the forward's snapshots: 0 never, 1 always, -1 by size).  Returns BFLY_E_ARG for an unknown name. */
 int bfly_set_option(const char* name, int value);
@@ -311,7 +325,10 @@ int bfly_selftest_bounded_wait(int polls, void* stream);
 #define BFLY_KERNEL_FW2 2  /* packed-pair forward kernel with its twiddle re-ordering kernel (bfly_fw2_kernel) */
 #define BFLY_KERNEL_BW2 3  /* backward phase kernel with accumulators in tensor memory (bfly_bw2_kernel) */
 #define BFLY_KERNEL_BW3 4  /* packed-pair backward phase kernel (bfly_bw3_kernel) */
-#define BFLY_KERNEL_IDS 5
+#define BFLY_KERNEL_MMA_FW 5  /* tensor-core forward pass (bfly_mma_fw_kernel) */
+#define BFLY_KERNEL_MMA_BW 6  /* tensor-core backward pass (bfly_mma_bw_kernel) */
+#define BFLY_KERNEL_MMA_OPS 7 /* their operators and the stages' gradients (bfly_mma_prep_kernel, bfly_mma_post_kernel) */
+#define BFLY_KERNEL_IDS 8
 void bfly_profile_enable(int on);
 int bfly_profile_collect(int64_t* launches, double* total_ms, int n_ids);
 

@@ -1,0 +1,126 @@
+"""Products as tensor-core passes (option "mma" = 1) against float64: tiles with few and missing rows, cut and padded columns,
+rows between alignments, several stacks, windows at every place of a row, both directions, both dtypes, both radices."""
+import pytest
+import torch
+
+from conftest import abi_option
+
+pytestmark = pytest.mark.gpu
+
+# A pass rounds its sums to 2^-24 four times and its result once, and drops what is below 2^-24 of a product: 1.2e-7 at most on
+# average over the columns, five passes at most; the operator gradient adds float32 sums over 128 rows at a time.
+TOL = 6e-7
+TOL_GRAD = 1.2e-6
+
+
+@pytest.fixture(scope="module")
+def dev():
+    return torch.device("cuda", 0)
+
+
+def rel2(a, b):
+    a, b = a.detach().cpu().to(b.dtype), b.detach()
+    return ((a - b).norm() / b.norm()).item()
+
+
+@pytest.mark.parametrize("cplx,log_n,nblocks,S,B,inc", [
+    (False, 6, 2, 1, 1, True), (False, 6, 2, 2, 129, False), (False, 7, 2, 3, 128, True), (False, 9, 1, 1, 127, True),
+    (False, 10, 1, 2, 300, False), (False, 10, 2, 4, 257, True), (False, 11, 2, 1, 130, False), (False, 12, 2, 1, 300, True),
+    (False, 13, 1, 1, 200, True), (False, 14, 1, 1, 65, False),
+    (True, 5, 2, 2, 300, True), (True, 6, 2, 1, 129, False), (True, 9, 1, 2, 128, True), (True, 10, 2, 1, 257, True),
+    (True, 11, 1, 1, 300, True), (True, 12, 1, 1, 70, False)])
+@pytest.mark.parametrize("save", [0, 1])
+def test_multiply(dev, oracle_mod, cplx, log_n, nblocks, S, B, inc, save):
+    import butterfly_b200 as bb
+    n, dt, wide = 1 << log_n, torch.complex64 if cplx else torch.float32, torch.complex128 if cplx else torch.float64
+    torch.manual_seed(log_n + B)
+    tw = torch.randn(S, nblocks, log_n, n // 2, 2, 2, dtype=dt) / 2 ** 0.5
+    x, g = torch.randn(B, S, n, dtype=dt), torch.randn(B, S, n, dtype=dt)
+    want_y = oracle_mod.multiply_fw(tw.to(wide), x.to(wide), inc)
+    want_d, want_dx = oracle_mod.multiply_bw(tw.to(wide), x.to(wide), g.to(wide), inc)
+    with abi_option("mma", 1), abi_option("autograd_save", save):
+        t, xd = tw.to(dev).requires_grad_(True), x.to(dev).requires_grad_(True)
+        y = bb.butterfly_multiply(t, xd, inc)
+        d, dx = torch.autograd.grad(y, [t, xd], g.to(dev))
+        d2, dx2 = bb.butterfly_multiply_bw(t.detach(), xd.detach(), g.to(dev), inc)
+    assert rel2(y, want_y) < TOL and rel2(dx, want_dx) < TOL and rel2(d, want_d) < TOL_GRAD
+    assert torch.equal(dx, dx2) and torch.equal(d, d2)  # the same bits with activations kept and made again
+    assert bb.abi.device_error() == 0
+
+
+@pytest.mark.parametrize("kind,in_size,out_size,nblocks,B", [
+    ("f32", 1000, 3000, 2, 150), ("f32", 1023, 1021, 2, 129), ("f32", 1024, 4096, 2, 200), ("f32", 70, 100, 2, 300),
+    ("f32", 4090, 4100, 1, 130), ("c64", 61, 64, 2, 300), ("c64", 500, 700, 2, 129), ("c64", 1999, 2000, 1, 40),
+    ("base4", 64, 64, 2, 129), ("base4", 1000, 2000, 2, 200), ("base4", 4096, 4000, 1, 100), ("base4", 500, 512, 2, 64)])
+@pytest.mark.parametrize("save", [0, 1])
+def test_layer(dev, oracle_mod, kind, in_size, out_size, nblocks, B, save):
+    import butterfly_b200 as bb
+    torch.manual_seed(in_size)
+    layer = (bb.ButterflyBase4 if kind == "base4" else bb.Butterfly)(in_size, out_size, bias=True, complex=kind == "c64", nblocks=nblocks)
+    dt, wide = (torch.complex64, torch.complex128) if kind == "c64" else (torch.float32, torch.float64)
+    x, g = torch.randn(B, in_size, dtype=dt), torch.randn(B, out_size, dtype=dt)
+    S, n = layer.nstacks, layer.n
+    xe = x.to(wide).unsqueeze(1).expand(B, S, in_size).contiguous()
+    gp = torch.zeros(B, S * n, dtype=wide)
+    gp[:, :out_size] = g
+    gp = gp.view(B, S, n)
+    if kind == "base4":
+        tws = [layer.twiddle4.detach().to(wide), layer.twiddle2.detach().to(wide)]
+        y = oracle_mod.base4_fw(*tws, xe, True)
+        *dtw, dx = oracle_mod.base4_bw(*tws, xe, gp, True)
+    else:
+        tws = [layer.twiddle.detach().to(wide)]
+        y = oracle_mod.multiply_fw(*tws, xe, True)
+        *dtw, dx = oracle_mod.multiply_bw(*tws, xe, gp, True)
+    want = [y.reshape(B, S * n)[:, :out_size] + layer.bias.detach().to(wide), dx.sum(1), g.to(wide).sum(0), *dtw]
+    layer = layer.to(dev)
+    params = [layer.twiddle4, layer.twiddle2] if kind == "base4" else [layer.twiddle]
+    xd = x.to(dev).requires_grad_(True)
+    with abi_option("mma", 1), abi_option("autograd_save", save):
+        out = layer(xd)
+        grads = torch.autograd.grad(out, [xd, layer.bias] + params, g.to(dev))
+    for got, ref, what in zip([out, *grads], want, ("output", "d_input", "d_bias", "d_twiddle", "d_twiddle2")):
+        if ref.numel():
+            assert rel2(got, ref) < (TOL if what in ("output", "d_input") else TOL_GRAD), what
+    assert bb.abi.device_error() == 0
+
+
+@pytest.mark.parametrize("pitch,offset", [(70, 0), (68, 4), (67, 1), (66, 2)])
+def test_strided_rows(dev, oracle_mod, pitch, offset):
+    import butterfly_b200 as bb
+    torch.manual_seed(pitch)
+    tw = torch.randn(1, 2, 6, 32, 2, 2) / 2 ** 0.5
+    rows, g = torch.randn(130, pitch, device=dev)[:, offset:offset + 64].unsqueeze(1), torch.randn(130, 1, 64)
+    want_d, want_dx = oracle_mod.multiply_bw(tw.double(), rows.cpu().double(), g.double(), True)
+    with abi_option("mma", 1):
+        d, dx = bb.butterfly_multiply_bw(tw.to(dev), rows, g.to(dev), True)
+    assert rel2(dx, want_dx) < TOL and rel2(d, want_d) < TOL_GRAD
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
+def test_values_at_the_ends_of_the_range(dev, value):
+    """A value that is not finite reaches what its row and its factors reach, and nothing else; the largest finite ones survive."""
+    import butterfly_b200 as bb
+    torch.manual_seed(3)
+    tw = (torch.randn(1, 2, 6, 32, 2, 2, device=dev) / 2 ** 0.5).abs() / 64
+    x, g = torch.rand(300, 1, 64, device=dev), torch.rand(300, 1, 64, device=dev)
+    outs = []
+    for v in (0.5, value):
+        g[131, 0, 5] = v
+        x[7, 0, 9] = v
+        with abi_option("mma", 1), abi_option("autograd_save", 1):
+            t, xd = tw.clone().requires_grad_(True), x.clone().requires_grad_(True)
+            y = bb.butterfly_multiply(t, xd, True)
+            outs.append([y.detach()] + list(torch.autograd.grad(y, [xd, t], g)))
+    (y0, dx0, _), (y1, dx1, d1) = outs
+    rest = torch.ones(300, dtype=torch.bool, device=dev)
+    rest[7] = False
+    assert torch.equal(y0[rest], y1[rest])
+    rest[7], rest[131] = True, False
+    assert torch.equal(dx0[rest], dx1[rest])
+    if value == 3.4e38:
+        assert torch.isfinite(y1).all() and torch.isfinite(dx1).all() and torch.isfinite(d1).all()
+    else:
+        assert not torch.isfinite(y1[7]).any() and not torch.isfinite(dx1[131]).any()
+        assert not torch.isfinite(d1).all()
+    assert bb.abi.device_error() == 0
