@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "bfly_fw2.h"
 #include "bfly_driver.h"
@@ -73,7 +74,9 @@ __device__ __forceinline__ void tma_store_box4(const CUtensorMap* map, uint32_t 
 // that reach across chunks -- and stores the box.  Every wait is bounded; a warp whose wait runs
 // out raises the CTA's give-up flag, which all warps read after the next CTA barrier.
 // THREADS = 512 (CTAS = 1): rows of 8192 columns, sixteen warps with one 512-column chunk each.
-template <int CTAS, int THREADS>
+// TAIL: rows with a cut block of columns (Fw2Params::x_tail); a variant of its own, since the other one has no registers left for
+// it (8192 x 8192, two blocks: 373 us with the branch, 361 without).
+template <int CTAS, int THREADS, bool TAIL>
 __global__ void __launch_bounds__(THREADS, CTAS)
 bfly_fw2_kernel(const __grid_constant__ Fw2Params p, const __grid_constant__ Fw2Maps maps, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -177,6 +180,18 @@ bfly_fw2_kernel(const __grid_constant__ Fw2Params p, const __grid_constant__ Fw2
         atomicExch(err, 1);
       }
       if (!p.cta_syncs) break;  // no other warp waits for this one
+    }
+    if (TAIL && chunk == (p.x_cols >> 9)) {
+      // The descriptor ends with the last whole block of 32 columns and the box has zeros behind it; the 4 to 28 columns
+      // of a cut block come by hand (12345 rows of 1000 columns, two blocks: 69 us; on the generic kernel 81).
+      const int c0 = p.x_cols & ~31, pieces = p.x_tail >> 2;
+      const float* src = p.x + (int64_t)row0 * p.x_sB + (p.x_stack ? stack * p.x_sS : 0) + c0;
+      for (int k = lane; k < Rw * pieces; k += 32) {
+        const int i = k / pieces, c = (k - i * pieces) * 4;
+        if (row0 + i < p.B)
+          *reinterpret_cast<float4*>(tile + fw2_tile_index(p.R, rg * Rw + i, c0 + c)) = __ldg(reinterpret_cast<const float4*>(src + i * p.x_sB + c));
+      }
+      __syncwarp();
     }
     bool alive = true;
     for (int gi = 0; gi < p.ngroups && alive; ++gi) {
@@ -320,7 +335,7 @@ int stack_sums_launch(const float* g, int64_t B, int S, int64_t n, int cols, flo
   return cudaGetLastError() == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
 }
 
-template <int CTAS, int THREADS>
+template <int CTAS, int THREADS, bool TAIL>
 static int fw2_launch_ctas(const Fw2Params& p, const Fw2Maps& maps, int grid, size_t smem, cudaStream_t stream, int* err) {
   static std::mutex mu;
   static bool attr_done[64] = {false};
@@ -329,9 +344,9 @@ static int fw2_launch_ctas(const Fw2Params& p, const Fw2Maps& maps, int grid, si
   {
     std::lock_guard<std::mutex> lk(mu);
     if (!attr_done[dev]) {
-      if (cudaFuncSetAttribute(bfly_fw2_kernel<CTAS, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      if (cudaFuncSetAttribute(bfly_fw2_kernel<CTAS, THREADS, TAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (CTAS == 1 ? 227 : 113) * 1024) != cudaSuccess ||
-          cudaFuncSetAttribute(bfly_fw2_kernel<CTAS, THREADS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+          cudaFuncSetAttribute(bfly_fw2_kernel<CTAS, THREADS, TAIL>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                cudaSharedmemCarveoutMaxShared) != cudaSuccess) {
         cudaGetLastError();
         return BFLY_E_CUDA;
@@ -347,7 +362,7 @@ static int fw2_launch_ctas(const Fw2Params& p, const Fw2Maps& maps, int grid, si
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(grid); c.blockDim = dim3(THREADS); c.dynamicSmemBytes = smem; c.stream = stream;
   c.attrs = &attr; c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, bfly_fw2_kernel<CTAS, THREADS>, p, maps, err) == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
+  return cudaLaunchKernelEx(&c, bfly_fw2_kernel<CTAS, THREADS, TAIL>, p, maps, err) == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
 }
 
 int fw2_launch(const Fw2Params& p_in, int ctas_per_sm, int sms, cudaStream_t stream, int* err, int* launches) {
@@ -372,7 +387,9 @@ int fw2_launch(const Fw2Params& p_in, int ctas_per_sm, int sms, cudaStream_t str
     for (int i = 0; i < kFw2MaxSnap; ++i)
       if (p.snap[i] && !fw2_describe_view(&maps.snap[i], p.snap[i], p.view_row, blk, pan, p.S, p.B, p.Rw)) return kFw2Declined;
   } else {
-  if (!fw2_describe(&maps.in, p.x, p.x_sB, p.x_sS, xc, p.B, p.S, p.Rw)) return kFw2Declined;
+  if (xc % 4 != 0 || !fw2_describe(&maps.in, p.x, p.x_sB, p.x_sS, xc & ~31, p.B, p.S, p.Rw)) return kFw2Declined;
+  p.x_cols = xc;
+  p.x_tail = xc & 31;
   p.x_stack = (p.S > 1 && p.x_sS != 0) ? 1 : 0;
   p.has_out = p.out != nullptr;
   if (p.has_out) {
@@ -390,9 +407,13 @@ int fw2_launch(const Fw2Params& p_in, int ctas_per_sm, int sms, cudaStream_t str
   bfly_fw2_pack_kernel<<<(int)std::min<int64_t>((entries + 255) / 256, 4 * sms), 256, 0, stream>>>(p);
   if (cudaGetLastError() != cudaSuccess) return BFLY_E_CUDA;
   const int grid = (int)std::min<int64_t>(fw2_num_tiles(p), (int64_t)ctas_per_sm * sms);
-  const int rc = fw2_threads(p) == kFw2WideThreads ? fw2_launch_ctas<1, kFw2WideThreads>(p, maps, grid, smem, stream, err)
-                 : ctas_per_sm == 1              ? fw2_launch_ctas<1, kFw2Threads>(p, maps, grid, smem, stream, err)
-                                                 : fw2_launch_ctas<2, kFw2Threads>(p, maps, grid, smem, stream, err);
+  auto go = [&](auto tail) {
+    constexpr bool T = decltype(tail)::value;
+    return fw2_threads(p) == kFw2WideThreads ? fw2_launch_ctas<1, kFw2WideThreads, T>(p, maps, grid, smem, stream, err)
+           : ctas_per_sm == 1              ? fw2_launch_ctas<1, kFw2Threads, T>(p, maps, grid, smem, stream, err)
+                                           : fw2_launch_ctas<2, kFw2Threads, T>(p, maps, grid, smem, stream, err);
+  };
+  const int rc = p.x_tail ? go(std::true_type()) : go(std::false_type());
   if (rc == BFLY_OK && launches) *launches = 2;
   return rc;
 }

@@ -150,6 +150,7 @@ struct Fw2Params {
   // the tensors themselves (the device kernel reaches them through TMA descriptors; the host
   // emulator through these)
   const float* x; int64_t x_sB, x_sS; int x_cols;
+  int x_tail;        // columns of the input behind its last whole block of 32, a multiple of 4 (set by the launcher)
   float* out; int64_t out_sB, out_sS;
   float* snap[kFw2MaxSnap];
   // optional bias added to the output before it is stored: bias[stack * n + column] for flat

@@ -54,7 +54,7 @@ struct EmulExec {
     Fw2Params p = p_in;
     const int n = 1 << p.log_n;
     if (p.view && ((p.panel.lseg != p.panel.logC && p.panel.lseg != 5) || p.bias)) return kFw2Declined;
-    if (p.x_cols % 32 != 0 && p.x_cols < n) return kFw2Declined;  // what the TMA descriptors would refuse
+    if (p.x_cols < n && (p.x_cols < 32 || p.x_cols % 4 != 0)) return kFw2Declined;  // what the descriptors and the cut block's copies refuse
     if (p.out && p.out_cols % 32 != 0) return kFw2Declined;
     p.has_out = p.out != nullptr;
     if (!p.has_out) p.out_cols = n;
