@@ -182,7 +182,8 @@ int bfly_bw_c64_saved(const void* twiddle, const void* x, int64_t x_sB, int64_t 
 
 /* The same pair with the two kinds of scratch apart: what the saving forward leaves (bfly_bw_snapshot_bytes), and the
  * backward's own work space (bfly_bw_saved_workspace_bytes, may be 0), so that nothing but the activations is held between
- * the two.  Large products run as tensor-core passes here and in bfly_bw_*, whose planes need that; the pair above stays on the phase kernels.  dtype is BFLY_F32 or BFLY_C64. */
+ * the two.  Large products run as tensor-core passes here and in bfly_bw_*, whose planes need that; the pair above stays
+ * on the phase kernels.  dtype is BFLY_F32 or BFLY_C64. */
 int64_t bfly_bw_snapshot_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks);
 int64_t bfly_bw_saved_workspace_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks);
 int bfly_fw_saving_ws(int dtype, const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, void* out, int batch,
