@@ -755,6 +755,42 @@ int plan_bw(const Problem& q, BwLayout<T>& lay) {
   return BFLY_OK;
 }
 
+// Work space of a backward that is told nothing but the sizes: the phase plan depends on the direction of the first block, so
+// the larger need of the two.
+template <typename T> inline int64_t bw_workspace_need(const Problem& q0) {
+  int64_t best = 0;
+  for (int inc = 0; inc < 2; ++inc) {
+    Problem q = q0;
+    q.inc = inc != 0;
+    BwLayout<T> lay;
+    const int rc = plan_bw<T>(q, lay);
+    if (rc) return rc;
+    best = std::max<int64_t>(best, (int64_t)lay.ws_bytes);
+  }
+  // tensor-core passes: at least a plane per group, like the phases with the forward's scratch behind it
+  return std::max(best, mma_either<T>(q0, [&](const MmaLayout& L) {
+    return std::max(L.bw_bytes(false) + kMmaSpare, L.g.size() * L.plane) + (q0.base4 ? 0 : fw_workspace_bytes<T>(q0));
+  }));
+}
+// What a saving forward has to leave for the backward, again for either direction: one of them may run as tensor-core passes
+// and the other as phases (float, 4096 columns, two blocks: three groups of stages one way, five the other).
+template <typename T> inline int64_t bw_snapshot_need(const Problem& q0) {
+  int64_t best = 0;
+  for (int inc = 0; inc < 2; ++inc) {
+    Problem q = q0;
+    q.inc = inc != 0;
+    MmaLayout M;
+    BwLayout<T> lay;
+    if (mma_layout<T>(q, M)) {
+      best = std::max<int64_t>(best, (int64_t)(M.kept() + kMmaSpare));
+    } else {
+      if (const int rc = plan_bw<T>(q, lay)) return rc;
+      best = std::max<int64_t>(best, (int64_t)lay.ws_bytes);
+    }
+  }
+  return best;
+}
+
 // Forward that also writes, into ws, the phase-boundary activations the backward of the same
 // problem starts from (the layout drive_bw expects when it is told the snapshots are ready).
 template <typename T, typename E>

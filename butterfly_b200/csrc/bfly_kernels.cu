@@ -856,32 +856,6 @@ static int bw_entry(bool base4, const void* tw2, const void* tw4, const void* x,
                      static_cast<T*>(d4), static_cast<T*>(dx), ws, ws_bytes, snapshots_ready, 0, extra, extra_bytes);
 }
 
-template <typename T>
-static int64_t ws_for(const Problem& q0) {
-  // the phase plan depends on the direction of the first block: report the larger need
-  int64_t best = 0;
-  for (int inc = 0; inc < 2; ++inc) {
-    Problem q = q0;
-    q.inc = inc != 0;
-    BwLayout<T> lay;
-    const int rc = plan_bw<T>(q, lay);
-    if (rc) return rc;
-    best = std::max<int64_t>(best, (int64_t)lay.ws_bytes);
-  }
-  // tensor-core passes: at least a plane per group, like the phases with the forward's scratch behind it
-  return std::max(best, mma_either<T>(q0, [&](const MmaLayout& L) {
-    return std::max(L.bw_bytes(false) + kMmaSpare, L.g.size() * L.plane) + (q0.base4 ? 0 : fw_workspace_bytes<T>(q0));
-  }));
-}
-// What a saving forward has to leave for the backward.
-template <typename T>
-static int64_t kept_for(const Problem& q0) {
-  const int64_t kept = mma_either<T>(q0, [](const MmaLayout& L) { return L.kept() + kMmaSpare; });
-  Problem q = q0;
-  q.phases = true;
-  return kept > 0 ? kept : ws_for<T>(q);
-}
-
 // f(element of the layer's type, problem)
 template <typename F> static int64_t layer_call(const bfly_layer_t* l, F&& f) {
   const Problem q{l->batch, l->nstacks, l->log_n, l->nblocks, l->input_size, 1 << (l->log_n & 31), l->increasing_stride != 0, l->base4 != 0};
@@ -896,8 +870,8 @@ static int64_t ws_entry(bool base4, int dtype, int B, int S, int log_n, int nblo
   Problem q{B, S, log_n, nblocks, 1, 1, true, base4};
   int rc = check_problem(q);
   if (rc) return rc;
-  if (dtype == BFLY_F32) return ws_for<float>(q);
-  if (dtype == BFLY_C64) return ws_for<cf>(q);
+  if (dtype == BFLY_F32) return bw_workspace_need<float>(q);
+  if (dtype == BFLY_C64) return bw_workspace_need<cf>(q);
   return BFLY_E_UNSUPPORTED;
 }
 
@@ -1165,8 +1139,8 @@ int64_t bfly_bw_snapshot_bytes(int dtype, int batch, int nstacks, int log_n, int
   Problem q{batch, nstacks, log_n, nblocks, 1, 1, true, false};
   const int rc = check_problem(q);
   if (rc) return rc;
-  if (dtype == BFLY_F32) return kept_for<float>(q);
-  if (dtype == BFLY_C64) return kept_for<cf>(q);
+  if (dtype == BFLY_F32) return bw_snapshot_need<float>(q);
+  if (dtype == BFLY_C64) return bw_snapshot_need<cf>(q);
   return BFLY_E_UNSUPPORTED;
 }
 int bfly_fw_saving_ws(int dtype, const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, void* out, int batch, int nstacks, int log_n,

@@ -575,3 +575,138 @@ int bfly_emul_bw_plan(int dtype, int base4, int B, int S, int log_n, int nblocks
   return nph;
 }
 }
+
+// ------------------------------------------------------------------ dry runs of whole training steps
+//
+// The drivers with an executor that launches nothing: every call gets buffers of exactly the queried sizes, at made-up
+// addresses, and each launch's tensors are checked to lie inside them.
+namespace {
+struct DryExec {
+  static constexpr bool kMma = true, kFusedBias = true;
+  struct Range { uintptr_t at; size_t bytes; };
+  std::vector<Range> ranges;
+  int outside = 0, passes = 0;  // tensors that left their buffer; tensor-core passes
+  // a buffer of `bytes` bytes, `skew` past a 256-byte boundary
+  template <typename T> T* buffer(size_t bytes, size_t skew = 0) {
+    if (!bytes) return nullptr;
+    ranges.push_back({((uintptr_t)(ranges.size() + 1) << 44) + skew, bytes});
+    return reinterpret_cast<T*>(ranges.back().at);
+  }
+  void in(const void* p, size_t bytes) {
+    const uintptr_t a = (uintptr_t)p;
+    for (auto& r : ranges)
+      if (a >= r.at && a + bytes <= r.at + r.bytes) return;
+    ++outside;
+  }
+  template <typename T> void rows(const T* p, int64_t B, int64_t S, int64_t sB, int64_t sS, int64_t cols) {
+    if (p && B > 0 && cols > 0) in(p, ((B - 1) * sB + (S - 1) * sS + cols) * sizeof(T));
+  }
+  int num_sms() const { return 148; }
+  int threads() const { return 256; }
+  bool has_bw2(size_t, int kw) const { return kw == 2; }
+  int run_fw2(const Fw2Params& p, int) {
+    const int64_t S = p.view ? 1 : p.S, n = p.view ? p.view_row : (int64_t)1 << p.log_n;
+    for (const float* s : p.snap)
+      if (s) in(s, (size_t)p.B * S * n * sizeof(float));
+    in(p.packed, (size_t)p.packed_stack * p.S * 16);
+    rows(p.x, p.B, S, p.x_sB, p.x_sS, p.view ? n : std::min<int64_t>(p.x_cols, n));
+    rows(p.out, p.B, S, p.out_sB, p.out_sS, p.view ? n : p.out_cols);
+    return BFLY_OK;
+  }
+  template <typename T> int run_fw(const FwParams<T>& p) {
+    const int64_t n = (int64_t)1 << p.log_n;
+    for (const T* s : p.snap)
+      if (s) in(s, ((size_t)p.B_rows * p.S << p.log_n) * sizeof(T));
+    rows(p.x, p.B_rows, p.S, p.x_sB, p.x_sS, std::min<int64_t>(p.x_cols, n));
+    rows(p.out, p.B_rows, p.S, p.out_sB, p.out_sS, std::min<int64_t>(p.out_cols, n));
+    return BFLY_OK;
+  }
+  template <typename T> int run_bw(const BwParams<T>& p, int) {
+    const int64_t n = (int64_t)1 << p.log_n;
+    rows(p.xin, p.B_rows, p.S, p.xin_sB, p.xin_sS, std::min<int64_t>(p.xin_cols, n));
+    rows(p.gin, p.B_rows, p.gin_flat > 0 ? 1 : p.S, p.gin_sB, p.gin_sS, p.gin_flat > 0 ? p.gin_flat : std::min<int64_t>(p.gin_cols, n));
+    rows(p.gout, p.B_rows, p.S, p.gout_sB, p.gout_sS, p.gout_cols);
+    return BFLY_OK;
+  }
+  bool can_run_bw3(const Bw3Params&) { return true; }
+  int run_bw3(const Bw3Params& p) { return run_bw(p.b, 2); }
+  int add_bias(float* out, const float* bias, int64_t B, int len, int64_t pitch) { rows(out, B, 1, pitch, 0, len); in(bias, len * 4); return BFLY_OK; }
+  template <typename T> int column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out, float* partial) {
+    rows(g, B, 1, pitch, 0, cols);
+    in(out, cols * sizeof(T));
+    if (const size_t f = column_sum_slices(B, cols * (int)(sizeof(T) / 4)).floats) in(partial, f * 4);
+    return BFLY_OK;
+  }
+  template <typename T> int stack_sums(const T* g, int64_t B, int S, int64_t n, int cols, T* out) {
+    in(g, B * S * n * sizeof(T));
+    in(out, B * cols * sizeof(T));
+    return BFLY_OK;
+  }
+  int zero(void* p, size_t bytes) { in(p, bytes); return BFLY_OK; }
+  int zero2d(void* p, size_t pitch, size_t width, size_t n) { if (n) in(p, (n - 1) * pitch + width); return BFLY_OK; }
+  void io(const MmaRowsIO& r, const MmaPass& p) {
+    if (r.flat > 0) rows(r.p, p.B, 1, r.sB, 0, r.flat);
+    else rows(r.p, p.B, p.S, r.sB, r.sS, std::min(r.cols, 1 << p.geo.log_nf));
+  }
+  void plane(const float* t, const MmaPass& p) { in(t, ((size_t)p.S * p.nt * kMmaRows << p.geo.log_nf) * sizeof(float)); }
+  int mma_prep(const MmaPrep& p, bool) { in(p.images, (size_t)p.ng * p.S * p.nq * kMmaImageBytes); return BFLY_OK; }
+  int mma_fw(const MmaPass& p) {
+    ++passes;
+    in(p.images, (size_t)p.S * p.nq * kMmaImageBytes);
+    if (p.in_t) plane(p.in_t, p); else io(p.in, p);
+    if (p.out_t) plane(p.out_t, p); else io(p.out, p);
+    return BFLY_OK;
+  }
+  int mma_bw(const MmaPass& p, int ctas) {
+    ++passes;
+    in(p.images, (size_t)p.S * p.nq * kMmaImageBytes);
+    if (p.in_t) plane(p.in_t, p); else io(p.in, p);
+    if (p.x_t) plane(p.x_t, p); else io(p.x, p);
+    if (p.out_t) plane(p.out_t, p); else io(p.out, p);
+    // the last slot that a CTA can leave (mma_slot)
+    const int used = mma_ctas(p.geo, (int64_t)p.S * p.nq * p.nt, ctas);
+    const int64_t last = mma_slot(p.geo, (int64_t)p.S * p.nq - 1, (used >> p.geo.sib) - 1) + 1;
+    in(p.slots, (size_t)last * kMmaSlotFloats * sizeof(float));
+    if (p.bias_slots) in(p.bias_slots, (size_t)last * kMmaCols * sizeof(float));
+    return BFLY_OK;
+  }
+  int mma_post(const MmaPost&, bool) { return BFLY_OK; }
+};
+
+// how: 0 the operator with saved activations and a work space of its own, 1 the backward that makes them itself.
+template <typename T> int dry_step(Problem q, int how, size_t skew, int* passes) {
+  DryExec ex;
+  const int64_t n = (int64_t)1 << q.log_n, DX = std::max<int64_t>(q.in_size, n);
+  int64_t stk[2];
+  twiddle_stack_sizes(q, stk);
+  T* tw2 = ex.buffer<T>(q.S * stk[0] * sizeof(T)), *tw4 = ex.buffer<T>(q.S * stk[1] * sizeof(T));
+  T* d2 = ex.buffer<T>(q.S * stk[0] * sizeof(T)), *d4 = ex.buffer<T>(q.S * stk[1] * sizeof(T));
+  const size_t BS = (size_t)q.B * q.S;
+  T* x = ex.buffer<T>(BS * q.in_size * sizeof(T)), *out = ex.buffer<T>(BS * n * sizeof(T));
+  T* g = ex.buffer<T>(BS * q.out_size * sizeof(T)), *dx = ex.buffer<T>(BS * DX * sizeof(T));
+  const int64_t x_sB = (int64_t)q.S * q.in_size, g_sB = (int64_t)q.S * q.out_size;
+  int rc = BFLY_OK;
+  if (how == 0) {
+    const int64_t kept = bw_snapshot_need<T>(q), own = mma_either<T>(q, [](const MmaLayout& L) { return L.bw_bytes(true) + kMmaSpare; });
+    if (kept < 0) return (int)kept;
+    char* k = ex.buffer<char>(kept, skew), *w = ex.buffer<char>(own, skew);
+    rc = drive_fw_saving<T>(ex, q, tw2, tw4, x, x_sB, q.in_size, out, k, kept);
+    if (rc == BFLY_OK)
+      rc = drive_bw<T>(ex, q, tw2, tw4, x, x_sB, q.in_size, g, g_sB, q.out_size, d2, d4, dx, k, kept, true, 0, w, own);
+  } else {
+    const int64_t need = bw_workspace_need<T>(q);
+    if (need < 0) return (int)need;
+    rc = drive_bw<T>(ex, q, tw2, tw4, x, x_sB, q.in_size, g, g_sB, q.out_size, d2, d4, dx, ex.buffer<char>(need, skew), need);
+  }
+  *passes = ex.passes;
+  return rc ? rc : (ex.outside ? 1 : 0);
+}
+}  // namespace
+extern "C" {
+// 0, a status of the library, or 1: a launch left the buffers it was given
+int bfly_emul_dry_step(int dtype, int base4, int how, int64_t skew, int B, int S, int log_n, int nblocks, int in_size, int out_size, int inc, int* passes) {
+  Problem q{B, S, log_n, nblocks, in_size, out_size, inc != 0, base4 != 0};
+  if (const int rc = check_problem(q)) return rc;
+  return dtype == 0 ? dry_step<float>(q, how, (size_t)skew, passes) : dry_step<cf>(q, how, (size_t)skew, passes);
+}
+}

@@ -678,3 +678,28 @@ def test_kronecker_twiddle_as_transforms_see_it():
         assert torch.autograd.gradgradcheck(k, (leaf,))
     with pytest.raises(RuntimeError, match="same device"):
         bb.combine.kronecker_twiddle(t1.to("meta"), t2, True)
+
+
+@pytest.mark.parametrize("dtype", [0, 1], ids=["f32", "c64"])
+@pytest.mark.parametrize("how", ["saved", "recomputed"])
+def test_queried_bytes_are_enough_for_what_runs(emul, dtype, how):
+    """Training steps under the default options with buffers of exactly the queried sizes, from 16 bytes past a boundary: both
+    directions, one to three blocks, up to 2^26 values, on either side of the rule for tensor-core passes.  Nothing is
+    refused and no launch leaves a buffer.  (A product may qualify for the passes in one direction and not in the other.)"""
+    routes = {}
+    for log_n in range(5, 16):
+        rows = [300, 777] + [(1 << k) + d for k in range(9, 18) for d in (0, 5)]
+        for B in rows:
+            for S in (1, 3):
+                if B * S << log_n > 1 << 26:
+                    continue
+                for nb in (1, 2, 3):
+                    for base4 in (0, 1):
+                        for inc in (0, 1):
+                            passes = ctypes.c_int(0)
+                            rc = emul.bfly_emul_dry_step(dtype, base4, int(how == "recomputed"), I64(16), B, S, log_n, nb, 1 << log_n, 1 << log_n, inc,
+                                                         ctypes.byref(passes))
+                            assert rc == 0, (log_n, B, S, nb, base4, inc, rc)
+                            routes[log_n, B, S, nb, base4, inc] = passes.value > 0
+    one_way = [k for k, v in routes.items() if v and not routes[k[:-1] + (1 - k[-1],)]]
+    assert one_way and any(routes.values()) and not all(routes.values())

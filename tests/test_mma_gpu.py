@@ -124,3 +124,24 @@ def test_values_at_the_ends_of_the_range(dev, value):
         assert not torch.isfinite(y1[7]).any() and not torch.isfinite(dx1[131]).any()
         assert not torch.isfinite(d1).all()
     assert bb.abi.device_error() == 0
+
+
+@pytest.mark.parametrize("cplx,log_n,B", [(False, 12, 16384), (True, 10, 1024)])
+@pytest.mark.parametrize("inc", [True, False])
+def test_large_training_steps_under_the_default_rule(dev, cplx, log_n, B, inc):
+    """Two blocks: one direction runs as passes, the other, which is cut into more groups, on the phases.  Both train, and agree
+    with the phases to what two float32 evaluations of 24 factors may differ by."""
+    import butterfly_b200 as bb
+    n, dt = 1 << log_n, torch.complex64 if cplx else torch.float32
+    torch.manual_seed(log_n)
+    tw = (torch.randn(1, 2, log_n, n // 2, 2, 2, dtype=dt, device=dev) / 2 ** 0.5).requires_grad_(True)
+    x, g = (torch.randn(B, 1, n, dtype=dt, device=dev) for _ in range(2))
+    x.requires_grad_(True)
+    got = []
+    for mma in (-1, 0):
+        with abi_option("mma", mma):
+            y = bb.butterfly_multiply(tw, x, inc)
+            got.append([y.detach()] + list(torch.autograd.grad(y, [tw, x], g)))
+    for a, b in zip(*got):
+        assert ((a - b).norm() / b.norm()).item() < 2e-6
+    assert bb.abi.device_error() == 0
