@@ -1125,7 +1125,7 @@ int bfly_bw_f32_saved(const float* twiddle, const float* x, int64_t x_sB, int64_
                       size_t snapshot_bytes, void* stream) {
   return bw_entry<float>(false, twiddle, nullptr, x, x_sB, x_sS, grad, g_sB, g_sS, d_twiddle, nullptr, d_x, batch,
                          nstacks, log_n, nblocks, input_size, output_size, increasing_stride, snapshots,
-                         snapshot_bytes, stream, true);
+                         snapshot_bytes, stream, true, nullptr, 0, true);
 }
 int bfly_bw_c64_saved(const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, const void* grad, int64_t g_sB,
                       int64_t g_sS, void* d_twiddle, void* d_x, int batch, int nstacks, int log_n, int nblocks,
@@ -1133,7 +1133,7 @@ int bfly_bw_c64_saved(const void* twiddle, const void* x, int64_t x_sB, int64_t 
                       void* stream) {
   return bw_entry<cf>(false, twiddle, nullptr, x, x_sB, x_sS, grad, g_sB, g_sS, d_twiddle, nullptr, d_x, batch,
                       nstacks, log_n, nblocks, input_size, output_size, increasing_stride, snapshots, snapshot_bytes,
-                      stream, true);
+                      stream, true, nullptr, 0, true);
 }
 int64_t bfly_bw_snapshot_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks) {
   Problem q{batch, nstacks, log_n, nblocks, 1, 1, true, false};

@@ -145,3 +145,21 @@ def test_large_training_steps_under_the_default_rule(dev, cplx, log_n, B, inc):
     for a, b in zip(*got):
         assert ((a - b).norm() / b.norm()).item() < 2e-6
     assert bb.abi.device_error() == 0
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_the_pair_of_one_buffer_stays_on_the_phases(dev, cplx):
+    """bfly_fw_*_saving and bfly_bw_*_saved have no work space for the passes, wherever these would run."""
+    from butterfly_b200 import abi
+    dt = torch.complex64 if cplx else torch.float32
+    torch.manual_seed(2)
+    tw = torch.randn(1, 2, 10, 512, 2, 2, dtype=dt, device=dev) / 2 ** 0.5
+    x, g = (torch.randn(300, 1, 1024, dtype=dt, device=dev) for _ in range(2))
+    with abi_option("mma", 1):
+        out, snaps, rc = abi.fw_saving(tw, x, True, check=False)
+        assert rc == 0
+        d, dx, rc = abi.bw_saved(tw, x, g, snaps, True, check=False)
+        assert rc == 0
+    with abi_option("mma", 0):
+        want, want_x, _ = abi.bw(tw, x, g, True)
+    assert torch.equal(dx, want_x) and ((d - want).norm() / want.norm()).item() < 1e-6
