@@ -47,12 +47,12 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float* v) {
                : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(addr));
 }
 
-// tcgen05 cuts the sum of every instruction (16 products and the accumulator) to 24 bits towards zero.  Mean relative
-// loss of the largest products of a tile, measured on normal deviates: 0.4e-8 after one instruction, 1.9e-8 after two,
-// 4.6e-8 after four, 8.0e-8 after eight (1.14e-7 in the 2-norm).  So 64 columns go to two accumulators, two instructions
-// each, and what is lost on average is added back.
-constexpr float kMmaTruncOut = 4.0e-8f;
-constexpr float kMmaTruncGrad = 8.0e-8f;
+// tcgen05 cuts the sum of every instruction (16 products and the accumulator) to 24 bits towards zero: half a unit of the
+// last place on average, always towards zero, where rounding has no mean.  A constant that puts the mean back is wrong
+// wherever nothing was cut, so the sums that count are kept exact instead: the largest part of an operator entry is a
+// multiple of 1/16 of the largest entry of its row and column (bfly_mma_prep_kernel), four bits at most beside the eight of
+// the rows' first slice, and values down to 2^-9 of the largest of 64 add up within 24 bits.  What is cut from the other
+// products is a sixteenth of a unit.
 
 // ------------------------------------------------------------------ values and slices
 
@@ -196,36 +196,32 @@ __device__ __forceinline__ float image_elem(const uint8_t* img, int j, int i) {
   const uint8_t* q = img + j * 128 + (((i >> 3) ^ (j & 7)) << 4) + (i & 7) * 2;
   float v = 0.f;
 #pragma unroll
-  for (int s = 2; s >= 0; --s) v += __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t*>(q + s * 8192) << 16);
+  for (int s = kMmaParts - 1; s >= 0; --s) v += __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t*>(q + s * 8192) << 16);
   return v;
 }
 
-// rows x operator (TRANS: transposed operator).  Slices 1 of both, the largest products, into columns 0 .. 63 of d (the
-// first 32 columns of the operand) and 192 .. (the others), all other products in between: 12, 21, 31 and 13, 22.  An
-// instruction takes its operands' bytes / 128 clocks (measured: N = 64 48, 128 64, 192 96), so few wide ones: 864 for a tile.
+// rows x operator (TRANS: transposed operator).  Accumulators of 64 columns: slice 1 of the rows and part 1 of the operator,
+// the largest products, into d, and behind them 12 21, 13 22 31 and 14 23 32, each about a 2^-5th to 2^-9th of the one
+// before.  An instruction takes its operands' bytes / 128 clocks (measured: N = 64 48, 128 64, 192 96, so 256 128): 1152 for a tile.
 template <bool PLANE, bool TRANS> __device__ __forceinline__ void issue_transform(uint32_t d, uint32_t op, uint32_t img) {
   constexpr uint32_t slice = PLANE ? 8192 : 16384;
-  constexpr uint32_t i64 = mma_idesc(64, PLANE, TRANS), i128 = mma_idesc(128, PLANE, TRANS), i192 = mma_idesc(192, PLANE, TRANS);
+  constexpr uint32_t i128 = mma_idesc(128, PLANE, TRANS), i192 = mma_idesc(192, PLANE, TRANS), i256 = mma_idesc(256, PLANE, TRANS);
   const uint64_t a0 = PLANE ? mma_desc(op, 24576, 1024) : mma_desc(op, 16, 1024);
   const uint64_t b0 = TRANS ? mma_desc(img, 8192, 1024) : mma_desc(img, 16, 1024);
-  constexpr uint64_t as = slice >> 4, bs = 8192 >> 4;
+  constexpr uint64_t as = slice >> 4;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const uint64_t a = a0 + k * ((PLANE ? 2048 : 32) >> 4), b = b0 + k * ((TRANS ? 2048 : 32) >> 4);
-    if (k < 2) {
-      mma_issue(d, a, b, i192, k > 0);
-    } else {
-      mma_issue(d + 192, a, b, i64, k > 2);
-      mma_issue(d + 64, a, b + bs, i128, true);
-    }
-    mma_issue(d + 64, a + as, b, i128, true);
-    mma_issue(d + 64, a + 2 * as, b, i64, true);
+    mma_issue(d, a, b, i256, k > 0);
+    mma_issue(d + 64, a + as, b, i192, true);
+    mma_issue(d + 128, a + 2 * as, b, i128, true);
   }
 }
 
-// g^T x over the tile's rows.  Slices of g: 1 and 2 stacked in the lanes, then 3 (upper lanes: whatever follows it).
-// P1 = d: g1|g2 x x1, taken out after every tile; P2 = d + 64: g1|g2 x (x2 | x3) and P3 = d + 192: g3 x x1 are 2^-8 as
-// large and run on (`keep`).
+// g^T x over the tile's rows, two slices of g stacked in the lanes.  Columns 0 .. of d: g1 x x1 of rows 0 .. 63 in the lower
+// lanes, 64 .. the same of rows 64 .. 127 (what lands in the upper lanes, g2 x x1, is not used): short sums, taken out after
+// every tile.  128 .. and 192 ..: all other products, g1|g2 x (x2|x3) and g2|g3 x x1, are 2^-8 as large and run on (`keep`).
+// 1280 clocks for a tile.
 template <bool GP, bool XP> __device__ __forceinline__ void issue_outer(uint32_t d, uint32_t g, uint32_t x, bool keep) {
   constexpr uint32_t i64 = mma_idesc(64, !GP, !XP), i128 = mma_idesc(128, !GP, !XP);
   constexpr uint64_t gs = (GP ? 8192 : 16384) >> 4, xs = (XP ? 8192 : 16384) >> 4;
@@ -233,25 +229,22 @@ template <bool GP, bool XP> __device__ __forceinline__ void issue_outer(uint32_t
   for (int k = 0; k < 8; ++k) {
     const uint32_t go = GP ? (k >> 2) * 24576 + (k & 3) * 32 : k * 2048, xo = XP ? (k >> 2) * 24576 + (k & 3) * 32 : k * 2048;
     const uint64_t a = mma_desc(g + go, GP ? 16 : 16384, 1024), b = mma_desc(x + xo, XP ? 16 : 16384, 1024);
-    mma_issue(d, a, b, i64, k > 0);
-    mma_issue(d + 64, a, b + xs, i128, keep || k > 0);
-    mma_issue(d + 192, a + 2 * gs, b, i64, keep || k > 0);
+    mma_issue(d + (k >> 2) * 64, a, b, i64, (k & 3) > 0);
+    mma_issue(d + 128, a, b + xs, i128, keep || k > 0);
+    mma_issue(d + 128, a + gs, b, i64, true);
   }
 }
 
-// Eight columns of what issue_transform left: two large sums and two small ones.
+// Eight columns of what issue_transform left.
 __device__ __forceinline__ void load_transform(uint32_t d, float* y) {
   float a[8], b[8], c[8];
   tmem_ld8(d, y);
-  tmem_ld8(d + 192, a);
-  tmem_ld8(d + 64, b);
-  tmem_ld8(d + 128, c);
+  tmem_ld8(d + 64, a);
+  tmem_ld8(d + 128, b);
+  tmem_ld8(d + 192, c);
   wait_ld();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float s = y[i] + a[i];
-    y[i] = s + fmaf(s, kMmaTruncOut, b[i] + c[i]);
-  }
+  for (int i = 0; i < 8; ++i) y[i] += a[i] + (b[i] + c[i]);
 }
 
 // N results of a thread's row (window columns j0 ..) into a plane: a warp writes 128 bytes of a column at a time.
@@ -324,7 +317,7 @@ template <int N> __device__ __forceinline__ void store_rows(const MmaRowsIO& io,
 // One CTA per SM, its warps in three roles that hand tiles on through mbarriers: eight warps fetch tiles into registers and
 // cut them into operand slices, one issues the matrix products, eight take the results out of tensor memory.  What a tile
 // needs most after HBM is shared memory: of the backward's 4300 clocks (64 KB in and 32 KB out at an SM's share of HBM)
-// the products take 2150 of its time and the writing of their operands 770.  So values go straight from registers into
+// the products take 2432 of its time and the writing of their operands 770.  So values go straight from registers into
 // slices (through a staging copy in shared memory they would take 1020 clocks more: 180 us against 162 for a pass of
 // 16384 x 4096), and all loads of an operand are issued at once (a register load waits on one of six counters, with
 // whatever younger load shares it).  All warps through all steps, one after the other: 290 us.
@@ -337,14 +330,16 @@ constexpr int kFlushTiles = 32;  // row tiles after which the small products of 
 constexpr int kCutRegs = 136, kStoreRegs = 88, kIssueRegs = 32;
 static_assert(128 * (2 * kCutRegs + 2 * kStoreRegs + kIssueRegs) <= kPassThreads * 96, "register split");
 
-template <bool BW> struct PassMem {
+// Shared memory: a pass has only the places that it uses.  Up to 195 KB leave 60 KB of the SM to the loads on their way, a
+// few bytes more leave 28 (three backward passes of 16384 x 4096: 643 us so, 562 within).
+template <bool BW, bool IN_P, bool OUT_P> struct PassMem {
   static constexpr int stages = 2;                // first operand; the backward's second has one place
   static constexpr uint32_t x = stages * kOpBytes;
   static constexpr uint32_t image = x + (BW ? kOpBytes : 0);
   static constexpr int turn_cols = BW ? 16 : 32;  // columns that turn at once on their way to the caller's rows
   static constexpr uint32_t turn = image + kMmaImageBytes;
-  static constexpr uint32_t sums = turn + kStoreWarps * 32 * turn_cols * 4;
-  static constexpr uint32_t control = sums + (BW ? kCutWarps * 64 * 4 : 0);
+  static constexpr uint32_t sums = turn + (OUT_P ? 0 : kStoreWarps * 32 * turn_cols * 4);
+  static constexpr uint32_t control = sums + (BW && !IN_P ? kCutWarps * 64 * 4 : 0);
 };
 // Tensor memory: the transformed tile in 256 columns, twice in the forward; the operator gradient in 256.
 constexpr uint32_t kOuterCol = 256;
@@ -359,7 +354,7 @@ struct Control {
   int special[8];                // the tile (number & 7) holds values that are not finite: the roles are up to six tiles apart
   int failed;                    // a wait ran out
 };
-template <bool BW> constexpr uint32_t pass_bytes() { return PassMem<BW>::control + (uint32_t)sizeof(Control) + 1024; }
+template <typename M> constexpr uint32_t pass_bytes() { return M::control + (uint32_t)sizeof(Control); }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -436,14 +431,17 @@ template <int REGS> __device__ __forceinline__ void registers_down() { asm volat
 
 template <bool BW, bool IN_P, bool X_P, bool OUT_P>
 __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __grid_constant__ MmaPass p, int* err) {
-  typedef PassMem<BW> Mem;
+  typedef PassMem<BW, IN_P, OUT_P> Mem;
   constexpr uint32_t DBUF = BW ? 1 : 2;      // transformed tiles tensor memory holds
   constexpr uint32_t ST = Mem::stages;
-  extern __shared__ uint8_t raw[];
-  uint8_t* sm = raw + ((1024 - (smem_u32(raw) & 1023)) & 1023);
+  extern __shared__ __align__(1024) uint8_t sm[];
   uint8_t* img = sm + Mem::image;
   Control* ctl = reinterpret_cast<Control*>(sm + Mem::control);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  if (smem_u32(sm) & 1023) {  // what the swizzle of the operands counts from
+    if (tid == 0) *err = 2;
+    return;
+  }
   if (tid == 0) {
     for (int i = 0; i < 4; ++i) {
       mbar_init(smem_u32(&ctl->gfull[i]), kCutWarps);
@@ -589,7 +587,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
     registers_down<kStoreRegs>();
     const int e = warp - kStoreWarp0, row = (e & 3) * 32 + lane, j0 = (e >> 2) * 32;
     const uint32_t lanes = (uint32_t)((e & 3) * 32) << 16;
-    float acc[BW ? 32 : 1];  // operator gradient: row `row` (slices 1 and 2 of the incoming gradient), columns j0 ..
+    float acc[BW ? 32 : 1];  // operator gradient: row `row` (two slices of the incoming gradient), columns j0 ..
 #pragma unroll
     for (int i = 0; i < (BW ? 32 : 1); ++i) acc[i] = 0.f;
     float fix[BW ? 64 : 32];  // only for tiles with values that are not finite
@@ -632,32 +630,22 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
         if (!await_warp(ctl, &ctl->pfull, i & 1)) break;
         fence_after_sync();
         const bool last = at.last_of_block(), flush = ++kept == kFlushTiles || last;
+        auto take = [&](uint32_t col, bool use) {  // (all warps together: a branch around the loads cost 30 us of 560)
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          float v[8];
-          tmem_ld8(tmem + kOuterCol + lanes + j0 + 8 * h, v);
-          wait_ld();
+          for (int h = 0; h < 4; ++h) {
+            float v[8], w[8];
+            tmem_ld8(tmem + kOuterCol + col + lanes + j0 + 8 * h, v);
+            tmem_ld8(tmem + kOuterCol + col + 64 + lanes + j0 + 8 * h, w);
+            wait_ld();
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            float& a = acc[BW ? 8 * h + c : 0];
-            a = fmaf(v[c], kMmaTruncGrad, a) + v[c];
+            for (int c = 0; c < 8; ++c)
+              if (use) acc[BW ? 8 * h + c : 0] += v[c] + w[c];
           }
-        }
+        };
+        take(0, row < kMmaCols);
         if (flush) {
           kept = 0;
-#pragma unroll 1
-          for (int k = 1; k < 4; ++k) {
-#pragma unroll
-            for (int h = 0; h < 4; ++h) {
-              float v[8];
-              tmem_ld8(tmem + kOuterCol + 64 * k + lanes + j0 + 8 * h, v);
-              wait_ld();
-              if (k < 3 || row < kMmaCols) {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) acc[BW ? 8 * h + c : 0] += v[c];
-              }
-            }
-          }
+          take(128, true);
         }
         fence_before_sync();
         __syncwarp();
@@ -793,36 +781,45 @@ __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_prep_kernel(c
     off += W * m.radix;
     __syncthreads();
   }
+  // Parts of an entry v: v to a multiple of 2^(E - 3), where 2^E is at most the largest entry of its row or its column, the
+  // larger of the two (exact sums, see above), and three bfloat16 slices of the rest.
+  __shared__ int top[2][kMmaCols];  // exponents of the largest entries of a row, a column
+  auto entry = [&](int j, int i) -> double {
+    if constexpr (CPLX) {
+      const cd z = work[(j >> 1) * W + (i >> 1)];
+      return (j & 1) == (i & 1) ? z.re : ((j & 1) ? z.im : -z.im);
+    } else {
+      return work[j * W + i];
+    }
+  };
+  if (threadIdx.x < 2 * kMmaCols) top[threadIdx.x / kMmaCols][threadIdx.x % kMmaCols] = -1100;
+  __syncthreads();
+  for (int it = threadIdx.x; it < kMmaCols * kMmaCols; it += T) {
+    const int j = it / kMmaCols, i = it % kMmaCols, e = ((__double2hiint(entry(j, i)) >> 20) & 0x7ff) - 1023;
+    atomicMax(&top[0][j], e);
+    atomicMax(&top[1][i], e);
+  }
+  __syncthreads();
   uint8_t* img = p.images + (((int64_t)blockIdx.z * p.S + s) * p.nq + q) * kMmaImageBytes;
   for (int it = threadIdx.x; it < kMmaCols * 8; it += T) {
     const int j = it >> 3, ch = it & 7;
-    uint32_t sl[3][4];
+    uint32_t sl[kMmaParts][4];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const int i = ch * 8 + e;
-      double v;
-      if constexpr (CPLX) {
-        const cd z = work[(j >> 1) * W + (i >> 1)];
-        v = (j & 1) == (i & 1) ? z.re : ((j & 1) ? z.im : -z.im);
-      } else {
-        v = work[j * W + i];
-      }
-      const float f = (float)v, beyond = (float)(v - (double)f);
-      uint32_t b[3];
-      b[0] = __float_as_uint(f) >> 16;
-      float left = f - __uint_as_float(b[0] << 16);
+      const int i = ch * 8 + e, E = min(max(max(top[0][j], top[1][i]), -120), 120);
+      double left = entry(j, i);
 #pragma unroll
-      for (int k = 1; k < 3; ++k) {
+      for (int k = 0; k < kMmaParts; ++k) {
+        float f = (float)left;
+        if (k == 0) f = (float)(rint(left * __hiloint2double((1023 + 3 - E) << 20, 0)) * __hiloint2double((1023 - 3 + E) << 20, 0));
         uint32_t r;
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(0.f), "f"(left));
-        b[k] = r & 0xffffu;
-        left = left - __uint_as_float(b[k] << 16) + beyond;
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(0.f), "f"(f));
+        left -= (double)__uint_as_float(r << 16);
+        sl[k][e >> 1] = (e & 1) ? sl[k][e >> 1] | (r << 16) : (r & 0xffffu);
       }
-#pragma unroll
-      for (int k = 0; k < 3; ++k) sl[k][e >> 1] = (e & 1) ? sl[k][e >> 1] | (b[k] << 16) : b[k];
     }
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
+    for (int k = 0; k < kMmaParts; ++k)
       *reinterpret_cast<uint4*>(img + k * 8192 + j * 128 + ((ch ^ (j & 7)) << 4)) = make_uint4(sl[k][0], sl[k][1], sl[k][2], sl[k][3]);
   }
 }
@@ -974,7 +971,7 @@ template <typename K> int smem_attr(K kernel, uint32_t bytes) {
 int launched() { return cudaGetLastError() == cudaSuccess ? BFLY_OK : BFLY_E_CUDA; }
 
 template <bool BW, bool IN_P, bool X_P, bool OUT_P> int pass_launch(const MmaPass& p, int ctas, cudaStream_t stream, int* err) {
-  constexpr uint32_t bytes = pass_bytes<BW>();
+  constexpr uint32_t bytes = pass_bytes<PassMem<BW, IN_P, OUT_P>>();
   static_assert(bytes <= 227 * 1024, "shared memory of a CTA");
   if (int rc = smem_attr(bfly_mma_pass_kernel<BW, IN_P, X_P, OUT_P>, bytes)) return rc;
   bfly_mma_pass_kernel<BW, IN_P, X_P, OUT_P><<<ctas, kPassThreads, bytes, stream>>>(p, err);

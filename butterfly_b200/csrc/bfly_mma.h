@@ -7,9 +7,10 @@
 // a small kernel takes apart into the gradients of the stages afterwards.  Per pass a tile crosses shared memory once,
 // whatever the number of stages, and the operators' arithmetic costs a quarter of the tile's trip through HBM.
 //
-// Precision.  A float32 value is the exact sum of three bfloat16 values (8 + 8 + 8 bits); products are formed from the
-// six pairs above 2^-24 and summed in float32, the largest apart from the others.  Operators are multiplied out in
-// float64.  tcgen05 truncates its sums: the mean of that loss is added back (kMmaTrunc*).
+// Precision.  A float32 value is the exact sum of three bfloat16 slices (8 + 8 + 8 bits).  Operators are multiplied out in
+// float64 and cut into four parts, the first of few bits.  Nine of the twelve products are formed (the others are below
+// 2^-25 of the whole) and summed in float32 by size.  tcgen05 cuts its sums towards zero, so those that count are kept
+// exact or short (bfly_mma.cu).
 //
 // Columns are counted in floats here: complex rows are rows of 2n floats whose bit 0 tells real from imaginary parts,
 // always inside the window, and a complex operator of 32 x 32 is a real one of 64 x 64.
@@ -33,7 +34,8 @@ constexpr int kMmaCols = 1 << kMmaWin;
 constexpr int kMmaRows = 128;                 // rows of a tile (the lanes of tensor memory)
 constexpr int kMmaMaxStages = 12;             // radix-2 stages a group may hold (a radix-4 factor counts as two)
 constexpr int kMmaMaxGroups = 8;
-constexpr int kMmaImageBytes = 3 * kMmaCols * kMmaCols * 2;  // one operator: three bfloat16 slices, swizzled as tcgen05 reads them
+constexpr int kMmaParts = 4;                  // bfloat16 parts of an operator
+constexpr int kMmaImageBytes = kMmaParts * kMmaCols * kMmaCols * 2;  // one operator, swizzled as tcgen05 reads it
 constexpr int kMmaBwMaxCtas = 160;            // most CTAs of a backward pass (one per SM)
 constexpr int kMmaSlotFloats = 2 * kMmaCols * kMmaCols;      // an operator gradient as a CTA leaves it: two halves to be added
 struct MmaStage {

@@ -163,3 +163,55 @@ def test_the_pair_of_one_buffer_stays_on_the_phases(dev, cplx):
     with abi_option("mma", 0):
         want, want_x, _ = abi.bw(tw, x, g, True)
     assert torch.equal(dx, want_x) and ((d - want).norm() / want.norm()).item() < 1e-6
+
+
+def _factors(kind, shape, dt):
+    """Twiddles, and rows or gradients to go with them."""
+    B, (nb, log_n, half) = 300, shape
+    tw, (x, g) = torch.randn(1, nb, log_n, half, 2, 2, dtype=dt) / 2 ** 0.5, torch.randn(2, B, 1, 2 * half, dtype=dt)
+    eye = torch.eye(2, dtype=dt).expand_as(tw)
+    if kind == "positive":
+        tw, x, g = (t.abs().to(dt) for t in (tw, x, g))
+    elif kind == "uniform":
+        tw, x, g = (torch.rand(t.shape).to(dt) for t in (tw, x, g))
+    elif kind == "one-hot rows":
+        x, g = (t * torch.nn.functional.one_hot(torch.randint(0, 2 * half, (B, 1)), 2 * half) for t in (x, g))
+    elif kind == "sparse rows":
+        x, g = (t * (torch.rand(t.shape) < 0.01) for t in (x, g))
+    elif kind == "near the identity":
+        tw = eye + 1e-3 * tw
+    elif kind == "averages":
+        tw, x, g = torch.full_like(tw, 0.5), x.abs().to(dt), g.abs().to(dt)
+    elif kind == "identity":
+        tw = eye
+    elif kind == "permutation":
+        tw = torch.where(torch.rand(1, nb, log_n, half, 1, 1) < 0.5, eye, eye.flip(-1))
+    elif kind == "powers of two":
+        tw = eye * 2.0 ** torch.randint(-2, 3, (1, nb, log_n, half, 1, 2)) * torch.where(torch.rand(1, nb, log_n, half, 1, 2) < 0.5, 1.0, -1.0)
+    return tw.contiguous(), x, g
+
+
+@pytest.mark.parametrize("cplx,log_n,nblocks,inc", [(False, 10, 2, True), (False, 10, 1, True), (False, 9, 2, False), (True, 8, 2, True)])
+@pytest.mark.parametrize("kind", ["normal", "positive", "uniform", "one-hot rows", "sparse rows", "near the identity", "averages", "identity",
+                                  "permutation", "powers of two"])
+def test_no_further_from_float64_than_the_phases(dev, oracle_mod, kind, cplx, log_n, nblocks, inc):
+    """Whatever the distribution.  A pass rounds each result once where the phases round once per factor; factors that only
+    move and scale columns give every bit back.  Gradients of the factors, sums over the rows, have a bound of their own: the
+    tensor cores' accumulators cut four times, half of 2^-23 each, and rows and gradients carry the error of up to three passes."""
+    import butterfly_b200 as bb
+    dt, wide = (torch.complex64, torch.complex128) if cplx else (torch.float32, torch.float64)
+    torch.manual_seed(log_n + nblocks)
+    tw, x, g = _factors(kind, (nblocks, log_n, 1 << (log_n - 1)), dt)
+    want_y = oracle_mod.multiply_fw(tw.to(wide), x.to(wide), inc)
+    want_d, want_dx = oracle_mod.multiply_bw(tw.to(wide), x.to(wide), g.to(wide), inc)
+    err = []
+    for mma in (0, 1):
+        with abi_option("mma", mma), abi_option("autograd_save", 1):
+            t, xd = tw.to(dev).requires_grad_(True), x.to(dev).requires_grad_(True)
+            y = bb.butterfly_multiply(t, xd, inc)
+            d, dx = torch.autograd.grad(y, [t, xd], g.to(dev))
+        err.append([rel2(y, want_y), rel2(dx, want_dx), rel2(d, want_d)])
+    phases, passes = err
+    assert passes[0] <= phases[0] and passes[1] <= phases[1] and passes[2] < 4 * 2 ** -24 + 3 * 2 ** -24
+    if kind in ("identity", "permutation", "powers of two"):
+        assert passes[:2] == [0.0, 0.0]
