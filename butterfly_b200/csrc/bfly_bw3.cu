@@ -22,6 +22,7 @@ bfly_bw3_kernel(const __grid_constant__ Bw3Params p, const __grid_constant__ CUt
                 const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_o, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const BwParams<float>& q = p.b;
+  if (q.guard && !*q.guard) return;
   float* sm = reinterpret_cast<float*>(smem);
   const uint32_t sm0 = tma_smem(smem);
   uint32_t* meta = reinterpret_cast<uint32_t*>(smem + bw3_tile_bytes(p));

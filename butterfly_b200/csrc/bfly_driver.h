@@ -21,6 +21,7 @@
 //   static constexpr bool kMma;                            // optional: the tensor-core passes (bfly_mma.h) are available:
 //   int  mma_prep(const MmaPrep&, bool cplx); int mma_fw(const MmaPass&); int mma_bw(const MmaPass&, int ctas);
 //   int  mma_post(const MmaPost&, bool cplx);
+//   const int* guard;                                      // with kMma: launches run only if *guard is not 0 (null: all run)
 #pragma once
 #include <cstdlib>
 #include <cstring>
@@ -382,6 +383,9 @@ int drive_fw2_view(E& ex, const Problem& q, const std::vector<Stage>& st, int t0
   return BFLY_OK;
 }
 
+template <typename T> struct BwLayout;
+template <typename T> int plan_bw(const Problem& q, BwLayout<T>& lay);
+
 // ------------------------------------------------------------------ products on the tensor cores (bfly_mma.h)
 
 template <typename E, typename = void> struct has_mma : std::false_type {};
@@ -407,6 +411,9 @@ inline bool mma_pays(const Problem& q, int F, int ng) {
   return passes * 1.12 < phases;
 }
 
+// What the phases need behind the passes, for values that are not ordinary; negative where they do not run.
+template <typename T> inline int64_t phases_bw_bytes(const Problem& q);
+
 // Does a training step of this shape run as tensor-core passes, and how?  Only shapes and the option decide, so that a
 // backward finds the planes its forward left.
 template <typename T> inline bool mma_layout(const Problem& q, MmaLayout& L) {
@@ -430,7 +437,11 @@ template <typename T> inline bool mma_layout(const Problem& q, MmaLayout& L) {
   L.images = ng * q.S * L.nq * kMmaImageBytes;
   L.slots = ng * slots * kMmaSlotFloats * sizeof(float);
   L.bias_slots = slots * kMmaCols * sizeof(float);
-  return true;
+  return phases_bw_bytes<T>(q) >= 0;
+}
+// Work space of the backward of the operator: the passes', or what the phases need instead of it.
+template <typename T> inline size_t mma_bw_need(const Problem& q, const MmaLayout& L, bool from_kept) {
+  return std::max(L.bw_bytes(from_kept), kMmaHead + (size_t)phases_bw_bytes<T>(q));
 }
 // The layout of either direction of a problem, for queries that do not name one: the larger need.
 template <typename T, typename F> inline int64_t mma_either(Problem q, F&& bytes) {
@@ -438,7 +449,7 @@ template <typename T, typename F> inline int64_t mma_either(Problem q, F&& bytes
   for (int inc = 0; inc < 2; ++inc) {
     q.inc = inc != 0;
     MmaLayout L;
-    if (mma_layout<T>(q, L)) best = std::max<int64_t>(best, (int64_t)bytes(L));
+    if (mma_layout<T>(q, L)) best = std::max<int64_t>(best, (int64_t)bytes(q, L));
   }
   return best;
 }
@@ -463,39 +474,52 @@ inline char* mma_align(void* p, size_t& bytes) {
   return static_cast<char*>(p) + skip;
 }
 
+// The phases behind the passes: what `f` launches runs only if the flag is up.  Launches that find it down take about 2.5 us
+// each (complex 1024 columns, two blocks, 8192 rows: ten of them, 317 us without and 343 with).
+template <typename E, typename F> int behind_flag(E& ex, const char* head, F&& f) {
+  ex.guard = reinterpret_cast<const int*>(head);
+  const int rc = f();
+  ex.guard = nullptr;
+  return rc;
+}
+
 template <typename T, typename E>
-int mma_run_prep(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, const T* tw4, uint8_t* images) {
+int mma_run_prep(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, const T* tw4, uint8_t* images, int* flag) {
   MmaPrep p;
   std::memset(&p, 0, sizeof(p));
   p.tw[0] = tw2; p.tw[1] = tw4;
   twiddle_stack_sizes(q, p.tw_stack);
   p.S = q.S; p.nq = L.nq; p.ng = (int)L.g.size();
-  p.images = images;
+  p.images = images; p.flag = flag;
+  if (int rc = ex.zero(flag, sizeof(int))) return rc;
   for (int i = 0; i < p.ng; ++i) p.g[i] = L.g[i];
   return ex.mma_prep(p, sizeof(T) == 8);
 }
 
-inline MmaPass mma_pass(const Problem& q, const MmaLayout& L, int g, const uint8_t* images) {
+inline MmaPass mma_pass(const Problem& q, const MmaLayout& L, int g, const uint8_t* images, int* flag) {
   MmaPass p;
   std::memset(&p, 0, sizeof(p));
   p.geo = L.g[g].geo;
   p.S = q.S; p.B = q.B; p.nq = L.nq; p.nt = (int)L.nt;
   p.images = images + (size_t)g * q.S * L.nq * kMmaImageBytes;
+  p.flag = flag;
   return p;
 }
 
-// Forward; the activations between the groups stay in `kept`, then the operators.  Groups [0, last_group) only when the
-// output is not wanted.
+// Forward; the flag, the activations between the groups and then the operators stay in `kept`.  The last group only when
+// the output is wanted.
 template <typename T, typename E>
 int drive_mma_fw(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, const T* tw4, const T* x, int64_t x_sB, int64_t x_sS, T* out, int out_cols,
                  const T* bias, int bias_len, char* kept) {
   constexpr int F = (int)(sizeof(T) / 4);
   const int64_t n = (int64_t)1 << q.log_n;
   const int ng = (int)L.g.size();
+  int* flag = reinterpret_cast<int*>(kept);
+  kept += kMmaHead;
   uint8_t* images = reinterpret_cast<uint8_t*>(kept) + (ng - 1) * L.plane;
-  if (int rc = mma_run_prep(ex, q, L, tw2, tw4, images)) return rc;
+  if (int rc = mma_run_prep(ex, q, L, tw2, tw4, images, flag)) return rc;
   for (int g = 0; g < (out ? ng : ng - 1); ++g) {
-    MmaPass p = mma_pass(q, L, g, images);
+    MmaPass p = mma_pass(q, L, g, images, flag);
     if (g == 0) p.in = mma_rows<T>(x, x_sB, x_sS, q.in_size, q.S);
     else p.in_t = reinterpret_cast<const float*>(kept + (g - 1) * L.plane);
     if (g + 1 < ng) {
@@ -510,7 +534,7 @@ int drive_mma_fw(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, cons
 }
 
 // Backward.  dx: rows of the input gradient, added to when `reduce`; d_bias (column sums of the gradient) may be null.
-// `kept`: what the forward left, untouched here, or null.
+// `kept`: what the forward left, untouched here, or null.  The flag is the first word of `ws`, in either case.
 template <typename T, typename E>
 int drive_mma_bw(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, const T* tw4, const T* x, int64_t x_sB, int64_t x_sS, const MmaRowsIO& grad,
                  const MmaRowsIO& dx, bool reduce, T* d_tw2, T* d_tw4, T* d_bias, int bias_len, const char* kept, char* ws, size_t ws_bytes) {
@@ -518,20 +542,26 @@ int drive_mma_bw(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, cons
   if (ws_bytes < L.bw_bytes(kept != nullptr)) return BFLY_E_WORKSPACE;
   const int ng = (int)L.g.size();
   const size_t slots_per_group = (size_t)q.S * L.nq + kMmaBwMaxCtas;
-  char* gplane = ws;
-  float* slots = reinterpret_cast<float*>(ws + (kept ? (ng > 1 ? L.plane : 0) : L.kept()));
+  char* gplane = ws + kMmaHead;
+  int* flag = reinterpret_cast<int*>(ws);
+  const int* kept_flag = reinterpret_cast<const int*>(kept);
+  float* slots = reinterpret_cast<float*>(ws + (kept ? kMmaHead + (ng > 1 ? L.plane : 0) : L.kept()));
   float* bias_slots = reinterpret_cast<float*>(reinterpret_cast<char*>(slots) + L.slots);
   if (!kept) {
     if (int rc = drive_mma_fw<T>(ex, q, L, tw2, tw4, x, x_sB, x_sS, (T*)nullptr, 0, (const T*)nullptr, 0, ws)) return rc;
     kept = ws;
-    if (ng > 1) gplane = ws + (ng - 2) * L.plane;  // a tile's activations are read before its gradient is written
+    if (ng > 1) gplane += (ng - 2) * L.plane;  // a tile's activations are read before its gradient is written
+  } else if (int rc = ex.zero(flag, sizeof(int))) {
+    return rc;
   }
+  kept += kMmaHead;
   const uint8_t* images = reinterpret_cast<const uint8_t*>(kept) + (ng - 1) * L.plane;
   const int ctas = (int)std::min<int64_t>(std::min(ex.num_sms(), kMmaBwMaxCtas), (int64_t)q.S * L.nq * L.nt);
   for (int g = ng - 1; g >= 0; --g) {
-    MmaPass p = mma_pass(q, L, g, images);
+    MmaPass p = mma_pass(q, L, g, images, flag);
     if (g == ng - 1) {
       p.in = grad;
+      p.kept_flag = kept_flag;
       if (d_bias) p.bias_slots = bias_slots;
     } else {
       p.in_t = reinterpret_cast<const float*>(gplane);
@@ -548,6 +578,7 @@ int drive_mma_bw(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, cons
   p.tw[0] = tw2; p.tw[1] = tw4; p.dtw[0] = d_tw2; p.dtw[1] = d_tw4;
   twiddle_stack_sizes(q, p.tw_stack);
   p.S = q.S; p.nq = L.nq; p.nt = (int)L.nt; p.ng = ng; p.ctas = ctas; p.last_group = ng - 1;
+  p.flag = flag;
   p.slots = slots; p.slots_group = (int64_t)slots_per_group * kMmaSlotFloats;
   if (d_bias) { p.bias_slots = bias_slots; p.dbias = reinterpret_cast<float*>(d_bias); p.dbias_len = bias_len * F; }
   for (int i = 0; i < ng; ++i) p.g[i] = L.g[i];
@@ -720,9 +751,6 @@ template <typename T> inline size_t fw_workspace_bytes(const Problem& q) {
   return fw2_packed_bytes(q.S, q.log_n, q.nblocks);
 }
 
-template <typename T> struct BwLayout;
-template <typename T> int plan_bw(const Problem& q, BwLayout<T>& lay);
-
 template <typename T> struct BwLayout {
   std::vector<BwPhase> phases;
   int kw;
@@ -755,6 +783,12 @@ int plan_bw(const Problem& q, BwLayout<T>& lay) {
   return BFLY_OK;
 }
 
+template <typename T> inline int64_t phases_bw_bytes(const Problem& q) {
+  BwLayout<T> lay;
+  const int rc = plan_bw<T>(q, lay);
+  return rc ? rc : (int64_t)lay.ws_bytes;
+}
+
 // Work space of a backward that is told nothing but the sizes: the phase plan depends on the direction of the first block, so
 // the larger need of the two.
 template <typename T> inline int64_t bw_workspace_need(const Problem& q0) {
@@ -767,10 +801,7 @@ template <typename T> inline int64_t bw_workspace_need(const Problem& q0) {
     if (rc) return rc;
     best = std::max<int64_t>(best, (int64_t)lay.ws_bytes);
   }
-  // tensor-core passes: at least a plane per group, like the phases with the forward's scratch behind it
-  return std::max(best, mma_either<T>(q0, [&](const MmaLayout& L) {
-    return std::max(L.bw_bytes(false) + kMmaSpare, L.g.size() * L.plane) + (q0.base4 ? 0 : fw_workspace_bytes<T>(q0));
-  }));
+  return std::max(best, mma_either<T>(q0, [&](const Problem& q, const MmaLayout& L) { return mma_bw_need<T>(q, L, false) + kMmaSpare; }));
 }
 // What a saving forward has to leave for the backward, again for either direction: one of them may run as tensor-core passes
 // and the other as phases (float, 4096 columns, two blocks: three groups of stages one way, five the other).
@@ -807,7 +838,10 @@ int drive_fw_saving(E& ex, const Problem& q, const T* tw2, const T* tw4, const T
     if (mma_layout<T>(q, L)) {
       char* kept = mma_align(ws, ws_bytes);
       if (!kept || ws_bytes < L.kept()) return BFLY_E_WORKSPACE;
-      return drive_mma_fw<T>(ex, q, L, tw2, tw4, x, x_sB, x_sS, out, q.out_size, (const T*)nullptr, 0, kept);
+      rc = drive_mma_fw<T>(ex, q, L, tw2, tw4, x, x_sB, x_sS, out, q.out_size, (const T*)nullptr, 0, kept);
+      if (rc != BFLY_OK) return rc;
+      // (what was kept is of no use if the flag is up: room for the twiddles in the phases' order)
+      return behind_flag(ex, kept, [&] { return drive_fw<T>(ex, q, tw2, tw4, x, x_sB, x_sS, out, kept + kMmaHead, L.kept() - kMmaHead); });
     }
   }
   BwLayout<T> lay;
@@ -854,13 +888,18 @@ int drive_bw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T* x, in
       size_t work_bytes = snapshots_ready ? extra_bytes : ws_bytes;
       char* work = mma_align(snapshots_ready ? extra : ws, work_bytes);
       const char* kept = snapshots_ready ? mma_align(ws, ws_bytes) : nullptr;
-      if (!work || (snapshots_ready && (!kept || ws_bytes < L.kept()))) return BFLY_E_WORKSPACE;
+      if (!work || work_bytes < mma_bw_need<T>(q, L, kept != nullptr) || (snapshots_ready && (!kept || ws_bytes < L.kept()))) return BFLY_E_WORKSPACE;
       const int64_t n = (int64_t)1 << q.log_n, DX = std::max<int64_t>(q.in_size, n);
       rc = drive_mma_bw<T>(ex, q, L, tw2, tw4, x, x_sB, x_sS, mma_rows<T>(grad, g_sB, g_sS, q.out_size, q.S, gin_flat),
                            mma_rows<T>(d_x, (int64_t)q.S * DX, DX, (int)std::min<int64_t>(q.in_size, n), q.S), false, d_tw2, d_tw4, (T*)nullptr, 0,
                            kept, work, work_bytes);
-      if (rc != BFLY_OK || q.in_size <= n) return rc;
-      return ex.zero2d(d_x + n, (size_t)DX * sizeof(T), (size_t)(q.in_size - n) * sizeof(T), (size_t)q.B * q.S);
+      if (rc == BFLY_OK && q.in_size > n) rc = ex.zero2d(d_x + n, (size_t)DX * sizeof(T), (size_t)(q.in_size - n) * sizeof(T), (size_t)q.B * q.S);
+      if (rc != BFLY_OK) return rc;
+      Problem stages = q;
+      stages.phases = true;
+      return behind_flag(ex, work, [&] {
+        return drive_bw<T>(ex, stages, tw2, tw4, x, x_sB, x_sS, grad, g_sB, g_sS, d_tw2, d_tw4, d_x, work + kMmaHead, work_bytes - kMmaHead, false, gin_flat);
+      });
     }
   }
   if (stk[0]) { rc = ex.zero(d_tw2, (size_t)q.S * stk[0] * sizeof(T)); if (rc) return rc; }
@@ -1032,7 +1071,11 @@ int drive_layer_fw(E& ex, const Problem& q, const T* tw2, const T* tw4, const T*
     if (snapshots && out_total > 0 && mma_layout<T>(q, M)) {
       char* kept = mma_align(snapshots, snapshot_bytes);
       if (!kept || snapshot_bytes < M.kept()) return BFLY_E_WORKSPACE;
-      return drive_mma_fw<T>(ex, q, M, tw2, tw4, x, x_sB, 0, out, (int)n, bias, out_total, kept);
+      rc = drive_mma_fw<T>(ex, q, M, tw2, tw4, x, x_sB, 0, out, (int)n, bias, out_total, kept);
+      if (rc != BFLY_OK) return rc;
+      return behind_flag(ex, kept, [&] {
+        return drive_layer_fw<T>(ex, q, tw2, tw4, x, x_sB, out, bias, out_total, nullptr, 0, kept + kMmaHead, M.kept() - kMmaHead);
+      });
     }
   }
   T* snaps[kMaxSnap] = {nullptr};
@@ -1233,7 +1276,9 @@ template <typename T> inline bool mma_layer_adds(const Problem& q, int out_total
 }
 template <typename T> inline size_t mma_layer_bw_bytes(const Problem& q, int out_total, const MmaLayout& M, bool saved) {
   const int64_t DX = std::max<int64_t>(q.in_size, (int64_t)1 << q.log_n);
-  return M.bw_bytes(saved) + (q.S > 1 && !mma_layer_adds<T>(q, out_total) ? (size_t)q.B * q.S * DX * sizeof(T) : 0);
+  LayerBwLayout L;
+  if (plan_layer_bw<T>(q, out_total, false, L) != BFLY_OK) L.ws_bytes = 0;  // (mma_layout asked)
+  return std::max(M.bw_bytes(saved) + (q.S > 1 && !mma_layer_adds<T>(q, out_total) ? (size_t)q.B * q.S * DX * sizeof(T) : 0), kMmaHead + L.ws_bytes);
 }
 template <typename T, typename E>
 int drive_mma_layer_bw(E& ex, const Problem& q, const MmaLayout& M, const T* tw2, const T* tw4, const T* x, int64_t x_sB, const T* grad, int64_t g_sB,
@@ -1278,7 +1323,13 @@ int drive_layer_bw(E& ex, const Problem& q_in, const T* tw2, const T* tw4, const
       twiddle_stack_sizes(q, stk);
       if (twiddle_missing(q, tw2, tw4) || (stk[0] && !d_tw2) || (stk[1] && !d_tw4)) return BFLY_E_ARG;
       if ((tw2 && !aligned16(tw2)) || (tw4 && !aligned16(tw4)) || (d_tw2 && !aligned16(d_tw2)) || (d_tw4 && !aligned16(d_tw4))) return BFLY_E_ALIGN;
-      return drive_mma_layer_bw<T>(ex, q, M, tw2, tw4, x, x_sB, grad, g_sB, d_tw2, d_tw4, d_in, d_bias, out_total, saved, saved_bytes, ws, ws_bytes);
+      rc = drive_mma_layer_bw<T>(ex, q, M, tw2, tw4, x, x_sB, grad, g_sB, d_tw2, d_tw4, d_in, d_bias, out_total, saved, saved_bytes, ws, ws_bytes);
+      if (rc != BFLY_OK) return rc;
+      char* work = mma_align(ws, ws_bytes);
+      q.phases = true;
+      return behind_flag(ex, work, [&] {
+        return drive_layer_bw<T>(ex, q, tw2, tw4, x, x_sB, grad, g_sB, d_tw2, d_tw4, d_in, d_bias, out_total, nullptr, 0, work + kMmaHead, ws_bytes - kMmaHead);
+      });
     }
   }
   q.phases = true;  // as the forward went, and as the work space is laid out

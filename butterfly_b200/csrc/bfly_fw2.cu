@@ -80,6 +80,7 @@ template <int CTAS, int THREADS, bool TAIL>
 __global__ void __launch_bounds__(THREADS, CTAS)
 bfly_fw2_kernel(const __grid_constant__ Fw2Params p, const __grid_constant__ Fw2Maps maps, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
+  if (p.guard && !*p.guard) return;  // (set before the re-ordering kernel began)
   float* tile = reinterpret_cast<float*>(smem);
   const uint32_t smem0 = tma_smem(smem);
   const uint32_t tile_bytes = (uint32_t)fw2_tile_bytes(p);
@@ -239,6 +240,7 @@ bfly_fw2_kernel(const __grid_constant__ Fw2Params p, const __grid_constant__ Fw2
 // Re-orders the twiddles of the launch into the per-thread order the kernel loads (fw2_pack_entry).
 __global__ void __launch_bounds__(256) bfly_fw2_pack_kernel(const __grid_constant__ Fw2Params p) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (p.guard && !*p.guard) return;
   const int64_t n = fw2_pack_entries(p);
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     float q[4];
@@ -256,7 +258,8 @@ __global__ void __launch_bounds__(256) bfly_fw2_pack_kernel(const __grid_constan
 // out[b, f] += bias[f] for f < len on a (B, width) matrix with row pitch `pitch`: the bias of a
 // fused linear layer when the forward ran on a kernel without the bias epilogue.
 __global__ void __launch_bounds__(256) bfly_bias_kernel(float* __restrict__ out, const float* __restrict__ bias, int64_t B,
-                                                         int len, int64_t pitch) {
+                                                         int len, int64_t pitch, const int* guard) {
+  if (guard && !*guard) return;
   const int64_t total = B * len;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / len;
@@ -264,10 +267,10 @@ __global__ void __launch_bounds__(256) bfly_bias_kernel(float* __restrict__ out,
     out[r * pitch + f] += __ldg(bias + f);
   }
 }
-int bias_add_launch(float* out, const float* bias, int64_t B, int len, int64_t pitch, int sms, cudaStream_t stream) {
+int bias_add_launch(float* out, const float* bias, int64_t B, int len, int64_t pitch, const int* guard, int sms, cudaStream_t stream) {
   if (B <= 0 || len <= 0) return BFLY_OK;
   const int64_t blocks = std::min<int64_t>((B * len + 255) / 256, (int64_t)sms * 8);
-  bfly_bias_kernel<<<(int)blocks, 256, 0, stream>>>(out, bias, B, len, pitch);
+  bfly_bias_kernel<<<(int)blocks, 256, 0, stream>>>(out, bias, B, len, pitch, guard);
   return cudaGetLastError() == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
 }
 
@@ -276,7 +279,8 @@ int bias_add_launch(float* out, const float* bias, int64_t B, int len, int64_t p
 // is one slice, else a matrix whose columns a second launch sums, so that every sum has one order whatever the schedule.
 template <int LANES>
 __global__ void __launch_bounds__(32 * LANES) bfly_column_sums_kernel(const float* __restrict__ g, int64_t pitch, int64_t B, int cols,
-                                                                       float* __restrict__ out, int64_t rows_per_slice) {
+                                                                       float* __restrict__ out, int64_t rows_per_slice, const int* guard) {
+  if (guard && !*guard) return;
   __shared__ float part[LANES][33];
   const int c = blockIdx.x * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
   const int64_t r0 = blockIdx.y * rows_per_slice, r1 = r0 + rows_per_slice < B ? r0 + rows_per_slice : B;
@@ -299,7 +303,7 @@ __global__ void __launch_bounds__(32 * LANES) bfly_column_sums_kernel(const floa
     out[(int64_t)blockIdx.y * cols + c] = acc;
   }
 }
-int column_sums_launch(const float* g, int64_t pitch, int64_t B, int cols, float* out, float* partial, cudaStream_t stream, int* launches) {
+int column_sums_launch(const float* g, int64_t pitch, int64_t B, int cols, float* out, float* partial, const int* guard, cudaStream_t stream, int* launches) {
   *launches = 0;
   if (cols <= 0) return BFLY_OK;
   const int gx = (cols + 31) / 32;
@@ -307,8 +311,8 @@ int column_sums_launch(const float* g, int64_t pitch, int64_t B, int cols, float
   if (s.count > 1 && !partial) return BFLY_E_WORKSPACE;
   auto launch = [&](const float* src, int64_t row_pitch, int64_t rows, float* dst, int64_t slices, int64_t per_slice) {
     const dim3 grid(gx, (unsigned)slices);
-    if (slices == 1 && rows > 64) bfly_column_sums_kernel<32><<<grid, 1024, 0, stream>>>(src, row_pitch, rows, cols, dst, per_slice);
-    else bfly_column_sums_kernel<8><<<grid, 256, 0, stream>>>(src, row_pitch, rows, cols, dst, per_slice);
+    if (slices == 1 && rows > 64) bfly_column_sums_kernel<32><<<grid, 1024, 0, stream>>>(src, row_pitch, rows, cols, dst, per_slice, guard);
+    else bfly_column_sums_kernel<8><<<grid, 256, 0, stream>>>(src, row_pitch, rows, cols, dst, per_slice, guard);
     ++*launches;
   };
   launch(g, pitch, B, s.count > 1 ? partial : out, s.count, s.rows);
@@ -317,7 +321,8 @@ int column_sums_launch(const float* g, int64_t pitch, int64_t B, int cols, float
 }
 // Input gradient of a layer whose stacks share their input.
 __global__ void __launch_bounds__(256) bfly_stack_sums_kernel(const float* __restrict__ g, int64_t B, int S, int64_t n, int cols,
-                                                               float* __restrict__ out) {
+                                                               float* __restrict__ out, const int* guard) {
+  if (guard && !*guard) return;
   const int64_t total = B * cols;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = e / cols;
@@ -328,10 +333,21 @@ __global__ void __launch_bounds__(256) bfly_stack_sums_kernel(const float* __res
     out[e] = acc;
   }
 }
-int stack_sums_launch(const float* g, int64_t B, int S, int64_t n, int cols, float* out, int sms, cudaStream_t stream) {
+int stack_sums_launch(const float* g, int64_t B, int S, int64_t n, int cols, float* out, const int* guard, int sms, cudaStream_t stream) {
   if (B <= 0 || cols <= 0) return BFLY_OK;
   const int64_t blocks = std::min<int64_t>((B * cols + 255) / 256, (int64_t)sms * 16);
-  bfly_stack_sums_kernel<<<(int)blocks, 256, 0, stream>>>(g, B, S, n, cols, out);
+  bfly_stack_sums_kernel<<<(int)blocks, 256, 0, stream>>>(g, B, S, n, cols, out, guard);
+  return cudaGetLastError() == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
+}
+
+// A memset that runs only if *guard is not 0 by then: `rows` times `width` bytes, multiples of four.
+__global__ void __launch_bounds__(256) bfly_guarded_zero_kernel(uint32_t* __restrict__ p, int64_t pitch, int64_t width, int64_t rows, const int* guard) {
+  if (!*guard) return;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < width * rows; e += (int64_t)gridDim.x * blockDim.x)
+    p[e / width * pitch + e % width] = 0u;
+}
+int guarded_zero_launch(void* p, size_t pitch, size_t width, size_t rows, const int* guard, int sms, cudaStream_t stream) {
+  bfly_guarded_zero_kernel<<<sms, 256, 0, stream>>>(static_cast<uint32_t*>(p), (int64_t)(pitch / 4), (int64_t)(width / 4), (int64_t)rows, guard);
   return cudaGetLastError() == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
 }
 

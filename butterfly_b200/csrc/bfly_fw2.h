@@ -164,6 +164,7 @@ struct Fw2Params {
   int view;
   int view_row;
   Panel panel;
+  const int* guard;  // optional: nothing runs while *guard is 0
   int threads;       // threads per CTA: 0 = 256; 512 for rows of 8192 columns (one CTA per SM)
   int ngroups;
   Fw2Group g[kFw2MaxGroups];

@@ -117,6 +117,7 @@ struct FwMaps {
 template <typename T, int KMAX, int LOGC, int ROWS, bool TMA, bool GLUE>
 __global__ void __launch_bounds__(kThreads, (FwOcc<T, KMAX>::kMinBlocks))
 bfly_fw_kernel(const __grid_constant__ FwParams<T> p, const __grid_constant__ FwMaps maps) {
+  if (p.guard && !*p.guard) return;
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   // the swizzle of the TMA unit works on address bits: the tile starts on a 1024-byte boundary
   unsigned char* smem_raw = smem_dyn + ((1024u - (tma_smem(smem_dyn) & 1023u)) & 1023u);
@@ -252,6 +253,7 @@ template <typename T, int KW, int NSG, int LOGC, int RB>
 __global__ void __launch_bounds__(kThreads, (BwOcc<T, KW, NSG>::kMinBlocks))
 bfly_bw_kernel(const __grid_constant__ BwParams<T> p, const __grid_constant__ CUtensorMap map_x,
                const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_o) {
+  if (p.guard && !*p.guard) return;
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   unsigned char* smem_raw = smem_dyn + ((1024u - (tma_smem(smem_dyn) & 1023u)) & 1023u);
   T* smX = reinterpret_cast<T*>(smem_raw);
@@ -352,6 +354,7 @@ template <typename T, int KW, int LOGC>
 __global__ void __launch_bounds__(kThreads, 2)
 bfly_bw2_kernel(const __grid_constant__ BwParams<T> p, const __grid_constant__ CUtensorMap map_x,
                 const __grid_constant__ CUtensorMap map_g, const __grid_constant__ CUtensorMap map_o) {
+  if (p.guard && !*p.guard) return;
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   // the swizzle of the TMA unit works on address bits: tiles start on a 1024-byte boundary
   unsigned char* smem_raw = smem_dyn + ((1024u - (tma_smem(smem_dyn) & 1023u)) & 1023u);
@@ -489,9 +492,9 @@ struct ProfileScope {
   cudaStream_t stream;
   bool on = false;
   ProfileRec rec{};
-  ProfileScope(int id, cudaStream_t s) : stream(s) {
+  ProfileScope(int id, cudaStream_t s, const int* guard = nullptr) : stream(s) {  // (guarded launches hardly ever do anything)
     std::lock_guard<std::mutex> lk(g_prof_mu);
-    if (!g_prof_on) return;
+    if (!g_prof_on || guard) return;
     if (cudaEventCreate(&rec.a) != cudaSuccess) return;
     if (cudaEventCreate(&rec.b) != cudaSuccess) { cudaEventDestroy(rec.a); return; }
     rec.id = id;
@@ -566,6 +569,7 @@ static int set_smem(K kernel, size_t bytes) {
 struct CudaExec {
   cudaStream_t stream;
   DeviceInfo dev;
+  const int* guard = nullptr;  // while set, what is launched runs only if *guard is not 0 by then
   int num_sms() const { return dev.sms; }
   int threads() const { return kThreads; }
   static bool use_tma() { return options().tma != 0; }
@@ -573,6 +577,7 @@ struct CudaExec {
 
   template <typename T, int KW, int LOGC> int launch_bw2(const BwParams<T>& p_in) {
     BwParams<T> p = p_in;
+    p.guard = guard;
     const size_t smem = bw2_smem_bytes(p, kThreads) + 32 + 1024;  // TMEM slot, two mbarriers, alignment slack
     int rc = set_smem(bfly_bw2_kernel<T, KW, LOGC>, smem);
     if (rc) return rc;
@@ -580,7 +585,7 @@ struct CudaExec {
     CUtensorMap mx, mg, mo;
     describe_bw(p, kBw2Rows, mx, mg, mo);
     {
-      ProfileScope prof(kKernBw2, stream);
+      ProfileScope prof(kKernBw2, stream, guard);
       bfly_bw2_kernel<T, KW, LOGC><<<bw_num_ctas(p), kThreads, smem, stream>>>(p, mx, mg, mo);
     }
     g_launches.fetch_add(1);
@@ -589,6 +594,7 @@ struct CudaExec {
 
   template <typename T, int KMAX, int LOGC, int ROWS> int launch_fw(const FwParams<T>& p_in) {
     FwParams<T> p = p_in;
+    p.guard = guard;
     const size_t smem = fw_smem_bytes(p, kThreads) + 16 + 1024;  // mbarrier, alignment slack
     // the TMA variant exists for the instances with a compile-time tile shape (the generic
     // instances have no registers to spare for it)
@@ -618,7 +624,7 @@ struct CudaExec {
     p.tma_sx = (p.S > 1 && p.x_sS != 0); p.tma_so = (p.S > 1 && p.out_sS != 0);
     p.tma_pbe = geo.pbe; p.tma_f = F;
     {
-      ProfileScope prof(kKernFw, stream);
+      ProfileScope prof(kKernFw, stream, guard);
       bool launched = false;
       if constexpr (kTmaInstance) {
         if (tma) {
@@ -647,13 +653,15 @@ struct CudaExec {
     }
     return launch_fw<T, KMAX, 0, 0>(p);
   }
-  int run_fw2(const Fw2Params& p, int ctas_per_sm) {
+  int run_fw2(const Fw2Params& p_in, int ctas_per_sm) {
+    Fw2Params p = p_in;
+    p.guard = guard;
     int* err = nullptr;
     int rc = device_error_ptr(&err);
     if (rc) return rc;
     int launches = 0;
     {
-      ProfileScope prof(kKernFw2, stream);
+      ProfileScope prof(kKernFw2, stream, guard);
       rc = fw2_launch(p, ctas_per_sm, dev.sms, stream, err, &launches);
     }
     if (rc == BFLY_OK) g_launches.fetch_add(launches);
@@ -667,6 +675,7 @@ struct CudaExec {
   }
   int run_bw3(const Bw3Params& p_in) {
     Bw3Params p = p_in;
+    p.b.guard = guard;
     CUtensorMap mx, mg, mo;
     describe_bw(p.b, kBw3Rows, mx, mg, mo);
     if (!p.b.tma) return kFw2Declined;
@@ -674,7 +683,7 @@ struct CudaExec {
     int rc = device_error_ptr(&err);
     if (rc) return rc;
     {
-      ProfileScope prof(kKernBw3, stream);
+      ProfileScope prof(kKernBw3, stream, guard);
       rc = bw3_launch(p, mx, mg, mo, stream, err);
     }
     if (rc == BFLY_OK) g_launches.fetch_add(1);
@@ -705,13 +714,14 @@ struct CudaExec {
 
   template <typename T, int KW, int NSG, int LOGC, int RB> int launch_bw(const BwParams<T>& p_in) {
     BwParams<T> p = p_in;
+    p.guard = guard;
     const size_t smem = ((size_t)(p.nsg + 1) * p.Rb * sizeof(T) << p.panel.logC) + 16 + 1024;  // two mbarriers, alignment slack
     int rc = set_smem(bfly_bw_kernel<T, KW, NSG, LOGC, RB>, smem);
     if (rc) return rc;
     CUtensorMap mx, mg, mo;
     describe_bw(p, p.Rb, mx, mg, mo);
     {
-      ProfileScope prof(kKernBw, stream);
+      ProfileScope prof(kKernBw, stream, guard);
       bfly_bw_kernel<T, KW, NSG, LOGC, RB><<<bw_num_ctas(p), kThreads, smem, stream>>>(p, mx, mg, mo);
     }
     g_launches.fetch_add(1);
@@ -744,7 +754,7 @@ struct CudaExec {
   }
   static constexpr bool kFusedBias = true;  // run_fw adds FwParams::bias
   int add_bias(float* out, const float* bias, int64_t B, int len, int64_t pitch) {
-    const int rc = bias_add_launch(out, bias, B, len, pitch, dev.sms, stream);
+    const int rc = bias_add_launch(out, bias, B, len, pitch, guard, dev.sms, stream);
     if (rc == BFLY_OK) g_launches.fetch_add(1);
     return rc;
   }
@@ -752,14 +762,14 @@ struct CudaExec {
   template <typename T> int column_sums(const T* g, int64_t pitch, int64_t B, int cols, T* out, float* partial) {
     int launches = 0;
     const int rc = column_sums_launch(reinterpret_cast<const float*>(g), pitch * (int)(sizeof(T) / 4), B, cols * (int)(sizeof(T) / 4),
-                                      reinterpret_cast<float*>(out), partial, stream, &launches);
+                                      reinterpret_cast<float*>(out), partial, guard, stream, &launches);
     if (rc == BFLY_OK) g_launches.fetch_add(launches);
     return rc;
   }
   // out[b, c] = sum over s of g[b, s, c], c < cols; g is (B, S, n)
   template <typename T> int stack_sums(const T* g, int64_t B, int S, int64_t n, int cols, T* out) {
     constexpr int F = (int)(sizeof(T) / 4);
-    const int rc = stack_sums_launch(reinterpret_cast<const float*>(g), B, S, n * F, cols * F, reinterpret_cast<float*>(out), dev.sms, stream);
+    const int rc = stack_sums_launch(reinterpret_cast<const float*>(g), B, S, n * F, cols * F, reinterpret_cast<float*>(out), guard, dev.sms, stream);
     if (rc == BFLY_OK) g_launches.fetch_add(1);
     return rc;
   }
@@ -786,10 +796,16 @@ struct CudaExec {
   }
   int zero(void* ptr, size_t bytes) {
     if (bytes == 0) return BFLY_OK;
+    if (guard) return zero2d(ptr, bytes, bytes, 1);
     return cudaMemsetAsync(ptr, 0, bytes, stream) == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
   }
   int zero2d(void* ptr, size_t pitch, size_t width, size_t rows) {
     if (width == 0 || rows == 0) return BFLY_OK;
+    if (guard) {
+      const int rc = guarded_zero_launch(ptr, pitch, width, rows, guard, dev.sms, stream);
+      if (rc == BFLY_OK) g_launches.fetch_add(1);
+      return rc;
+    }
     return cudaMemset2DAsync(ptr, pitch, 0, width, rows, stream) == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
   }
 };
@@ -1168,9 +1184,8 @@ int64_t bfly_bw_saved_workspace_bytes(int dtype, int batch, int nstacks, int log
   Problem q{batch, nstacks, log_n, nblocks, 1, 1, true, false};
   const int rc = check_problem(q);
   if (rc) return rc;
-  auto bytes = [](const MmaLayout& L) { return L.bw_bytes(true) + kMmaSpare; };
-  if (dtype == BFLY_F32) return mma_either<float>(q, bytes);
-  if (dtype == BFLY_C64) return mma_either<cf>(q, bytes);
+  if (dtype == BFLY_F32) return mma_either<float>(q, [](const Problem& d, const MmaLayout& L) { return mma_bw_need<float>(d, L, true) + kMmaSpare; });
+  if (dtype == BFLY_C64) return mma_either<cf>(q, [](const Problem& d, const MmaLayout& L) { return mma_bw_need<cf>(d, L, true) + kMmaSpare; });
   return BFLY_E_UNSUPPORTED;
 }
 int bfly_bw_f32_noalloc(const float* twiddle, const float* x, int64_t x_sB, int64_t x_sS, const float* grad,

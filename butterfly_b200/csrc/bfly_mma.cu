@@ -57,17 +57,17 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float* v) {
 // ------------------------------------------------------------------ values and slices
 
 // Eight neighbouring float32 values as their three bfloat16 slices, 16 bytes each.  The first slice cuts (rounding would
-// turn the largest finite values into infinities), the second rounds, the third is what is left: exact.  CARE: returns
-// false when one of the values is not finite; these become zeros and the caller sees to them.  Otherwise they become
-// slices that make every sum they enter NaN.
-template <bool CARE> __device__ __forceinline__ bool split8(const float* v, uint4& s1, uint4& s2, uint4& s3) {
+// turn the largest finite values into infinities), the second rounds, the third is what is left: exact.  `probe`: the largest
+// magnitudes so far (a bfloat16 pair of any signs).
+__device__ __forceinline__ void split8(const float* v, uint4& s1, uint4& s2, uint4& s3, uint32_t& probe) {
   uint32_t a1[4], a2[4], a3[4];
-  uint64_t probe = 0, minus, zero = 0;
+  uint64_t minus;
   asm("mov.b64 %0, {%1, %1};" : "=l"(minus) : "f"(-1.f));
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const uint32_t u = __float_as_uint(v[2 * i]), w = __float_as_uint(v[2 * i + 1]);
     a1[i] = __byte_perm(u, w, 0x7632);
+    asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(probe) : "r"(probe), "r"(a1[i]));
     uint64_t x, h, r;
     uint32_t ru, rw;
     asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(u), "r"(w));
@@ -77,38 +77,20 @@ template <bool CARE> __device__ __forceinline__ bool split8(const float* v, uint
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(a2[i]) : "f"(__uint_as_float(rw)), "f"(__uint_as_float(ru)));
     asm("mov.b64 %0, {%1, %2};" : "=l"(h) : "r"(a2[i] << 16), "r"(a2[i] & 0xffff0000u));
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(h), "l"(minus), "l"(r));
-    if (CARE) asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(probe) : "l"(r), "l"(zero), "l"(probe));  // infinity - infinity and what follows a NaN stay NaN
     asm("mov.b64 {%0, %1}, %2;" : "=r"(ru), "=r"(rw) : "l"(r));
     a3[i] = __byte_perm(ru, rw, 0x7632);
-  }
-  float pu, pw;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(pu), "=f"(pw) : "l"(probe));
-  const bool fine = !CARE || pu + pw == 0.f;
-  if (CARE && !fine) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint32_t keep = 0;
-      if (isfinite(v[2 * i])) keep |= 0xffffu;
-      if (isfinite(v[2 * i + 1])) keep |= 0xffff0000u;
-      a1[i] &= keep; a2[i] &= keep; a3[i] &= keep;
-    }
   }
   s1 = make_uint4(a1[0], a1[1], a1[2], a1[3]);
   s2 = make_uint4(a2[0], a2[1], a2[2], a2[3]);
   s3 = make_uint4(a3[0], a3[1], a3[2], a3[3]);
-  return fine;
+}
+__device__ __forceinline__ bool beyond(uint32_t probe) {
+  constexpr uint32_t most = (127 + kMmaRowBits) << 7;
+  return (probe & 0x7fff) >= most || ((probe >> 16) & 0x7fff) >= most;
 }
 
 // Where a CTA is: stack, first column of its block, row tile.
 struct Spot { int stack, cbase, tile; };
-
-// One element of a tile, wherever it lies.
-template <bool PLANE> __device__ float tile_elem(const float* plane, const MmaRowsIO& io, const MmaPass& p, const Spot& at, int row, int j) {
-  if (PLANE) return plane[((((int64_t)at.stack * p.nt + at.tile) << p.geo.log_nf) + at.cbase + p.geo.col(j)) * kMmaRows + row];
-  const int64_t r = (int64_t)at.tile * kMmaRows + row;
-  const int c = at.cbase + p.geo.col(j);
-  return r < p.B && c < mma_cols(io, at.stack, p.geo.log_nf) ? io.p[r * io.sB + at.stack * io.sS + c] : 0.f;
-}
 
 __device__ __forceinline__ void load8(const float* src, float* v) {  // 32-byte aligned
   asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -173,9 +155,9 @@ __device__ __forceinline__ void load_tile(const float* __restrict__ plane, const
 // Operand of a tile in shared memory, 48 KB: from a plane [row half][slice][column][64 rows], from rows [slice][row][64
 // columns]; 128-byte lines whose 16-byte chunks are swizzled.
 constexpr uint32_t kOpBytes = 3 * kMmaRows * kMmaCols * 2;
-template <bool PLANE, bool CARE> __device__ __forceinline__ bool store_unit(uint8_t* op, int u, const float* v) {
+template <bool PLANE> __device__ __forceinline__ void store_unit(uint8_t* op, int u, const float* v, uint32_t& probe) {
   uint4 s1, s2, s3;
-  const bool fine = split8<CARE>(v, s1, s2, s3);
+  split8(v, s1, s2, s3, probe);
   uint8_t* d;
   constexpr int slice = PLANE ? 8192 : 16384;
   if (PLANE) {
@@ -188,16 +170,6 @@ template <bool PLANE, bool CARE> __device__ __forceinline__ bool store_unit(uint
   *reinterpret_cast<uint4*>(d) = s1;
   *reinterpret_cast<uint4*>(d + slice) = s2;
   *reinterpret_cast<uint4*>(d + 2 * slice) = s3;
-  return fine;
-}
-
-// Entry (j, i) of an operator image.
-__device__ __forceinline__ float image_elem(const uint8_t* img, int j, int i) {
-  const uint8_t* q = img + j * 128 + (((i >> 3) ^ (j & 7)) << 4) + (i & 7) * 2;
-  float v = 0.f;
-#pragma unroll
-  for (int s = kMmaParts - 1; s >= 0; --s) v += __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t*>(q + s * 8192) << 16);
-  return v;
 }
 
 // rows x operator (TRANS: transposed operator).  Accumulators of 64 columns: slice 1 of the rows and part 1 of the operator,
@@ -349,9 +321,8 @@ struct Control {
   uint64_t xfull;                // backward, second operand: written (read: pfull)
   uint64_t dfull[2], dempty[2];  // transformed tile in tensor memory: complete, taken out
   uint64_t pfull, pempty;        // operator gradient: complete for a tile, taken out
-  uint64_t sync[2];              // all warps that cut, that store
+  uint64_t sync;                 // all warps that cut
   uint32_t tmem;
-  int special[8];                // the tile (number & 7) holds values that are not finite: the roles are up to six tiles apart
   int failed;                    // a wait ran out
 };
 template <typename M> constexpr uint32_t pass_bytes() { return M::control + (uint32_t)sizeof(Control); }
@@ -405,27 +376,6 @@ struct Walk {
   }
 };
 
-// What values of the first operand that are not finite add to 32 results of a row (fix[0..32)) and, in the backward, to 32 entries of
-// the operator gradient (fix[32..64)): they enter the products as zeros.
-template <bool BW, bool IN_P, bool X_P>
-__device__ __noinline__ void special_terms(const MmaPass& p, const Spot& at, const uint8_t* img, int row, int j0, float* fix) {
-  for (int c = 0; c < (BW ? 64 : 32); ++c) fix[c] = 0.f;
-  for (int j = 0; j < kMmaCols; ++j) {
-    const float v = tile_elem<IN_P>(p.in_t, p.in, p, at, row, j);
-    if (isfinite(v)) continue;
-    for (int c = 0; c < 32; ++c) {
-      const float m = BW ? image_elem(img, j, j0 + c) : image_elem(img, j0 + c, j);
-      if (m != 0.f) fix[c] = fmaf(m, v, fix[c]);
-    }
-  }
-  if (BW && row < kMmaCols)
-    for (int r = 0; r < kMmaRows; ++r) {
-      const float g = tile_elem<IN_P>(p.in_t, p.in, p, at, r, row);
-      if (isfinite(g)) continue;
-      for (int c = 0; c < 32; ++c) fix[32 + c] = fmaf(g, tile_elem<X_P>(p.x_t, p.x, p, at, r, j0 + c), fix[32 + c]);
-    }
-}
-
 template <int REGS> __device__ __forceinline__ void registers_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS)); }
 template <int REGS> __device__ __forceinline__ void registers_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
 
@@ -454,10 +404,9 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
     mbar_init(smem_u32(&ctl->xfull), kCutWarps);
     mbar_init(smem_u32(&ctl->pfull), 1);
     mbar_init(smem_u32(&ctl->pempty), kStoreWarps);
-    mbar_init(smem_u32(&ctl->sync[0]), kCutWarps);
-    mbar_init(smem_u32(&ctl->sync[1]), kStoreWarps);
-    for (int i = 0; i < 8; ++i) ctl->special[i] = 0;
+    mbar_init(smem_u32(&ctl->sync), kCutWarps);
     ctl->failed = 0;
+    if (BW && blockIdx.x == 0 && p.kept_flag && *p.kept_flag) *p.flag = 1;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kIssueWarp) {
@@ -476,7 +425,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
     float bsum[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) bsum[i] = 0.f;
-    uint32_t turn = 0, i = 0;
+    uint32_t turn = 0, i = 0, probe = 0;
     int held = -1;       // block whose operator shared memory holds
     // Tile i, whose values are there: its place, and its operator if that is another than the last tile's.
     auto place = [&](int block) -> bool {
@@ -492,11 +441,9 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
       }
       return true;
     };
-    auto cut = [&](auto plane, auto care, uint8_t* op, float (*v)[8], uint64_t* full) {
-      bool fine = true;
+    auto cut = [&](auto plane, uint8_t* op, float (*v)[8], uint64_t* full) {
 #pragma unroll
-      for (int u = 0; u < kUnits; ++u) fine &= store_unit<decltype(plane)::value, decltype(care)::value>(op, tid + u * kCutThreads, v[u]);
-      if (!fine) ctl->special[i & 7] = 1;
+      for (int u = 0; u < kUnits; ++u) store_unit<decltype(plane)::value>(op, tid + u * kCutThreads, v[u], probe);
       fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(full);
@@ -509,7 +456,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
       if (ahead.more()) load_tile<IN_P>(p.in_t, p.in, p, ahead.at, tid, vb);
       auto step = [&](float (*v)[8]) -> bool {
         if (!place(at.block)) return false;
-        cut(std::integral_constant<bool, IN_P>(), std::true_type(), sm + (i % ST) * kOpBytes, v, &ctl->gfull[i % ST]);
+        cut(std::integral_constant<bool, IN_P>(), sm + (i % ST) * kOpBytes, v, &ctl->gfull[i % ST]);
         at.next(p);
         ahead.next(p);
         if (ahead.more()) load_tile<IN_P>(p.in_t, p.in, p, ahead.at, tid, v);
@@ -526,7 +473,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
         const bool last = at.last_of_block();
         at.next(p);
         uint8_t* op = sm + (i % ST) * kOpBytes;
-        cut(std::integral_constant<bool, IN_P>(), std::true_type(), op, va, &ctl->gfull[i % ST]);
+        cut(std::integral_constant<bool, IN_P>(), op, va, &ctl->gfull[i % ST]);
         if (!IN_P) {
 #pragma unroll
           for (int u = 0; u < kUnits; ++u)
@@ -535,7 +482,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
         }
         if (at.more()) load_tile<IN_P>(p.in_t, p.in, p, at.at, tid, va);
         if (i >= 1 && !await_warp(ctl, &ctl->pfull, (i - 1) & 1)) break;
-        cut(std::integral_constant<bool, X_P>(), std::false_type(), sm + Mem::x, vb, &ctl->xfull);
+        cut(std::integral_constant<bool, X_P>(), sm + Mem::x, vb, &ctl->xfull);
         if (at.more()) load_tile<X_P>(p.x_t, p.x, p, at.at, tid, vb);
         if (!IN_P && last) {
           if (p.bias_slots) {  // column sums of the block's rows: this thread has columns 8 (tid % 8) ..
@@ -546,19 +493,20 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
               bsum[e] += __shfl_xor_sync(0xffffffffu, bsum[e], 16);
               if (lane < 8) sums[warp * 64 + lane * 8 + e] = bsum[e];
             }
-            if (!role_sync(ctl, &ctl->sync[0], turn)) break;
+            if (!role_sync(ctl, &ctl->sync, turn)) break;
             if (tid < 64) {
               float v = 0.f;
               for (int k = 0; k < kCutWarps; ++k) v += sums[k * 64 + tid];
               p.bias_slots[mma_slot(p.geo, block, blockIdx.x >> p.geo.sib) * 64 + tid] = v;
             }
-            if (!role_sync(ctl, &ctl->sync[0], turn)) break;
+            if (!role_sync(ctl, &ctl->sync, turn)) break;
           }
 #pragma unroll
           for (int e = 0; e < 8; ++e) bsum[e] = 0.f;
         }
       }
     }
+    if (beyond(probe)) *p.flag = 1;
   } else if (warp >= kIssueWarp) {
     registers_down<kIssueRegs>();
     // ---------------- issue the products
@@ -590,24 +538,12 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
     float acc[BW ? 32 : 1];  // operator gradient: row `row` (two slices of the incoming gradient), columns j0 ..
 #pragma unroll
     for (int i = 0; i < (BW ? 32 : 1); ++i) acc[i] = 0.f;
-    float fix[BW ? 64 : 32];  // only for tiles with values that are not finite
-    uint32_t turn = 0;
     int kept = 0;
     for (uint32_t i = 0; at.more(); ++i) {
       const uint32_t d = i % DBUF;
       if (!await_warp(ctl, &ctl->dfull[d], (i / DBUF) & 1)) break;
       fence_after_sync();
       const Spot now = at.at;
-      const bool special = *reinterpret_cast<volatile int*>(&ctl->special[i & 7]);
-      if (special) {
-        special_terms<BW, IN_P, X_P>(p, now, img, row, j0, fix);
-        if (!role_sync(ctl, &ctl->sync[1], turn)) break;  // passes from plane to plane work in place
-        if (e == 0) ctl->special[i & 7] = 0;
-        if (BW) {
-#pragma unroll
-          for (int c = 0; c < (BW ? 32 : 0); ++c) acc[c] += fix[32 + c];
-        }
-      }
       constexpr int NY = Mem::turn_cols;  // columns of a row at a time (the backward has no registers for all 32)
 #pragma unroll
       for (int c0 = 0; c0 < 32; c0 += NY) {
@@ -618,10 +554,6 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
           fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&ctl->dempty[d]);
-        }
-        if (special) {
-#pragma unroll
-          for (int c = 0; c < NY; ++c) y[c] += fix[c0 + c];
         }
         if (OUT_P) store_plane<NY>(p.out_t, p, now, row, j0 + c0, y);
         else store_rows<NY>(p.out, p, now, row - lane, j0 + c0, y, sm + Mem::turn + e * 32 * NY * 4, BW && p.reduce != 0, BW ? nullptr : p.bias);
@@ -677,10 +609,9 @@ template <> struct Num<false> {
   static __device__ double one(bool o) { return o ? 1.0 : 0.0; }
   static __device__ double up(float a) { return a; }
   static __device__ float down(double a) { return (float)a; }
-  static __device__ double mul(double a, double b) { return a * b; }
   static __device__ double fma(double a, double b, double c) { return ::fma(a, b, c); }   // a b + c
   static __device__ double fmac(double a, double b, double c) { return ::fma(a, b, c); }  // conj(a) b + c
-  static __device__ bool none(double a) { return a == 0.0; }
+  static __device__ bool below(double a, double most) { return fabs(a) < most; }
   static __device__ double zero() { return 0.0; }
   static __device__ double add(double a, double b) { return a + b; }
   static __device__ double shuffle(double v, int h) { return __shfl_xor_sync(0xffffffffu, v, h); }
@@ -693,7 +624,7 @@ template <> struct Num<true> {
   static __device__ float2 down(cd a) { return make_float2((float)a.re, (float)a.im); }
   static __device__ cd fma(cd a, cd b, cd c) { return cd{::fma(a.re, b.re, ::fma(-a.im, b.im, c.re)), ::fma(a.re, b.im, ::fma(a.im, b.re, c.im))}; }
   static __device__ cd fmac(cd a, cd b, cd c) { return cd{::fma(a.re, b.re, ::fma(a.im, b.im, c.re)), ::fma(a.re, b.im, ::fma(-a.im, b.re, c.im))}; }
-  static __device__ bool none(cd a) { return a.re == 0.0 && a.im == 0.0; }
+  static __device__ bool below(cd a, double most) { return fabs(a.re) < most && fabs(a.im) < most; }
   static __device__ cd zero() { return cd{0.0, 0.0}; }
   static __device__ cd add(cd a, cd b) { return cd{a.re + b.re, a.im + b.im}; }
   static __device__ cd shuffle(cd v, int h) { return cd{__shfl_xor_sync(0xffffffffu, v.re, h), __shfl_xor_sync(0xffffffffu, v.im, h)}; }
@@ -730,12 +661,13 @@ __device__ void gather_twiddles(typename Num<CPLX>::T* dst, const MmaGroup& g, i
   }
 }
 
-// work (W x W) <- factor x work, and a float32 copy of it (keep may be null)
+// work (W x W) <- factor x work, and a float32 copy of it (keep may be null); are the results below 2^kMmaOpBits?
 template <bool CPLX, int RAD>
-__device__ __forceinline__ void apply_stage(typename Num<CPLX>::T* work, int lbit, const typename Num<CPLX>::T* tw, typename Num<CPLX>::S* keep) {
+__device__ __forceinline__ bool apply_stage(typename Num<CPLX>::T* work, int lbit, const typename Num<CPLX>::T* tw, typename Num<CPLX>::S* keep) {
   typedef Num<CPLX> N;
   constexpr int W = N::W;
   const int lane = threadIdx.x & 31, d = W << lbit;
+  bool fine = true;
   for (int u = threadIdx.x >> 5; u < W / RAD; u += blockDim.x >> 5) {
     typename N::T t[RAD * RAD];
 #pragma unroll
@@ -752,15 +684,16 @@ __device__ __forceinline__ void apply_stage(typename Num<CPLX>::T* work, int lbi
 #pragma unroll
         for (int i = 0; i < RAD; ++i) a = N::fma(t[o * RAD + i], x[i], a);
         work[c + o * d] = a;
+        fine &= N::below(a, (double)(1 << kMmaOpBits));
         if (keep) keep[c + o * d] = N::down(a);
       }
     }
   }
+  return fine;
 }
 template <bool CPLX, bool FOUR>
-__device__ __forceinline__ void apply_stage(typename Num<CPLX>::T* work, const MmaStage& m, const typename Num<CPLX>::T* tw, typename Num<CPLX>::S* keep) {
-  if (FOUR && m.radix == 4) apply_stage<CPLX, 4>(work, m.lbit, tw, keep);
-  else apply_stage<CPLX, 2>(work, m.lbit, tw, keep);
+__device__ __forceinline__ bool apply_stage(typename Num<CPLX>::T* work, const MmaStage& m, const typename Num<CPLX>::T* tw, typename Num<CPLX>::S* keep) {
+  return FOUR && m.radix == 4 ? apply_stage<CPLX, 4>(work, m.lbit, tw, keep) : apply_stage<CPLX, 2>(work, m.lbit, tw, keep);
 }
 
 // Latency: at most twelve short stages with a barrier each; blocks of all groups run side by side.
@@ -775,12 +708,14 @@ __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_prep_kernel(c
   gather_twiddles<CPLX>(tw, g, cbase, s, p.tw, p.tw_stack);
   for (int i = threadIdx.x; i < W * W; i += T) work[i] = N::one(i / W == i % W);
   __syncthreads();
+  bool fine = true;
   for (int k = 0, off = 0; k < g.nst; ++k) {
     const MmaStage m = g.st[k];
-    apply_stage<CPLX, FOUR>(work, m, tw + off, (typename N::S*)nullptr);
+    fine &= apply_stage<CPLX, FOUR>(work, m, tw + off, (typename N::S*)nullptr);
     off += W * m.radix;
     __syncthreads();
   }
+  if (!fine) *p.flag = 1;
   // Parts of an entry v: v to a multiple of 2^(E - 3), where 2^E is at most the largest entry of its row or its column, the
   // larger of the two (exact sums, see above), and three bfloat16 slices of the rest.
   __shared__ int top[2][kMmaCols];  // exponents of the largest entries of a row, a column
@@ -869,7 +804,7 @@ __device__ __forceinline__ void unstack_stage(typename Num<CPLX>::T* G, const ty
       for (int o = 0; o < RAD; ++o)
 #pragma unroll
         for (int i = 0; i < RAD; ++i)
-          if (!N::none(r[i])) a[o * RAD + i] = N::fmac(r[i], g[o], a[o * RAD + i]);  // (a NaN elsewhere in the block stays there)
+          a[o * RAD + i] = N::fmac(r[i], g[o], a[o * RAD + i]);
       if (R) {
 #pragma unroll
         for (int i = 0; i < RAD; ++i) {
@@ -919,6 +854,10 @@ __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_post_kernel(c
         sum[i] += (double)v.x; sum[i + 1] += (double)v.y; sum[i + 2] += (double)v.z; sum[i + 3] += (double)v.w;
       }
   }
+  bool fine = true;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) fine &= isfinite(sum[i]);
+  if (!fine) *p.flag = 1;
   gather_twiddles<CPLX>(tw, g, cbase, s, p.tw, p.tw_stack);
   for (int i = tid; i < W * W; i += THREADS) G[i] = N::one(i / W == i % W);
   __syncthreads();

@@ -12,6 +12,12 @@
 // 2^-25 of the whole) and summed in float32 by size.  tcgen05 cuts its sums towards zero, so those that count are kept
 // exact or short (bfly_mma.cu).
 //
+// Range.  Operators and slices stand for the stages only while values are ordinary: no infinities or NaN, which spread stage
+// by stage, nothing that overflows halfway.  Rows, gradients and activations from 2^40 on, operators (or products of some of
+// their stages) from 2^20 on and sums that overflow raise a flag, whatever else they are; behind the passes the phase
+// kernels are launched too and run if the flag is up (bfly_driver.h).  Their results, from the caller's tensors, then
+// replace everything.
+//
 // Columns are counted in floats here: complex rows are rows of 2n floats whose bit 0 tells real from imaginary parts,
 // always inside the window, and a complex operator of 32 x 32 is a real one of 64 x 64.
 //
@@ -36,6 +42,8 @@ constexpr int kMmaMaxStages = 12;             // radix-2 stages a group may hold
 constexpr int kMmaMaxGroups = 8;
 constexpr int kMmaParts = 4;                  // bfloat16 parts of an operator
 constexpr int kMmaImageBytes = kMmaParts * kMmaCols * kMmaCols * 2;  // one operator, swizzled as tcgen05 reads it
+constexpr int kMmaRowBits = 40, kMmaOpBits = 20;             // rows below 2^40, operators below 2^20
+constexpr size_t kMmaHead = 256;              // in front of what a forward leaves and of a backward's work space: the flag
 constexpr int kMmaBwMaxCtas = 160;            // most CTAs of a backward pass (one per SM)
 constexpr int kMmaSlotFloats = 2 * kMmaCols * kMmaCols;      // an operator gradient as a CTA leaves it: two halves to be added
 struct MmaStage {
@@ -88,6 +96,8 @@ struct MmaPass {
   int bias_len;
   float* slots;           // backward: operator gradients, slot = block of (stack, q) + CTA
   float* bias_slots;      // backward: column sums of the incoming gradient, 64 per slot; may be null
+  int* flag;              // set to 1 for values that are not ordinary
+  const int* kept_flag;   // backward: the forward's, taken over; may be null
 };
 
 struct MmaPrep {
@@ -95,6 +105,7 @@ struct MmaPrep {
   int64_t tw_stack[2];
   int S, nq, ng;
   uint8_t* images;        // (group, stack, block)
+  int* flag;
   MmaGroup g[kMmaMaxGroups];
 };
 struct MmaPost {
@@ -106,6 +117,7 @@ struct MmaPost {
   const float* slots;     // (group, slot)
   int64_t slots_group;    // floats from a group to the next
   const float* bias_slots;
+  int* flag;
   float* dbias;           // with bias_slots: column sums of the last group's incoming gradient
   int dbias_len;
   MmaGroup g[kMmaMaxGroups];
@@ -179,11 +191,11 @@ struct MmaLayout {
   size_t plane;                 // bytes of a plane
   size_t images;                // operators of all groups
   size_t slots, bias_slots;     // backward: operator gradients of all groups, bias sums
-  // what a forward leaves: the activations between the groups, the operators
-  size_t kept() const { return (g.size() - 1) * plane + images; }
+  // what a forward leaves: the flag, the activations between the groups, the operators
+  size_t kept() const { return kMmaHead + (g.size() - 1) * plane + images; }
   // work space of a backward that starts from that (a gradient plane), and of one that makes it itself (the gradient takes
   // the place of the last activations)
-  size_t bw_bytes(bool from_kept) const { return slots + bias_slots + (from_kept ? (g.size() > 1 ? plane : 0) : kept()); }
+  size_t bw_bytes(bool from_kept) const { return slots + bias_slots + (from_kept ? kMmaHead + (g.size() > 1 ? plane : 0) : kept()); }
 };
 
 }  // namespace bfly

@@ -583,6 +583,7 @@ int bfly_emul_bw_plan(int dtype, int base4, int B, int S, int log_n, int nblocks
 namespace {
 struct DryExec {
   static constexpr bool kMma = true, kFusedBias = true;
+  const int* guard = nullptr;
   struct Range { uintptr_t at; size_t bytes; };
   std::vector<Range> ranges;
   int outside = 0, passes = 0;  // tensors that left their buffer; tensor-core passes
@@ -687,7 +688,7 @@ template <typename T> int dry_step(Problem q, int how, size_t skew, int* passes)
   const int64_t x_sB = (int64_t)q.S * q.in_size, g_sB = (int64_t)q.S * q.out_size;
   int rc = BFLY_OK;
   if (how == 0) {
-    const int64_t kept = bw_snapshot_need<T>(q), own = mma_either<T>(q, [](const MmaLayout& L) { return L.bw_bytes(true) + kMmaSpare; });
+    const int64_t kept = bw_snapshot_need<T>(q), own = mma_either<T>(q, [](const Problem& d, const MmaLayout& L) { return mma_bw_need<T>(d, L, true) + kMmaSpare; });
     if (kept < 0) return (int)kept;
     char* k = ex.buffer<char>(kept, skew), *w = ex.buffer<char>(own, skew);
     rc = drive_fw_saving<T>(ex, q, tw2, tw4, x, x_sB, q.in_size, out, k, kept);
