@@ -56,21 +56,23 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float* v) {
 
 // ------------------------------------------------------------------ values and slices
 
-// Eight neighbouring float32 values as their three bfloat16 slices, 16 bytes each.  The first slice cuts (rounding would
+// Eight neighbouring float32 values, times 2^kMmaScale, as their three bfloat16 slices, 16 bytes each.  The first slice cuts (rounding would
 // turn the largest finite values into infinities), the second rounds, the third is what is left: exact.  `probe`: the largest
 // magnitudes so far (a bfloat16 pair of any signs).
 __device__ __forceinline__ void split8(const float* v, uint4& s1, uint4& s2, uint4& s3, uint32_t& probe) {
   uint32_t a1[4], a2[4], a3[4];
-  uint64_t minus;
+  uint64_t minus, scale;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(scale) : "f"((float)(1 << kMmaScale)));
   asm("mov.b64 %0, {%1, %1};" : "=l"(minus) : "f"(-1.f));
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint32_t u = __float_as_uint(v[2 * i]), w = __float_as_uint(v[2 * i + 1]);
+    uint64_t x, h, r;
+    uint32_t u, w, ru, rw;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(v[2 * i]), "f"(v[2 * i + 1]));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(x) : "l"(x), "l"(scale));
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(u), "=r"(w) : "l"(x));
     a1[i] = __byte_perm(u, w, 0x7632);
     asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(probe) : "r"(probe), "r"(a1[i]));
-    uint64_t x, h, r;
-    uint32_t ru, rw;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(u), "r"(w));
     asm("mov.b64 %0, {%1, %2};" : "=l"(h) : "r"(u & 0xffff0000u), "r"(w & 0xffff0000u));
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(h), "l"(minus), "l"(x));
     asm("mov.b64 {%0, %1}, %2;" : "=r"(ru), "=r"(rw) : "l"(r));
@@ -85,7 +87,7 @@ __device__ __forceinline__ void split8(const float* v, uint4& s1, uint4& s2, uin
   s3 = make_uint4(a3[0], a3[1], a3[2], a3[3]);
 }
 __device__ __forceinline__ bool beyond(uint32_t probe) {
-  constexpr uint32_t most = (127 + kMmaRowBits) << 7;
+  constexpr uint32_t most = (127 + kMmaScale + kMmaRowBits) << 7;
   return (probe & 0x7fff) >= most || ((probe >> 16) & 0x7fff) >= most;
 }
 
@@ -216,7 +218,7 @@ __device__ __forceinline__ void load_transform(uint32_t d, float* y) {
   tmem_ld8(d + 192, c);
   wait_ld();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) y[i] += a[i] + (b[i] + c[i]);
+  for (int i = 0; i < 8; ++i) y[i] = (y[i] + (a[i] + (b[i] + c[i]))) * (1.f / ((int64_t)1 << 2 * kMmaScale));
 }
 
 // N results of a thread's row (window columns j0 ..) into a plane: a warp writes 128 bytes of a column at a time.
@@ -602,6 +604,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
 // ------------------------------------------------------------------ operators and their gradients
 
 struct cd { double re, im; };
+constexpr double kKept = (double)(1ll << 40);  // products of some factors, below 2^20, keep 24 bits down to 2^-166
 template <bool CPLX> struct Num;
 template <> struct Num<false> {
   typedef double T; typedef float S;
@@ -609,6 +612,7 @@ template <> struct Num<false> {
   static __device__ double one(bool o) { return o ? 1.0 : 0.0; }
   static __device__ double up(float a) { return a; }
   static __device__ float down(double a) { return (float)a; }
+  static __device__ double times(double a, double s) { return a * s; }
   static __device__ double fma(double a, double b, double c) { return ::fma(a, b, c); }   // a b + c
   static __device__ double fmac(double a, double b, double c) { return ::fma(a, b, c); }  // conj(a) b + c
   static __device__ bool below(double a, double most) { return fabs(a) < most; }
@@ -622,6 +626,7 @@ template <> struct Num<true> {
   static __device__ cd one(bool o) { return cd{o ? 1.0 : 0.0, 0.0}; }
   static __device__ cd up(float2 a) { return cd{a.x, a.y}; }
   static __device__ float2 down(cd a) { return make_float2((float)a.re, (float)a.im); }
+  static __device__ cd times(cd a, double s) { return cd{a.re * s, a.im * s}; }
   static __device__ cd fma(cd a, cd b, cd c) { return cd{::fma(a.re, b.re, ::fma(-a.im, b.im, c.re)), ::fma(a.re, b.im, ::fma(a.im, b.re, c.im))}; }
   static __device__ cd fmac(cd a, cd b, cd c) { return cd{::fma(a.re, b.re, ::fma(a.im, b.im, c.re)), ::fma(a.re, b.im, ::fma(-a.im, b.re, c.im))}; }
   static __device__ bool below(cd a, double most) { return fabs(a.re) < most && fabs(a.im) < most; }
@@ -661,7 +666,7 @@ __device__ void gather_twiddles(typename Num<CPLX>::T* dst, const MmaGroup& g, i
   }
 }
 
-// work (W x W) <- factor x work, and a float32 copy of it (keep may be null); are the results below 2^kMmaOpBits?
+// work (W x W) <- factor x work, and a float32 copy of it times kKept (keep may be null); are the results below 2^kMmaOpBits?
 template <bool CPLX, int RAD>
 __device__ __forceinline__ bool apply_stage(typename Num<CPLX>::T* work, int lbit, const typename Num<CPLX>::T* tw, typename Num<CPLX>::S* keep) {
   typedef Num<CPLX> N;
@@ -685,7 +690,7 @@ __device__ __forceinline__ bool apply_stage(typename Num<CPLX>::T* work, int lbi
         for (int i = 0; i < RAD; ++i) a = N::fma(t[o * RAD + i], x[i], a);
         work[c + o * d] = a;
         fine &= N::below(a, (double)(1 << kMmaOpBits));
-        if (keep) keep[c + o * d] = N::down(a);
+        if (keep) keep[c + o * d] = N::down(N::times(a, kKept));
       }
     }
   }
@@ -716,15 +721,15 @@ __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_prep_kernel(c
     __syncthreads();
   }
   if (!fine) *p.flag = 1;
-  // Parts of an entry v: v to a multiple of 2^(E - 3), where 2^E is at most the largest entry of its row or its column, the
+  // Parts of an entry v (scaled): v to a multiple of 2^(E - 3), where 2^E is at most the largest entry of its row or its column, the
   // larger of the two (exact sums, see above), and three bfloat16 slices of the rest.
   __shared__ int top[2][kMmaCols];  // exponents of the largest entries of a row, a column
   auto entry = [&](int j, int i) -> double {
     if constexpr (CPLX) {
       const cd z = work[(j >> 1) * W + (i >> 1)];
-      return (j & 1) == (i & 1) ? z.re : ((j & 1) ? z.im : -z.im);
+      return ((j & 1) == (i & 1) ? z.re : ((j & 1) ? z.im : -z.im)) * (1 << kMmaScale);
     } else {
-      return work[j * W + i];
+      return work[j * W + i] * (1 << kMmaScale);
     }
   };
   if (threadIdx.x < 2 * kMmaCols) top[threadIdx.x / kMmaCols][threadIdx.x % kMmaCols] = -1100;
@@ -798,7 +803,7 @@ __device__ __forceinline__ void unstack_stage(typename Num<CPLX>::T* G, const ty
 #pragma unroll
       for (int i = 0; i < RAD; ++i) {
         g[i] = G[at + c + i * d];
-        r[i] = R ? N::up(R[at + c + i * d]) : N::one(r0 + (i << m.lbit) == c + lane);
+        r[i] = R ? N::times(N::up(R[at + c + i * d]), 1.0 / kKept) : N::one(r0 + (i << m.lbit) == c + lane);
       }
 #pragma unroll
       for (int o = 0; o < RAD; ++o)
@@ -822,7 +827,7 @@ __device__ __forceinline__ void unstack_stage(typename Num<CPLX>::T* G, const ty
 
 // Gradients of a group's factors from the gradient of their product, for one block: with R the product of the factors
 // before a factor and G the gradient of the product up to it, its own gradient is (G R^H) where it has entries, and G
-// continues as (factor)^H G.  R before every factor is kept (float32); G runs in float64.
+// continues as (factor)^H G.  R before every factor is kept (float32, times kKept); G runs in float64.
 template <bool CPLX, bool FOUR>
 __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_post_kernel(const __grid_constant__ MmaPost p) {
   typedef Num<CPLX> N;
@@ -856,7 +861,10 @@ __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_post_kernel(c
   }
   bool fine = true;
 #pragma unroll
-  for (int i = 0; i < PER; ++i) fine &= isfinite(sum[i]);
+  for (int i = 0; i < PER; ++i) {
+    fine &= isfinite(sum[i]);
+    sum[i] *= 1.0 / ((int64_t)1 << 2 * kMmaScale);
+  }
   if (!fine) *p.flag = 1;
   gather_twiddles<CPLX>(tw, g, cbase, s, p.tw, p.tw_stack);
   for (int i = tid; i < W * W; i += THREADS) G[i] = N::one(i / W == i % W);

@@ -7,7 +7,7 @@
 // a small kernel takes apart into the gradients of the stages afterwards.  Per pass a tile crosses shared memory once,
 // whatever the number of stages, and the operators' arithmetic costs a quarter of the tile's trip through HBM.
 //
-// Precision.  A float32 value is the exact sum of three bfloat16 slices (8 + 8 + 8 bits).  Operators are multiplied out in
+// Precision.  A float32 value, scaled (kMmaScale), is the exact sum of three bfloat16 slices (8 + 8 + 8 bits).  Operators are multiplied out in
 // float64 and cut into four parts, the first of few bits.  Nine of the twelve products are formed (the others are below
 // 2^-25 of the whole) and summed in float32 by size.  tcgen05 cuts its sums towards zero, so those that count are kept
 // exact or short (bfly_mma.cu).
@@ -43,6 +43,9 @@ constexpr int kMmaMaxGroups = 8;
 constexpr int kMmaParts = 4;                  // bfloat16 parts of an operator
 constexpr int kMmaImageBytes = kMmaParts * kMmaCols * kMmaCols * 2;  // one operator, swizzled as tcgen05 reads it
 constexpr int kMmaRowBits = 40, kMmaOpBits = 20;             // rows below 2^40, operators below 2^20
+// Rows and operators enter the products times 2^24 each: the last of a value's 24 bits, 2^-149 at the least, is then a normal
+// bfloat16 (which have the exponents of float32, and 8 bits).  From 2^40 and 2^20 up to there nothing overflows either.
+constexpr int kMmaScale = 24;
 constexpr size_t kMmaHead = 256;              // in front of what a forward leaves and of a backward's work space: the flag
 constexpr int kMmaBwMaxCtas = 160;            // most CTAs of a backward pass (one per SM)
 constexpr int kMmaSlotFloats = 2 * kMmaCols * kMmaCols;      // an operator gradient as a CTA leaves it: two halves to be added

@@ -159,6 +159,36 @@ def test_layers_of_values_that_are_not_ordinary(dev, kind, in_size, out_size, pl
     assert bb.abi.device_error() == 0
 
 
+@pytest.mark.parametrize("cplx,log_n", [(False, 6), (False, 10), (True, 9)])
+@pytest.mark.parametrize("what", ["rows", "gradients", "both", "factors", "subnormal rows"])
+def test_small_values_keep_24_bits(dev, oracle_mod, cplx, log_n, what):
+    """Down to the end of float32's range: slices and operators are scaled, so that their last parts stay normal numbers."""
+    import butterfly_b200 as bb
+    n, B = 1 << log_n, 300
+    dt, wide = (torch.complex64, torch.complex128) if cplx else (torch.float32, torch.float64)
+    torch.manual_seed(log_n)
+    tw = torch.randn(1, 2, log_n, n // 2, 2, 2, dtype=dt) / 2 ** 0.5
+    x, g = torch.randn(B, 1, n, dtype=dt), torch.randn(B, 1, n, dtype=dt)
+    if what == "factors":  # operators of 2^-108
+        tw = tw / 2 ** (108 // (2 * log_n))
+    elif what == "subnormal rows":
+        tw = torch.eye(2, dtype=dt).expand_as(tw).contiguous()
+        x, g = x * 2.0 ** -131, g * 2.0 ** -131
+    else:
+        x = x * (2.0 ** -115 if what == "rows" else 2.0 ** -55 if what == "both" else 1)
+        g = g * (2.0 ** -115 if what == "gradients" else 2.0 ** -55 if what == "both" else 1)
+    want_y = oracle_mod.multiply_fw(tw.to(wide), x.to(wide), True)
+    want_d, want_dx = oracle_mod.multiply_bw(tw.to(wide), x.to(wide), g.to(wide), True)
+    with abi_option("mma", 1):
+        t, xd = tw.to(dev).requires_grad_(True), x.to(dev).requires_grad_(True)
+        y = bb.butterfly_multiply(t, xd, True)
+        d, dx = torch.autograd.grad(y, [t, xd], g.to(dev))
+    if what == "subnormal rows":
+        assert torch.equal(y.detach().cpu(), x) and torch.equal(dx.cpu(), g)  # (products of two such values are below the range)
+    else:
+        assert rel2(y, want_y) < TOL and rel2(dx, want_dx) < TOL and rel2(d, want_d) < TOL_GRAD
+
+
 def test_the_largest_ordinary_values_stay_on_the_passes(dev, oracle_mod):
     """Rows below 2^40 and operators below 2^20, whatever the phases make of them."""
     import butterfly_b200 as bb
