@@ -24,7 +24,7 @@ SYMBOLS = (
     "bfly_layer_bw_workspace_bytes", "bfly_layer_bw", "bfly_bw_f32_noalloc",
     "bfly_linear_fw_f32", "bfly_linear_bw_f32", "bfly_linear_bw_workspace_bytes", "bfly_device_error", "bfly_set_option", "bfly_get_option", "bfly4_fw_c64", "bfly4_bw_c64", "bfly_fw_f32_saving", "bfly_fw_c64_saving", "bfly_bw_f32_saved", "bfly_bw_c64_saved",
     "bfly_unitary_twiddle_fw", "bfly_unitary_twiddle_bw", "bfly_fw_glue_f32", "bfly_fw_glue_c64",
-    "bfly_selftest_bounded_wait", "bfly_device_error_async",
+    "bfly_selftest_bounded_wait", "bfly_device_error_async", "bfly_fw_saving_bytes", "bfly_option_changes",
 )
 
 NOALLOC_SCRATCH_BYTES = 32 << 20

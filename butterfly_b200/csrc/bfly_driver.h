@@ -23,6 +23,7 @@
 //   int  mma_post(const MmaPost&, bool cplx);
 //   const int* guard;                                      // with kMma: launches run only if *guard is not 0 (null: all run)
 #pragma once
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 
@@ -85,11 +86,18 @@ inline Options& options() {
   }();
   return opt;
 }
+// How often an option was set: what a forward saves is laid out as the options of the moment say, and a backward reads it
+// only if none was set in between.
+inline std::atomic<int64_t>& option_changes() {
+  static std::atomic<int64_t> n{0};
+  return n;
+}
 inline int set_option(const char* name, int value) {
   int cnt = 0;
   const OptionName* names = option_names(&cnt);
   for (int i = 0; name && i < cnt; ++i)
     if (std::strcmp(names[i].name, name) == 0) {
+      option_changes().fetch_add(1);
       options().*(names[i].field) = value;
       return BFLY_OK;
     }
@@ -803,23 +811,11 @@ template <typename T> inline int64_t bw_workspace_need(const Problem& q0) {
   }
   return std::max(best, mma_either<T>(q0, [&](const Problem& q, const MmaLayout& L) { return mma_bw_need<T>(q, L, false) + kMmaSpare; }));
 }
-// What a saving forward has to leave for the backward, again for either direction: one of them may run as tensor-core passes
-// and the other as phases (float, 4096 columns, two blocks: three groups of stages one way, five the other).
-template <typename T> inline int64_t bw_snapshot_need(const Problem& q0) {
-  int64_t best = 0;
-  for (int inc = 0; inc < 2; ++inc) {
-    Problem q = q0;
-    q.inc = inc != 0;
-    MmaLayout M;
-    BwLayout<T> lay;
-    if (mma_layout<T>(q, M)) {
-      best = std::max<int64_t>(best, (int64_t)(M.kept() + kMmaSpare));
-    } else {
-      if (const int rc = plan_bw<T>(q, lay)) return rc;
-      best = std::max<int64_t>(best, (int64_t)lay.ws_bytes);
-    }
-  }
-  return best;
+// What a saving forward has to leave for the backward.  The directions differ: one may run as tensor-core passes and the other
+// as phases (float, 4096 columns, two blocks: three groups of stages one way, five the other).
+template <typename T> inline int64_t bw_snapshot_need(const Problem& q) {
+  MmaLayout M;
+  return mma_layout<T>(q, M) ? (int64_t)(M.kept() + kMmaSpare) : phases_bw_bytes<T>(q);
 }
 
 // Forward that also writes, into ws, the phase-boundary activations the backward of the same

@@ -939,6 +939,7 @@ const char* bfly_strerror(int status) {
 int bfly_version(void) { return 200; }
 int bfly_set_option(const char* name, int value) { return set_option(name, value); }
 int bfly_get_option(const char* name, int* value) { return get_option(name, value); }
+int64_t bfly_option_changes(void) { return option_changes().load(); }
 int bfly_cuda_version(void) { return CUDA_VERSION; }
 int64_t bfly_launch_count(void) { return g_launches.load(); }
 
@@ -1151,13 +1152,17 @@ int bfly_bw_c64_saved(const void* twiddle, const void* x, int64_t x_sB, int64_t 
                       nstacks, log_n, nblocks, input_size, output_size, increasing_stride, snapshots, snapshot_bytes,
                       stream, true, nullptr, 0, true);
 }
-int64_t bfly_bw_snapshot_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks) {
-  Problem q{batch, nstacks, log_n, nblocks, 1, 1, true, false};
+int64_t bfly_fw_saving_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks, int increasing_stride) {
+  Problem q{batch, nstacks, log_n, nblocks, 1, 1, increasing_stride != 0, false};
   const int rc = check_problem(q);
   if (rc) return rc;
   if (dtype == BFLY_F32) return bw_snapshot_need<float>(q);
   if (dtype == BFLY_C64) return bw_snapshot_need<cf>(q);
   return BFLY_E_UNSUPPORTED;
+}
+int64_t bfly_bw_snapshot_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks) {
+  const int64_t up = bfly_fw_saving_bytes(dtype, batch, nstacks, log_n, nblocks, 1), down = bfly_fw_saving_bytes(dtype, batch, nstacks, log_n, nblocks, 0);
+  return up < 0 ? up : down < 0 ? down : std::max(up, down);
 }
 int bfly_fw_saving_ws(int dtype, const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, void* out, int batch, int nstacks, int log_n,
                       int nblocks, int input_size, int output_size, int increasing_stride, void* snapshots, size_t snapshot_bytes, void* stream) {

@@ -61,10 +61,10 @@ Tensor rows_view(const Tensor& t) {
 bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
 bool has_tangent(const c10::optional<Tensor>& t) { return t.has_value() && has_tangent(*t); }
 
-// Shared by the plain operator and the autograd node: with `snapshots` the forward also writes
-// the activations the backward starts its phases from (bfly_fw_*_saving).
+// Shared by the plain operator and the autograd node: with `snapshots`, a buffer of bfly_fw_saving_bytes, the forward also
+// writes there what the backward starts from.
 Tensor fw_impl(const Tensor& twiddle, const Tensor& input, bool increasing_stride,
-               c10::optional<int64_t> output_size, Tensor* snapshots) {
+               c10::optional<int64_t> output_size, const Tensor* snapshots) {
   BFLY_CHECK_CUDA(twiddle); BFLY_CHECK_CUDA(input); BFLY_CHECK_SAME_DEVICE(twiddle, input);
   BFLY_CHECK_DIM(twiddle, 6); BFLY_CHECK_DIM(input, 3);
   const int64_t batch = input.size(0), nstacks = input.size(1), input_size = input.size(2);
@@ -85,12 +85,9 @@ Tensor fw_impl(const Tensor& twiddle, const Tensor& input, bool increasing_strid
   auto stream = at::cuda::getCurrentCUDAStream();
   int rc;
   if (snapshots) {
-    const int64_t ws_bytes = bfly_bw_snapshot_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks);
-    TORCH_CHECK(ws_bytes >= 0, "butterfly_multiply failed: ", bfly_strerror((int)ws_bytes));
-    *snapshots = torch::empty({ws_bytes}, input.options().dtype(at::kByte));
-    void* sp = ws_bytes ? snapshots->data_ptr() : nullptr;
     rc = bfly_fw_saving_ws(dt, tw.data_ptr(), x.data_ptr(), x.stride(0), x.stride(1), output.data_ptr(), (int)batch, (int)nstacks, (int)log_n,
-                           (int)nblocks, (int)input_size, (int)out_size, increasing_stride, sp, (size_t)ws_bytes, stream.stream());
+                           (int)nblocks, (int)input_size, (int)out_size, increasing_stride, snapshots->data_ptr(), (size_t)snapshots->numel(),
+                           stream.stream());
   } else {
     // optional scratch of the forward (room for the re-ordered twiddles of its fastest kernel)
     const int64_t fws = bfly_fw_workspace_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks);
@@ -143,8 +140,8 @@ std::tuple<Tensor, Tensor> bw_impl(const Tensor& twiddle, const Tensor& input, c
   const Tensor g = rows_view(grad);
   Tensor d_twiddle = torch::empty_like(tw);
   Tensor d_input = torch::empty({batch, nstacks, std::max(input_size, n)}, input.options());
-  const int64_t kept = snapshots && snapshots->defined() ? bfly_bw_snapshot_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks) : 0;
-  const bool saved = kept > 0 && snapshots->numel() >= kept;
+  const int64_t kept = snapshots ? snapshots->numel() : 0;
+  const bool saved = kept > 0;
   const int64_t ws_bytes = saved ? bfly_bw_saved_workspace_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks)
                                  : bfly_bw_workspace_bytes(dt, (int)batch, (int)nstacks, (int)log_n, (int)nblocks);
   TORCH_CHECK(ws_bytes >= 0, "butterfly_multiply_bw failed: ", bfly_strerror((int)ws_bytes));
@@ -202,19 +199,18 @@ class ButterflyMultiply : public torch::autograd::Function<ButterflyMultiply> {
   static Tensor forward(AutogradContext* ctx, Tensor twiddle, Tensor input, bool increasing_stride,
                         c10::optional<int64_t> output_size, bool wants_grad) {
     ctx->saved_data["increasing_stride"] = increasing_stride;
-    bool save = false;
+    int64_t ws = 0;
     if (wants_grad && twiddle.is_cuda() && input.is_cuda() && twiddle.dim() == 6 && input.dim() == 3 &&
         (input.scalar_type() == at::kFloat || input.scalar_type() == at::kComplexFloat)) {
-      const int64_t ws = bfly_bw_snapshot_bytes(input.scalar_type() == at::kFloat ? BFLY_F32 : BFLY_C64,
-                                                 (int)input.size(0), (int)input.size(1), (int)twiddle.size(2),
-                                                 (int)twiddle.size(1));
-      save = ws > 0 && autograd_saves(ws);
+      ctx->saved_data["options"] = bfly_option_changes();
+      ws = bfly_fw_saving_bytes(input.scalar_type() == at::kFloat ? BFLY_F32 : BFLY_C64, (int)input.size(0), (int)input.size(1),
+                                (int)twiddle.size(2), (int)twiddle.size(1), increasing_stride);
     }
-    if (!save) {
+    if (ws <= 0 || !autograd_saves(ws)) {
       ctx->save_for_backward({twiddle, input});
       return butterfly_multiply_fw(twiddle, input, increasing_stride, output_size);
     }
-    Tensor snapshots;
+    const Tensor snapshots = torch::empty({ws}, input.options().dtype(at::kByte));
     Tensor out = fw_impl(twiddle, input, increasing_stride, output_size, &snapshots);
     ctx->save_for_backward({twiddle, input, snapshots});
     return out;
@@ -222,7 +218,7 @@ class ButterflyMultiply : public torch::autograd::Function<ButterflyMultiply> {
   static variable_list backward(AutogradContext* ctx, variable_list grad_output) {
     auto saved = ctx->get_saved_variables();
     auto result = bw_impl(saved[0], saved[1], grad_output[0], ctx->saved_data["increasing_stride"].toBool(),
-                          saved.size() > 2 ? &saved[2] : nullptr);
+                          saved.size() > 2 && ctx->saved_data["options"].toInt() == bfly_option_changes() ? &saved[2] : nullptr);
     return {std::get<0>(result), std::get<1>(result), Tensor(), Tensor(), Tensor()};
   }
 };
@@ -371,6 +367,7 @@ class ButterflyLayer : public torch::autograd::Function<ButterflyLayer> {
                         bool increasing_stride, int64_t out_size, bool wants_grad) {
     const Tensor t2 = twiddle2.has_value() ? *twiddle2 : Tensor();
     Tensor snapshots;
+    if (wants_grad) ctx->saved_data["options"] = bfly_option_changes();
     Tensor out = layer_fw(twiddle, t2, input, bias, increasing_stride, out_size, wants_grad ? &snapshots : nullptr);
     if (wants_grad) {
       ctx->saved_data["increasing_stride"] = increasing_stride;
@@ -382,7 +379,7 @@ class ButterflyLayer : public torch::autograd::Function<ButterflyLayer> {
   static variable_list backward(AutogradContext* ctx, variable_list grad_output) {
     auto saved = ctx->get_saved_variables();
     auto r = layer_bw(saved[0], saved[1], saved[2], grad_output[0], ctx->saved_data["increasing_stride"].toBool(),
-                      ctx->saved_data["bias"].toBool(), saved[3]);
+                      ctx->saved_data["bias"].toBool(), ctx->saved_data["options"].toInt() == bfly_option_changes() ? saved[3] : Tensor());
     return {r.twiddle, r.twiddle2, r.input, r.bias, Tensor(), Tensor(), Tensor()};
   }
 };

@@ -183,7 +183,12 @@ int bfly_bw_c64_saved(const void* twiddle, const void* x, int64_t x_sB, int64_t 
 /* The same pair with the two kinds of scratch apart: what the saving forward leaves (bfly_bw_snapshot_bytes), and the
  * backward's own work space (bfly_bw_saved_workspace_bytes, may be 0), so that nothing but the activations is held between
  * the two.  Large products run as tensor-core passes here and in bfly_bw_*, whose planes need that; the pair above stays
- * on the phase kernels.  dtype is BFLY_F32 or BFLY_C64. */
+ * on the phase kernels.  dtype is BFLY_F32 or BFLY_C64.  bfly_fw_saving_bytes is the need of one direction (the products of
+ * the two may run differently), bfly_bw_snapshot_bytes the larger of both.  Options (bfly_set_option) are not to be set between
+ * the two calls; bfly_option_changes tells: the number of times that one was set in this process.  The torch operators
+ * recompute what they had saved if it has grown. */
+int64_t bfly_fw_saving_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks, int increasing_stride);
+int64_t bfly_option_changes(void);
 int64_t bfly_bw_snapshot_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks);
 int64_t bfly_bw_saved_workspace_bytes(int dtype, int batch, int nstacks, int log_n, int nblocks);
 int bfly_fw_saving_ws(int dtype, const void* twiddle, const void* x, int64_t x_sB, int64_t x_sS, void* out, int batch,
@@ -200,7 +205,7 @@ int bfly_bw_saved_ws(int dtype, const void* twiddle, const void* x, int64_t x_sB
  * per-thread tile copies instead of the TMA unit), "fw2" (BFLY_FW2: 0 = generic forward kernel
  * only), "bw_v2" (BFLY_BW_V2), "fw_kmax", "fw_rows", "fw_logcmax", "bw_rows", "bw_maxsg" (planner
  * overrides; -1 = default), "mma" (BFLY_MMA: tensor-core passes of large products; 0 never, 1 wherever they can run, -1 by
- * size; not to be changed between a saving forward and its backward), "fw_spread" (BFLY_FW_SPREAD), "virtual_rows" (BFLY_VIRTUAL_ROWS: 0 = rows one by
+ * size), "fw_spread" (BFLY_FW_SPREAD), "virtual_rows" (BFLY_VIRTUAL_ROWS: 0 = rows one by
  * one), "autograd_save" (BFLY_AUTOGRAD_SAVE: the torch autograd operators, butterfly_multiply and the layers, keep
  * the forward's snapshots: 0 never, 1 always, -1 by size).  Returns BFLY_E_ARG for an unknown name. */
 int bfly_set_option(const char* name, int value);

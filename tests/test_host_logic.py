@@ -703,3 +703,17 @@ def test_queried_bytes_are_enough_for_what_runs(emul, dtype, how):
                             routes[log_n, B, S, nb, base4, inc] = passes.value > 0
     one_way = [k for k, v in routes.items() if v and not routes[k[:-1] + (1 - k[-1],)]]
     assert one_way and any(routes.values()) and not all(routes.values())
+
+
+def test_saved_bytes_of_one_direction():
+    """What is held between forward and backward is what the direction needs, not the larger of both (three planes of phases
+    against two of passes for 16384 rows of 4096 floats, two blocks)."""
+    from butterfly_b200 import abi
+    lib = abi.lib()
+    for name in ("bfly_fw_saving_bytes", "bfly_bw_snapshot_bytes"):
+        getattr(lib, name).restype = ctypes.c_int64
+    up, down = (lib.bfly_fw_saving_bytes(0, 16384, 1, 12, 2, inc) for inc in (1, 0))
+    plane = 16384 * 4096 * 4
+    assert 2 * plane < up < 2.1 * plane and 3 * plane < down < 3.1 * plane
+    assert lib.bfly_bw_snapshot_bytes(0, 16384, 1, 12, 2) == max(up, down)
+    assert lib.bfly_fw_saving_bytes(0, 16384, 1, 40, 2, 1) < 0

@@ -225,6 +225,32 @@ def test_large_training_steps_under_the_default_rule(dev, cplx, log_n, B, inc):
     assert bb.abi.device_error() == 0
 
 
+@pytest.mark.parametrize("kind", ["multiply", "layer", "base4"])
+@pytest.mark.parametrize("first,then", [(1, 0), (0, 1)])
+def test_an_option_set_between_forward_and_backward(dev, kind, first, then):
+    """What the forward saved is laid out for the passes or for the phases; a backward after the switch does not read it."""
+    import butterfly_b200 as bb
+    torch.manual_seed(6)
+    if kind == "multiply":
+        tw = (torch.randn(1, 2, 9, 256, 2, 2, device=dev) / 2 ** 0.5).requires_grad_(True)
+        f, params = lambda r: bb.butterfly_multiply(tw, r, True), [tw]
+    else:
+        f = (bb.ButterflyBase4 if kind == "base4" else bb.Butterfly)(512, 512, bias=False, nblocks=2).to(dev)
+        params = [p for p in f.parameters() if p.numel()]
+    x = torch.randn(300, *((1,) if kind == "multiply" else ()), 512, device=dev, requires_grad=True)
+    g = torch.randn_like(x)
+    res = []
+    for a, b in ((first, then), (0, 0)):
+        with abi_option("autograd_save", 1):
+            with abi_option("mma", a):
+                y = f(x)
+            with abi_option("mma", b):
+                res.append(torch.autograd.grad(y, [x] + params, g))
+    for a, b in zip(*res):
+        assert ((a - b).norm() / b.norm()).item() < 2 * TOL_GRAD
+    assert bb.abi.device_error() == 0
+
+
 @pytest.mark.parametrize("cplx", [False, True])
 def test_the_pair_of_one_buffer_stays_on_the_phases(dev, cplx):
     """bfly_fw_*_saving and bfly_bw_*_saved have no work space for the passes, wherever these would run."""
