@@ -399,24 +399,40 @@ template <typename T> int plan_bw(const Problem& q, BwLayout<T>& lay);
 template <typename E, typename = void> struct has_mma : std::false_type {};
 template <typename E> struct has_mma<E, decltype((void)E::kMma)> : std::true_type {};
 
-// Microseconds of a training step, passes against phases, fitted to measurements of 2^20 to 2^25 floats (f = 1: 2^25).
-// A group costs a forward and a backward pass, an operator its block in the kernels before and after them.  A stage of the
-// phases costs more where rows are complex, wide or (complex) narrow and where factors are radix 4.  Measured, us, phases
-// against passes, in short runs: float 4096 two blocks 2^25 669 : 532, 2^24 371 : 333; float 1024 two blocks 2^25 576 : 510, 2^24
-// 323 : 326; float 4096 one block 383 : 493; float 8192 two blocks (five groups) 815 : 859; radix 4, 16384, 642 : 549;
-// complex 2048 514 : 482, 1024 two blocks 845 : 497, 256 two blocks 1180 : 495, 512 one block with 2^21 123 : 131.
-// Radix-2 floats below 0.75 2^25 stay on the phases altogether: little to gain, and a forward that records keeps the bits
-// of one that does not.  The margin: under the power cap (runs above 0.1 s) the clock falls to 1.65 GHz with the passes and
-// stays at 1.96 with the phases (complex 2048: 535 against 514 then).  (Forward-only calls stay there at any size: the packed-pair kernel keeps rows on chip.)
+// Microseconds of a training step, passes against phases, for f times 2^25 floats.  Fitted to 280 shapes (2^21 to 2^26 floats,
+// n from 32 to 16384, one to four blocks, both directions, one to eight stacks) in loops of 0.7 s: there the passes meet the
+// power cap (1.65 to 1.9 GHz) and the phases do not, so that short runs do better than this, by up to 15 %.
+// Passes: a group costs a forward and a backward pass, 150 us at f = 1, and its operators, a chain as long as its stages, with
+// many partial sums where rows have one window only; below a total of about 200 us the launches count.  Activations beyond
+// 1 GiB are not kept (autograd_saves) and are made again.  Phases: us per stage at f = 1, and per launch; complex rows below
+// 1024 columns run their backward stage by stage.
+// Long and short runs, us, phases / passes: float two blocks 4096 columns f = 2 1212 / 1065 (1208 / 940), f = 1 661 / 604
+// (661 / 550), f = 0.5 364 / 363; 2048 columns f = 1 602 / 582; 1024 columns f = 2 1040 / 1046, f = 1 570 / 576 (stay on the phases, like
+// every float product of one block: 378 / 559 at 4096).  Radix 4 16384 f = 2 1171 / 1087 (1170 / 977), f = 1 641 / 634 (phases); 4096 two blocks
+// f = 0.25 284 / 226, f = 0.125 172 / 181 (phases).  Complex 1024 two blocks f = 1 846 / 582, f = 0.125 224 / 194, f = 0.0625 166 / 164
+// (phases); 2048 one block f = 1 515 / 563 (phases); 512 one block f = 0.5 376 / 310, f = 0.25 201 / 201 (phases); 64 two blocks f = 1
+// 1577 / 545.  Products that decrease first have more groups: complex 1024 two blocks f = 1 849 / 910 (phases).
+// (Forward-only calls stay there at any size: the packed-pair kernel keeps rows on chip.)
 inline bool mma_pays(const Problem& q, int F, int ng) {
   if (q.B < 512) return false;  // an operator meets too few rows
   const double f = (double)((int64_t)q.B * q.S << (q.log_n + F)) / (1 << 25), w = (double)q.nblocks * q.log_n;
-  const double passes = 35 + 0.08 * ng * (double)((int64_t)q.S << (q.log_n + F - kMmaWin)) + ng * (17 + 128 * f);
+  const double operators = (double)((int64_t)q.S << (q.log_n + F - kMmaWin));
+  const bool radix2 = !F && !q.base4;
+  double passes = 43 + 3.4 * w + ng * (150 * f + 0.14 * operators + 55 / operators + (radix2 ? 4 : 0));
+  if ((ng - 1) * f >= 8) passes += (ng - 1) * (8 + 65 * f);
+  passes = std::max(passes, 120. + 25 * ng);
   double phases;
-  if (F) phases = q.log_n <= 9 ? 60 + 70 * w * f : 90 + 38.5 * w * f;
-  else if (q.base4) phases = q.log_n <= 12 ? 75 + 30 * w * f : 65 + 38 * w * f;
-  else phases = f < 0.75 ? 0 : 45 + 25 * w * f;
-  return passes * 1.12 < phases;
+  if (F && q.log_n <= 9) {
+    const int l = q.log_n;
+    phases = 10 + 25 * q.nblocks + (l <= 5 ? 150 : l == 6 ? 120 : l == 7 ? 78 : l == 8 ? 70 : 74) * w * f;
+  } else if (F) {
+    phases = 50 + 45 * q.nblocks + (q.log_n == 10 ? 33.5 : 38) * w * f;
+  } else if (q.base4) {
+    phases = q.log_n <= 12 ? 60 + 20 * q.nblocks + 29 * w * f : 50 + 50 * q.nblocks + (q.log_n == 13 ? 35.5 : 37.5) * w * f;
+  } else {
+    phases = 50 + 10 * q.nblocks + 24.5 * w * f;
+  }
+  return passes * 1.03 < phases;
 }
 
 // What the phases need behind the passes, for values that are not ordinary; negative where they do not run.

@@ -204,7 +204,7 @@ def test_the_largest_ordinary_values_stay_on_the_passes(dev, oracle_mod):
     assert rel2(y, want_y) < TOL and rel2(dx, want_dx) < TOL and rel2(d, want_d) < TOL_GRAD
 
 
-@pytest.mark.parametrize("cplx,log_n,B", [(False, 12, 16384), (True, 10, 1024)])
+@pytest.mark.parametrize("cplx,log_n,B", [(False, 12, 16384), (True, 10, 4096)])
 @pytest.mark.parametrize("inc", [True, False])
 def test_large_training_steps_under_the_default_rule(dev, cplx, log_n, B, inc):
     """Two blocks: one direction runs as passes, the other, which is cut into more groups, on the phases.  Both train, and agree
@@ -215,11 +215,15 @@ def test_large_training_steps_under_the_default_rule(dev, cplx, log_n, B, inc):
     tw = (torch.randn(1, 2, log_n, n // 2, 2, 2, dtype=dt, device=dev) / 2 ** 0.5).requires_grad_(True)
     x, g = (torch.randn(B, 1, n, dtype=dt, device=dev) for _ in range(2))
     x.requires_grad_(True)
-    got = []
+    got, passes = [], []
     for mma in (-1, 0):
         with abi_option("mma", mma):
+            bb.abi.profile_enable()
             y = bb.butterfly_multiply(tw, x, inc)
             got.append([y.detach()] + list(torch.autograd.grad(y, [tw, x], g)))
+            passes.append(sum(n for k, (n, _) in bb.abi.profile_collect().items() if "mma" in k))
+            bb.abi.profile_enable(False)
+    assert (passes[0] > 0) == inc and passes[1] == 0
     for a, b in zip(*got):
         assert ((a - b).norm() / b.norm()).item() < 2e-6
     assert bb.abi.device_error() == 0
