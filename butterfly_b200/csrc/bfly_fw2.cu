@@ -378,7 +378,9 @@ static int fw2_launch_ctas(const Fw2Params& p, const Fw2Maps& maps, int grid, si
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(grid); c.blockDim = dim3(THREADS); c.dynamicSmemBytes = smem; c.stream = stream;
   c.attrs = &attr; c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, bfly_fw2_kernel<CTAS, THREADS, TAIL>, p, maps, err) == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
+  if (cudaLaunchKernelEx(&c, bfly_fw2_kernel<CTAS, THREADS, TAIL>, p, maps, err) == cudaSuccess) return BFLY_OK;
+  cudaGetLastError();  // reported here, not by the next call that asks
+  return BFLY_E_CUDA;
 }
 
 int fw2_launch(const Fw2Params& p_in, int ctas_per_sm, int sms, cudaStream_t stream, int* err, int* launches) {
