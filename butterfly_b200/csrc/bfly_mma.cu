@@ -6,6 +6,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <type_traits>
 
 #include "bfly_fast.h"
@@ -912,16 +913,42 @@ __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_post_kernel(c
 
 // ------------------------------------------------------------------ launches
 
-template <typename K> int smem_attr(K kernel, uint32_t bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess ? BFLY_OK : BFLY_E_CUDA;
-}
+// Room for `bytes` of dynamic shared memory, the most that any launch of the kernel asks for: set once per device, since
+// threads with launches of different sizes would undo one another's setting.
+struct SmemOnce {
+  std::mutex mu;
+  bool done[64] = {false};
+  template <typename K> int operator()(K kernel, uint32_t bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BFLY_E_NODEVICE;
+    std::lock_guard<std::mutex> lk(mu);
+    if (done[dev]) return BFLY_OK;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return BFLY_E_CUDA;
+    }
+    done[dev] = true;
+    return BFLY_OK;
+  }
+};
 int launched() { return cudaGetLastError() == cudaSuccess ? BFLY_OK : BFLY_E_CUDA; }
 
 template <bool BW, bool IN_P, bool X_P, bool OUT_P> int pass_launch(const MmaPass& p, int ctas, cudaStream_t stream, int* err) {
   constexpr uint32_t bytes = pass_bytes<PassMem<BW, IN_P, OUT_P>>();
   static_assert(bytes <= 227 * 1024, "shared memory of a CTA");
-  if (int rc = smem_attr(bfly_mma_pass_kernel<BW, IN_P, X_P, OUT_P>, bytes)) return rc;
+  static SmemOnce smem;
+  if (int rc = smem(bfly_mma_pass_kernel<BW, IN_P, X_P, OUT_P>, bytes)) return rc;
   bfly_mma_pass_kernel<BW, IN_P, X_P, OUT_P><<<ctas, kPassThreads, bytes, stream>>>(p, err);
+  return launched();
+}
+
+// `stages`: most factors of a group, whose products the kernel keeps.
+template <bool CPLX, bool FOUR> int post_launch(const MmaPost& p, int stages, cudaStream_t stream) {
+  constexpr int W = Num<CPLX>::W, size = CPLX ? 8 : 4;
+  auto bytes = [](int stages) { return (uint32_t)(size * (2 * W * W + 2 * kMmaMaxStages * 2 * W + (stages - 1) * W * W)); };
+  static SmemOnce smem;
+  if (int rc = smem(bfly_mma_post_kernel<CPLX, FOUR>, bytes(kMmaMaxStages))) return rc;
+  bfly_mma_post_kernel<CPLX, FOUR><<<dim3(p.nq, p.S, p.ng), op_threads(CPLX, FOUR), bytes(stages), stream>>>(p);
   return launched();
 }
 
@@ -960,7 +987,6 @@ int mma_bw_launch(const MmaPass& p, int most, cudaStream_t stream, int* err) {
 
 // Groups of few factors need less shared memory (two CTAs to an SM up to seven), so they go in a launch of their own.
 int mma_post_launch(const MmaPost& all, bool cplx, cudaStream_t stream, int* launches) {
-  const int W = cplx ? 32 : 64, size = cplx ? 8 : 4;
   for (int many = 1; many >= 0; --many) {
     MmaPost p = all;
     p.ng = 0;
@@ -972,17 +998,9 @@ int mma_post_launch(const MmaPost& all, bool cplx, cudaStream_t stream, int* lau
         stages = std::max(stages, all.g[i].nst);
       }
     if (!p.ng) continue;
-    const uint32_t bytes = (uint32_t)(size * (2 * W * W + 2 * kMmaMaxStages * 2 * W + (stages - 1) * W * W));
-    const dim3 grid(p.nq, p.S, p.ng);
-    auto go = [&](auto kernel, int threads) -> int {
-      if (int rc = smem_attr(kernel, bytes)) return rc;
-      kernel<<<grid, threads, bytes, stream>>>(p);
-      return launched();
-    };
-    const bool four = has_radix4(p.g, p.ng);
-    if (int rc = cplx ? go(bfly_mma_post_kernel<true, true>, op_threads(true, true))
-                      : four ? go(bfly_mma_post_kernel<false, true>, op_threads(false, true)) : go(bfly_mma_post_kernel<false, false>, op_threads(false, false)))
-      return rc;
+    const int rc = cplx ? post_launch<true, true>(p, stages, stream)
+                   : has_radix4(p.g, p.ng) ? post_launch<false, true>(p, stages, stream) : post_launch<false, false>(p, stages, stream);
+    if (rc) return rc;
     ++*launches;
   }
   return BFLY_OK;

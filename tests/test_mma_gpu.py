@@ -323,3 +323,36 @@ def test_no_further_from_float64_than_the_phases(dev, oracle_mod, kind, cplx, lo
     assert passes[0] <= phases[0] and passes[1] <= phases[1] and passes[2] < 4 * 2 ** -24 + 3 * 2 ** -24
     if kind in ("identity", "permutation", "powers of two"):
         assert passes[:2] == [0.0, 0.0]
+
+
+def test_threads_with_products_of_different_groups(dev):
+    """Launches of one kernel with different amounts of shared memory, from two host threads on streams of their own."""
+    import threading
+    import butterfly_b200 as bb
+    torch.manual_seed(8)
+    jobs = []
+    for log_n, nblocks in ((6, 2), (10, 1)):  # groups of twelve factors, and of five
+        tw = torch.randn(1, nblocks, log_n, 1 << (log_n - 1), 2, 2, device=dev) / 2 ** 0.5
+        x, g = (torch.randn(200, 1, 1 << log_n, device=dev) for _ in range(2))
+        jobs.append((tw, x, g))
+    got, errors = [[], []], []
+    with abi_option("mma", 1):
+        want = [bb.butterfly_multiply_bw(*j, True) for j in jobs]
+        torch.cuda.synchronize()
+
+        def work(k):
+            try:
+                with torch.cuda.stream(torch.cuda.Stream(dev)):
+                    for _ in range(200):
+                        got[k] = bb.butterfly_multiply_bw(*jobs[k], True)
+                    torch.cuda.current_stream().synchronize()
+            except Exception as e:  # (a refused launch)
+                errors.append(e)
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    assert not errors
+    for a, b in zip(want, got):
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
