@@ -527,7 +527,7 @@ def run_gpu_arm(args):
     (dom_op, dom), (dom_launches, dom_ms) = max(shares.items(), key=lambda kv: kv[1][1])
     # the backward's phase launches carry the backward's algorithmic bytes; its forward pass
     # (snapshots) is extra work of the design and gets none
-    phase_kernels = [k for (op, k) in shares if op == "bw" and k.startswith(("bfly_bw", "bfly_mma_bw"))]
+    phase_kernels = [k for (op, k) in shares if op == "bw" and k.startswith(("bfly_bw", "bfly_mma_pass_kernel (backward)"))]
     if dom_op == "fw":
         alg = fwb / dom_launches
     elif dom in phase_kernels:

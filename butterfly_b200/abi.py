@@ -395,8 +395,8 @@ def device_error():
     return rc
 
 
-KERNEL_NAMES = ("bfly_fw_kernel", "bfly_bw_kernel", "bfly_fw2_kernel", "bfly_bw2_kernel", "bfly_bw3_kernel", "bfly_mma_fw_kernel",
-                "bfly_mma_bw_kernel", "bfly_mma_operator_kernels")
+KERNEL_NAMES = ("bfly_fw_kernel", "bfly_bw_kernel", "bfly_fw2_kernel", "bfly_bw2_kernel", "bfly_bw3_kernel", "bfly_mma_pass_kernel (forward)",
+                "bfly_mma_pass_kernel (backward)", "bfly_mma_prep_kernel, bfly_mma_post_kernel")
 
 
 def profile_enable(on=True):

@@ -320,7 +320,7 @@ template <bool BW, bool IN_P, bool OUT_P> struct PassMem {
 constexpr uint32_t kOuterCol = 256;
 
 struct Control {
-  uint64_t gfull[4], gempty[4];  // operand tile (backward: first operand): written, read by the products
+  uint64_t gfull[2], gempty[2];  // operand tile (backward: first operand): written, read by the products
   uint64_t xfull;                // backward, second operand: written (read: pfull)
   uint64_t dfull[2], dempty[2];  // transformed tile in tensor memory: complete, taken out
   uint64_t pfull, pempty;        // operator gradient: complete for a tile, taken out
@@ -396,11 +396,9 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
     return;
   }
   if (tid == 0) {
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&ctl->gfull[i]), kCutWarps);
       mbar_init(smem_u32(&ctl->gempty[i]), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&ctl->dfull[i]), 1);
       mbar_init(smem_u32(&ctl->dempty[i]), kStoreWarps);
     }

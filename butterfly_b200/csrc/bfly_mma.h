@@ -5,7 +5,8 @@
 // block of 64 columns ("operator").  A pass multiplies tiles of 128 rows by these operators; the backward multiplies the
 // gradient by the transposed operator and accumulates the gradient of the whole operator, g^T x over the rows, which
 // a small kernel takes apart into the gradients of the stages afterwards.  Per pass a tile crosses shared memory once,
-// whatever the number of stages, and the operators' arithmetic costs a quarter of the tile's trip through HBM.
+// whatever the number of stages.  The operators' arithmetic takes 1152 clocks of a tile (2432 in the backward) where the
+// tile's trip through HBM takes 2900 (4300).
 //
 // Precision.  A float32 value, scaled (kMmaScale), is the exact sum of three bfloat16 slices (8 + 8 + 8 bits).  Operators are multiplied out in
 // float64 and cut into four parts, the first of few bits.  Nine of the twelve products are formed (the others are below

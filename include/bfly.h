@@ -331,8 +331,8 @@ int bfly_selftest_bounded_wait(int polls, void* stream);
 #define BFLY_KERNEL_FW2 2  /* packed-pair forward kernel with its twiddle re-ordering kernel (bfly_fw2_kernel) */
 #define BFLY_KERNEL_BW2 3  /* backward phase kernel with accumulators in tensor memory (bfly_bw2_kernel) */
 #define BFLY_KERNEL_BW3 4  /* packed-pair backward phase kernel (bfly_bw3_kernel) */
-#define BFLY_KERNEL_MMA_FW 5  /* tensor-core forward pass (bfly_mma_fw_kernel) */
-#define BFLY_KERNEL_MMA_BW 6  /* tensor-core backward pass (bfly_mma_bw_kernel) */
+#define BFLY_KERNEL_MMA_FW 5  /* tensor-core pass, forward (bfly_mma_pass_kernel) */
+#define BFLY_KERNEL_MMA_BW 6  /* tensor-core pass, backward (the same kernel) */
 #define BFLY_KERNEL_MMA_OPS 7 /* their operators and the stages' gradients (bfly_mma_prep_kernel, bfly_mma_post_kernel) */
 #define BFLY_KERNEL_IDS 8
 void bfly_profile_enable(int on);
