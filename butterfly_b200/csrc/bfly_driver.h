@@ -1292,6 +1292,21 @@ template <typename T> inline size_t mma_layer_bw_bytes(const Problem& q, int out
   if (plan_layer_bw<T>(q, out_total, false, L) != BFLY_OK) L.ws_bytes = 0;  // (mma_layout asked)
   return std::max(M.bw_bytes(saved) + (q.S > 1 && !mma_layer_adds<T>(q, out_total) ? (size_t)q.B * q.S * DX * sizeof(T) : 0), kMmaHead + L.ws_bytes);
 }
+// What a layer's forward leaves, and the work space of its backward.
+template <typename T> inline int64_t layer_snapshot_need(const Problem& q, int out_total) {
+  MmaLayout M;
+  if (out_total > 0 && mma_layout<T>(q, M)) return (int64_t)(M.kept() + kMmaSpare);
+  BwLayout<T> lay;
+  const int rc = plan_bw<T>(q, lay);
+  return rc ? rc : (lay.chunked ? 0 : (int64_t)lay.ws_bytes);
+}
+template <typename T> inline int64_t layer_bw_need(const Problem& q, int out_total, bool saved) {
+  MmaLayout M;
+  if (out_total > 0 && mma_layout<T>(q, M)) return (int64_t)(mma_layer_bw_bytes<T>(q, out_total, M, saved) + kMmaSpare);
+  LayerBwLayout L;
+  const int rc = plan_layer_bw<T>(q, out_total, saved, L);
+  return rc ? rc : (int64_t)L.ws_bytes;
+}
 template <typename T, typename E>
 int drive_mma_layer_bw(E& ex, const Problem& q, const MmaLayout& M, const T* tw2, const T* tw4, const T* x, int64_t x_sB, const T* grad, int64_t g_sB,
                        T* d_tw2, T* d_tw4, T* d_in, T* d_bias, int out_total, void* saved, size_t saved_bytes, void* ws, size_t ws_bytes) {

@@ -1081,11 +1081,7 @@ int bfly_linear_bw_f32(const float* twiddle, const float* x, int64_t x_sB, const
 int64_t bfly_layer_snapshot_bytes(const bfly_layer_t* l) {
   if (!l) return BFLY_E_ARG;
   return layer_call(l, [&](auto t, const Problem& q) -> int64_t {
-    MmaLayout M;
-    if (l->output_size > 0 && mma_layout<decltype(t)>(q, M)) return (int64_t)(M.kept() + kMmaSpare);
-    BwLayout<decltype(t)> lay;
-    const int rc = plan_bw<decltype(t)>(q, lay);
-    return rc ? rc : (lay.chunked ? 0 : (int64_t)lay.ws_bytes);
+    return layer_snapshot_need<decltype(t)>(q, l->output_size);
   });
 }
 int bfly_layer_fw(const bfly_layer_t* l, const void* twiddle2, const void* twiddle4, const void* x, int64_t x_sB, void* out,
@@ -1103,11 +1099,7 @@ int bfly_layer_fw(const bfly_layer_t* l, const void* twiddle2, const void* twidd
 int64_t bfly_layer_bw_workspace_bytes(const bfly_layer_t* l, int with_snapshots) {
   if (!l) return BFLY_E_ARG;
   return layer_call(l, [&](auto t, const Problem& q) -> int64_t {
-    MmaLayout M;
-    if (l->output_size > 0 && mma_layout<decltype(t)>(q, M)) return (int64_t)(mma_layer_bw_bytes<decltype(t)>(q, l->output_size, M, with_snapshots != 0) + kMmaSpare);
-    LayerBwLayout L;
-    const int rc = plan_layer_bw<decltype(t)>(q, l->output_size, with_snapshots != 0, L);
-    return rc ? rc : (int64_t)L.ws_bytes;
+    return layer_bw_need<decltype(t)>(q, l->output_size, with_snapshots != 0);
   });
 }
 int bfly_layer_bw(const bfly_layer_t* l, const void* twiddle2, const void* twiddle4, const void* x, int64_t x_sB, const void* grad,

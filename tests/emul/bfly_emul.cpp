@@ -674,6 +674,85 @@ struct DryExec {
   int mma_post(const MmaPost&, bool) { return BFLY_OK; }
 };
 
+// A layer: bias, gradients of everything.
+template <typename T> int dry_layer(const Problem& q, int out_total, bool save, size_t skew, int* passes) {
+  DryExec ex;
+  const int64_t n = (int64_t)1 << q.log_n, DX = std::max<int64_t>(q.in_size, n);
+  int64_t stk[2];
+  twiddle_stack_sizes(q, stk);
+  T* tw2 = ex.buffer<T>(q.S * stk[0] * sizeof(T)), *tw4 = ex.buffer<T>(q.S * stk[1] * sizeof(T));
+  T* d2 = ex.buffer<T>(q.S * stk[0] * sizeof(T)), *d4 = ex.buffer<T>(q.S * stk[1] * sizeof(T));
+  T* x = ex.buffer<T>((size_t)q.B * q.in_size * sizeof(T)), *out = ex.buffer<T>((size_t)q.B * q.S * n * sizeof(T));
+  T* g = ex.buffer<T>((size_t)q.B * out_total * sizeof(T)), *dx = ex.buffer<T>((size_t)q.B * (q.S > 1 ? q.in_size : DX) * sizeof(T));
+  T* bias = ex.buffer<T>(out_total * sizeof(T)), *db = ex.buffer<T>(out_total * sizeof(T));
+  const int64_t kept = save ? layer_snapshot_need<T>(q, out_total) : 0;
+  if (kept < 0) return (int)kept;
+  const int64_t own = layer_bw_need<T>(q, out_total, kept > 0);
+  if (own < 0) return (int)own;
+  const size_t fws = kept > 0 || q.base4 ? 0 : fw_workspace_bytes<T>(q);
+  char* k = ex.buffer<char>(kept, skew), *f = ex.buffer<char>(fws, skew), *w = ex.buffer<char>(own, skew);
+  int rc = drive_layer_fw<T>(ex, q, tw2, tw4, x, q.in_size, out, bias, out_total, k, kept, f, fws);
+  if (rc == BFLY_OK) rc = drive_layer_bw<T>(ex, q, tw2, tw4, x, q.in_size, g, out_total, d2, d4, dx, db, out_total, k, kept, w, own);
+  *passes = ex.passes;
+  return rc ? rc : (ex.outside ? 1 : 0);
+}
+
+// Is the plan of the passes one?  Groups that hold all stages in order, windows that hold their bits, blocks that tile the
+// row, CTAs that take every tile once and leave no two sums in one slot.  0, or the number of what is wrong.
+template <typename T> int check_mma_plan(const Problem& q, int most) {
+  MmaLayout L;
+  if (!mma_layout<T>(q, L)) return 0;
+  const std::vector<Stage> st = problem_stages(q);
+  const int cols = 1 << L.log_nf;
+  int next = 0;
+  if (L.g.size() > (size_t)kMmaMaxGroups) return 1;
+  for (const MmaGroup& g : L.g) {
+    if (g.t0 != next || g.t1 <= g.t0 || g.nst != g.t1 - g.t0) return 2;
+    next = g.t1;
+    int weight = 0, active = 0;
+    for (int k = 0; k < g.nst; ++k) {
+      const MmaStage& m = g.st[k];
+      const Stage& s = st[g.t0 + k];
+      weight += m.radix == 4 ? 2 : 1;
+      for (int b = 0; b < (m.radix == 4 ? 2 : 1); ++b) {
+        active |= 1 << (m.lbit + b);
+        if (g.geo.col(1 << (m.lbit + b + L.F)) != 1 << (s.bit + b + L.F)) return 3;  // the window's bit is the row's
+      }
+      if (m.gbit != s.bit || m.tw_off != s.tw_off || m.which != s.which || m.radix != s.radix) return 4;
+    }
+    if (weight > kMmaMaxStages || (active & g.passive) || (active | g.passive) != (kMmaCols >> L.F) - 1) return 5;
+    std::vector<char> seen(cols, 0);
+    for (int b = 0; b < L.nq; ++b)
+      for (int j = 0; j < kMmaCols; ++j) {
+        const int c = g.geo.base(b) + g.geo.col(j);
+        if (c < 0 || c >= cols || seen[c]++) return 6;
+      }
+    // the work, as Walk takes it
+    const int64_t blocks = (int64_t)q.S * L.nq, nt = L.nt;
+    const int ctas = mma_ctas(g.geo, blocks * nt, most), sib = g.geo.sib, G = ctas >> sib;
+    if (ctas < 1 || blocks % (1 << sib)) return 7;
+    const int64_t W = (blocks >> sib) * nt;
+    std::vector<char> tile(blocks * nt, 0), slot(blocks + kMmaBwMaxCtas, 0);
+    for (int cta = 0; cta < ctas; ++cta) {
+      const int c = cta >> sib;
+      int64_t last = -1;
+      for (int64_t w = mma_first_tile(W, G, c); w < mma_first_tile(W, G, c + 1); ++w) {
+        if (mma_cta_of(W, G, w) != c) return 8;
+        const int64_t block = ((w / nt) << sib) + (cta & ((1 << sib) - 1));
+        if (tile[block * nt + w % nt]++) return 9;
+        if (block != last) {
+          const int64_t at = mma_slot(g.geo, block, c);
+          if (at < 0 || at >= (int64_t)slot.size() || slot[at]++) return 10;
+          last = block;
+        }
+      }
+    }
+    for (char t : tile)
+      if (!t) return 11;
+  }
+  return next == (int)st.size() ? -(int)L.g.size() : 12;
+}
+
 // how: 0 the operator with saved activations and a work space of its own, 1 the backward that makes them itself.
 template <typename T> int dry_step(Problem q, int how, size_t skew, int* passes) {
   DryExec ex;
@@ -709,5 +788,16 @@ int bfly_emul_dry_step(int dtype, int base4, int how, int64_t skew, int B, int S
   Problem q{B, S, log_n, nblocks, in_size, out_size, inc != 0, base4 != 0};
   if (const int rc = check_problem(q)) return rc;
   return dtype == 0 ? dry_step<float>(q, how, (size_t)skew, passes) : dry_step<cf>(q, how, (size_t)skew, passes);
+}
+int bfly_emul_dry_layer(int dtype, int base4, int save, int64_t skew, int B, int S, int log_n, int nblocks, int in_size, int out_total, int inc, int* passes) {
+  Problem q{B, S, log_n, nblocks, in_size, 1 << log_n, inc != 0, base4 != 0};
+  if (const int rc = check_problem(q)) return rc;
+  return dtype == 0 ? dry_layer<float>(q, out_total, save != 0, (size_t)skew, passes) : dry_layer<cf>(q, out_total, save != 0, (size_t)skew, passes);
+}
+// minus the number of groups, 0 where the passes do not run, or what is wrong
+int bfly_emul_check_mma_plan(int dtype, int base4, int B, int S, int log_n, int nblocks, int inc, int ctas) {
+  Problem q{B, S, log_n, nblocks, 1 << log_n, 1 << log_n, inc != 0, base4 != 0};
+  if (const int rc = check_problem(q)) return rc;
+  return dtype == 0 ? check_mma_plan<float>(q, ctas) : check_mma_plan<cf>(q, ctas);
 }
 }

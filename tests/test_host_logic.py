@@ -705,6 +705,48 @@ def test_queried_bytes_are_enough_for_what_runs(emul, dtype, how):
     assert one_way and any(routes.values()) and not all(routes.values())
 
 
+@pytest.mark.parametrize("dtype", [0, 1], ids=["f32", "c64"])
+@pytest.mark.parametrize("save", [0, 1])
+def test_queried_bytes_are_enough_for_layers(emul, dtype, save):
+    """The same for whole layers: widths that are cut, several stacks, the last one cut short, bias."""
+    routes = set()
+    for log_n in (6, 9, 10, 12, 14):
+        n = 1 << log_n
+        for B in (5, 300, 777, 2048, 8192 + 3, 65536):
+            for in_size, out_total in ((n, n), (n - 24, n - 20), (n, 4 * n), (n - 24, 3 * n - 72), (n + 5, n), (n, 2 * n + 1)):
+                S = -(-out_total // n)
+                if B * S << log_n > 1 << 26:
+                    continue
+                for nb, base4, inc in ((1, 0, 1), (2, 0, 1), (2, 0, 0), (1, 1, 1), (2, 1, 1), (2, 1, 0)):
+                    passes = ctypes.c_int(0)
+                    rc = emul.bfly_emul_dry_layer(dtype, base4, save, I64(16), B, S, log_n, nb, in_size, out_total, inc, ctypes.byref(passes))
+                    assert rc == 0, (log_n, B, in_size, out_total, nb, base4, inc, rc)
+                    routes.add(passes.value > 0)
+    assert routes == {True, False}
+
+
+@pytest.mark.parametrize("dtype", [0, 1], ids=["f32", "c64"])
+def test_plan_of_the_passes(emul, dtype):
+    """Wherever the passes can run: every stage in one group and its bits in the group's window, every column in one block,
+    every tile at one CTA, every sum in a slot of its own."""
+    assert emul.bfly_emul_set_option(b"mma", 1) == 0
+    try:
+        groups = set()
+        for log_n in range(5, 16):
+            for nb in (1, 2, 3):
+                for base4 in (0, 1):
+                    for inc in (0, 1):
+                        for B, S, ctas in ((1, 1, 148), (300, 3, 148), (5000, 1, 148), (4097, 5, 132), (129, 2, 7), (20000, 1, 160)):
+                            if B * S << log_n > 1 << 25:
+                                continue
+                            got = emul.bfly_emul_check_mma_plan(dtype, base4, B, S, log_n, nb, inc, ctas)
+                            assert got <= 0, (log_n, nb, base4, inc, B, S, ctas, got)
+                            groups.add(-got)
+        assert {1, 2, 3, 5} <= groups
+    finally:
+        emul.bfly_emul_set_option(b"mma", -1)
+
+
 def test_saved_bytes_of_one_direction():
     """What is held between forward and backward is what the direction needs, not the larger of both (three planes of phases
     against two of passes for 16384 rows of 4096 floats, two blocks)."""

@@ -229,6 +229,32 @@ def test_large_training_steps_under_the_default_rule(dev, cplx, log_n, B, inc):
     assert bb.abi.device_error() == 0
 
 
+@pytest.mark.parametrize("cplx,log_n", [(False, 6), (False, 7), (True, 5)])
+def test_many_tiles_to_a_cta(dev, oracle_mod, cplx, log_n):
+    """700001 rows of one or two windows: 37 to 74 tiles of a block to every CTA, so that the sums that run on over 32 tiles are
+    taken out on the way and at the end, and the barriers go through many turns.  A product of n columns is an n x n matrix:
+    its gradient, made in float64, goes through the oracle."""
+    import butterfly_b200 as bb
+    n, B = 1 << log_n, 700001
+    dt, wide = (torch.complex64, torch.complex128) if cplx else (torch.float32, torch.float64)
+    torch.manual_seed(log_n)
+    tw = torch.randn(1, 2, log_n, n // 2, 2, 2, dtype=dt) / 2 ** 0.5
+    x, g = (torch.randn(B, 1, n, dtype=dt, device=dev) for _ in range(2))
+    with abi_option("mma", 1):
+        t, xd = tw.to(dev).requires_grad_(True), x.requires_grad_(True)
+        y = bb.butterfly_multiply(t, xd, True)
+        d, dx = torch.autograd.grad(y, [t, xd], g)
+    eye = torch.eye(n, dtype=wide).unsqueeze(1)
+    m = oracle_mod.multiply_fw(tw.to(wide), eye, True)[:, 0]  # row i: the product's i-th column
+    xw, gw = x.detach()[:, 0].to(wide), g[:, 0].to(wide)
+    want_d, _ = oracle_mod.multiply_bw(tw.to(wide), eye, (xw.conj().T @ gw).cpu().unsqueeze(1), True)
+    md = m.to(dev)
+    for got, want in ((y[:, 0], xw @ md), (dx[:, 0], gw @ md.conj().T)):
+        assert ((got.detach().to(wide) - want).norm() / want.norm()).item() < TOL
+    assert rel2(d, want_d) < TOL_GRAD
+    assert bb.abi.device_error() == 0
+
+
 @pytest.mark.parametrize("kind", ["multiply", "layer", "base4"])
 @pytest.mark.parametrize("first,then", [(1, 0), (0, 1)])
 def test_an_option_set_between_forward_and_backward(dev, kind, first, then):
