@@ -219,8 +219,8 @@ template <typename T> struct FwParams {
   // Virtual rows: a tile row is 2^vr consecutive rows of 2^log_n columns side by side (panel: one row of log_n + vr bits),
   // so that narrow rows fill the threads.  B and R count tile rows; B_rows the rows themselves.
   int vr, B_rows;
-  const int* guard;          // optional: nothing runs while *guard is 0
   FwGroup g[kMaxFwGroups];
+  const int* guard;          // optional: nothing runs while *guard is 0
 };
 
 // One sub-group of a backward phase.  With a 2-bit window (KW = 2): up to two radix-2
@@ -263,10 +263,10 @@ template <typename T> struct BwParams {
   int vr, B_rows;    // virtual rows, as in FwParams (B, Rb and the slices count tile rows)
   T* dbias;
   int dbias_len;
-  const int* guard;  // optional: nothing runs while *guard is 0
   Panel panel;
   int nsg;
   BwSg sg[kMaxSg];
+  const int* guard;  // optional: nothing runs while *guard is 0
 };
 
 // Rows of the tensors below tile row `end` of a slice.
