@@ -382,3 +382,28 @@ def test_threads_with_products_of_different_groups(dev):
     assert not errors
     for a, b in zip(want, got):
         assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+def test_captured_training_steps_look_at_the_values_of_each_replay(dev):
+    import butterfly_b200 as bb
+    torch.manual_seed(9)
+    tw = (torch.randn(1, 2, 9, 256, 2, 2, device=dev) / 2 ** 0.5).requires_grad_(True)
+    x, g = torch.randn(300, 1, 512, device=dev, requires_grad=True), torch.randn(300, 1, 512, device=dev)
+
+    def step():
+        y = bb.butterfly_multiply(tw, x, True)
+        return [y.detach()] + list(torch.autograd.grad(y, [x, tw], g))
+    with abi_option("mma", 1):
+        side = torch.cuda.Stream(dev)
+        with torch.cuda.stream(side):
+            step()
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = step()
+        for value in (1.0, float("inf"), 2.0, float("nan"), 3.0):
+            with torch.no_grad():
+                x.view(-1)[5] = value
+            graph.replay()
+            _same(outs, step(), (True, True, False))
+    assert bb.abi.device_error() == 0
