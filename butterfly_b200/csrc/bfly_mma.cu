@@ -733,11 +733,14 @@ __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_prep_kernel(c
   };
   if (threadIdx.x < 2 * kMmaCols) top[threadIdx.x / kMmaCols][threadIdx.x % kMmaCols] = -1100;
   __syncthreads();
+  static_assert(T % kMmaCols == 0 && kMmaCols % 32 == 0, "a thread stays in its column, a warp in a row");
+  int column = -1100;
   for (int it = threadIdx.x; it < kMmaCols * kMmaCols; it += T) {
-    const int j = it / kMmaCols, i = it % kMmaCols, e = ((__double2hiint(entry(j, i)) >> 20) & 0x7ff) - 1023;
-    atomicMax(&top[0][j], e);
-    atomicMax(&top[1][i], e);
+    const int e = ((__double2hiint(entry(it / kMmaCols, it % kMmaCols)) >> 20) & 0x7ff) - 1023, row = __reduce_max_sync(0xffffffffu, e);
+    column = max(column, e);
+    if ((threadIdx.x & 31) == 0) atomicMax(&top[0][it / kMmaCols], row);
   }
+  atomicMax(&top[1][threadIdx.x % kMmaCols], column);
   __syncthreads();
   uint8_t* img = p.images + (((int64_t)blockIdx.z * p.S + s) * p.nq + q) * kMmaImageBytes;
   for (int it = threadIdx.x; it < kMmaCols * 8; it += T) {
