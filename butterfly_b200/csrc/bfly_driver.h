@@ -456,7 +456,8 @@ template <typename T> inline bool mma_layout(const Problem& q, MmaLayout& L) {
   if (L.nt * L.nq * q.S >= ((int64_t)1 << 30)) return false;
   // ends in pieces below a sector: 2 to 4 times a pass
   if (opt < 0 && (std::min(L.g.front().geo.ib, L.g.back().geo.ib) < 3 || !mma_pays(q, L.F, (int)L.g.size()))) return false;
-  const size_t ng = L.g.size(), slots = (size_t)q.S * L.nq + kMmaBwMaxCtas;
+  L.parts = mma_parts((int64_t)q.S * L.nq, L.nt);
+  const size_t ng = L.g.size(), slots = L.slots_per_group(q.S);
   L.plane = (((size_t)q.S * kMmaRows * sizeof(float)) << L.log_nf) * L.nt;
   L.images = ng * q.S * L.nq * kMmaImageBytes;
   L.slots = ng * slots * kMmaSlotFloats * sizeof(float);
@@ -524,7 +525,7 @@ inline MmaPass mma_pass(const Problem& q, const MmaLayout& L, int g, const uint8
   MmaPass p;
   std::memset(&p, 0, sizeof(p));
   p.geo = L.g[g].geo;
-  p.S = q.S; p.B = q.B; p.nq = L.nq; p.nt = (int)L.nt;
+  p.S = q.S; p.B = q.B; p.nq = L.nq; p.nt = (int)L.nt; p.parts = L.parts;
   p.images = images + (size_t)g * q.S * L.nq * kMmaImageBytes;
   p.flag = flag;
   return p;
@@ -565,7 +566,7 @@ int drive_mma_bw(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, cons
   constexpr int F = (int)(sizeof(T) / 4);
   if (ws_bytes < L.bw_bytes(kept != nullptr)) return BFLY_E_WORKSPACE;
   const int ng = (int)L.g.size();
-  const size_t slots_per_group = (size_t)q.S * L.nq + kMmaBwMaxCtas;
+  const size_t slots_per_group = L.slots_per_group(q.S);
   char* gplane = ws + kMmaHead;
   int* flag = reinterpret_cast<int*>(ws);
   const int* kept_flag = reinterpret_cast<const int*>(kept);
@@ -601,7 +602,7 @@ int drive_mma_bw(E& ex, const Problem& q, const MmaLayout& L, const T* tw2, cons
   std::memset(&p, 0, sizeof(p));
   p.tw[0] = tw2; p.tw[1] = tw4; p.dtw[0] = d_tw2; p.dtw[1] = d_tw4;
   twiddle_stack_sizes(q, p.tw_stack);
-  p.S = q.S; p.nq = L.nq; p.nt = (int)L.nt; p.ng = ng; p.ctas = ctas; p.last_group = ng - 1;
+  p.S = q.S; p.nq = L.nq; p.nt = (int)L.nt; p.parts = L.parts; p.ng = ng; p.ctas = ctas; p.last_group = ng - 1;
   p.flag = flag;
   p.slots = slots; p.slots_group = (int64_t)slots_per_group * kMmaSlotFloats;
   if (d_bias) { p.bias_slots = bias_slots; p.dbias = reinterpret_cast<float*>(d_bias); p.dbias_len = bias_len * F; }

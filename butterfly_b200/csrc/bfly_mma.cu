@@ -369,7 +369,7 @@ struct Walk {
     at = Spot{block / nq, p.geo.base(block % nq), (int)(w % nt)};
   }
   __device__ bool more() const { return w < end; }
-  __device__ bool last_of_block() const { return at.tile + 1 == nt || w + 1 == end; }
+  __device__ bool last_of_part(const MmaParts& p) const { return at.tile + 1 == nt || w + 1 == end || p.ends(at.tile); }
   __device__ void next(const MmaPass& p) {
     ++w;
     if (++at.tile == nt) {
@@ -471,7 +471,8 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
       for (; at.more(); ++i) {
         if (!place(at.block)) break;
         const int block = at.block;
-        const bool last = at.last_of_block();
+        const bool last = at.last_of_part(p.parts);
+        const int part = p.parts.of(at.at.tile);
         at.next(p);
         uint8_t* op = sm + (i % ST) * kOpBytes;
         cut(std::integral_constant<bool, IN_P>(), op, va, &ctl->gfull[i % ST]);
@@ -498,7 +499,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
             if (tid < 64) {
               float v = 0.f;
               for (int k = 0; k < kCutWarps; ++k) v += sums[k * 64 + tid];
-              p.bias_slots[mma_slot(p.geo, block, blockIdx.x >> p.geo.sib) * 64 + tid] = v;
+              p.bias_slots[mma_slot(p.geo, p.parts, block, part, blockIdx.x >> p.geo.sib) * 64 + tid] = v;
             }
             if (!role_sync(ctl, &ctl->sync, turn)) break;
           }
@@ -526,7 +527,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
         fence_after_sync();
         issue_outer<IN_P, X_P>(tmem + kOuterCol, op, smem_u32(sm + Mem::x), kept > 0);
         mma_commit(smem_u32(&ctl->pfull));
-        kept = kept + 1 == kFlushTiles || at.last_of_block() ? 0 : kept + 1;
+        kept = kept + 1 == kFlushTiles || at.last_of_part(p.parts) ? 0 : kept + 1;
       }
       mma_commit(smem_u32(&ctl->gempty[s]));
       at.next(p);
@@ -539,6 +540,16 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
     float acc[BW ? 32 : 1];  // operator gradient: row `row` (two slices of the incoming gradient), columns j0 ..
 #pragma unroll
     for (int i = 0; i < (BW ? 32 : 1); ++i) acc[i] = 0.f;
+    if (BW && p.parts.begins(at.at.tile)) {  // a free slot in front
+      const int64_t free = mma_slot(p.geo, p.parts, at.block, p.parts.of(at.at.tile) - 1, blockIdx.x >> p.geo.sib);
+      float* dst = p.slots + free * kMmaSlotFloats + row * kMmaCols + j0;
+#pragma unroll
+      for (int c = 0; c < 32; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.bias_slots && e == 0) {
+        p.bias_slots[free * kMmaCols + lane] = 0.f;
+        p.bias_slots[free * kMmaCols + lane + 32] = 0.f;
+      }
+    }
     int kept = 0;
     for (uint32_t i = 0; at.more(); ++i) {
       const uint32_t d = i % DBUF;
@@ -562,7 +573,7 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
       if (BW) {
         if (!await_warp(ctl, &ctl->pfull, i & 1)) break;
         fence_after_sync();
-        const bool last = at.last_of_block(), flush = ++kept == kFlushTiles || last;
+        const bool last = at.last_of_part(p.parts), flush = ++kept == kFlushTiles || last;
         auto take = [&](uint32_t col, bool use) {  // (all warps together: a branch around the loads cost 30 us of 560)
 #pragma unroll
           for (int h = 0; h < 4; ++h) {
@@ -583,8 +594,8 @@ __global__ void __launch_bounds__(kPassThreads, 1) bfly_mma_pass_kernel(const __
         fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive(&ctl->pempty);
-        if (last) {  // the block's last tile here: leave its sums
-          float* dst = p.slots + mma_slot(p.geo, at.block, blockIdx.x >> p.geo.sib) * kMmaSlotFloats + row * kMmaCols + j0;
+        if (last) {  // the part's last tile here: leave its sums
+          float* dst = p.slots + mma_slot(p.geo, p.parts, at.block, p.parts.of(at.at.tile), blockIdx.x >> p.geo.sib) * kMmaSlotFloats + row * kMmaCols + j0;
 #pragma unroll
           for (int c = 0; c < (BW ? 32 : 0); c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
 #pragma unroll
@@ -842,17 +853,18 @@ __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_post_kernel(c
   S* R = reinterpret_cast<S*>(tw + kMmaMaxStages * 2 * W);  // before factor k: R + (k - 1) W W
   const MmaGroup& g = p.g[blockIdx.z];
   const int q = blockIdx.x, s = blockIdx.y, cbase = g.geo.base(q), tid = threadIdx.x;
-  // the CTAs of the backward pass that worked on this block; their sums, on their way while R is made
+  // what the CTAs of the backward pass left for this block; on its way while R is made
   const int sib = g.geo.sib, ctas = (p.ctas >> sib);
   const int64_t block = (int64_t)s * p.nq + q, first = (block >> sib) * p.nt, tiles = ((int64_t)p.S * p.nq >> sib) * p.nt;
-  const int c0 = mma_cta_of(tiles, ctas, first), c1 = mma_cta_of(tiles, ctas, first + p.nt - 1);
+  const int64_t slot0 = mma_slot(g.geo, p.parts, block, 0, mma_cta_of(tiles, ctas, first));
+  const int64_t slot1 = mma_slot(g.geo, p.parts, block, p.parts.of(p.nt - 1), mma_cta_of(tiles, ctas, first + p.nt - 1));
   constexpr int PER = kMmaCols * kMmaCols / THREADS;  // entries of a thread, neighbours
-  const float* slots = p.slots + p.group[blockIdx.z] * p.slots_group + mma_slot(g.geo, block, c0) * kMmaSlotFloats + tid * PER;
+  const float* slots = p.slots + p.group[blockIdx.z] * p.slots_group + slot0 * kMmaSlotFloats + tid * PER;
   double sum[PER];
 #pragma unroll
   for (int i = 0; i < PER; ++i) sum[i] = 0.0;
 #pragma unroll 2
-  for (int c = c0; c <= c1; ++c, slots += kMmaSlotFloats << sib) {
+  for (int64_t slot = slot0; slot <= slot1; slot += 1 << sib, slots += kMmaSlotFloats << sib) {
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -896,7 +908,7 @@ __global__ void __launch_bounds__(op_threads(CPLX, FOUR)) bfly_mma_post_kernel(c
   }
   if (p.bias_slots && p.group[blockIdx.z] == p.last_group && tid < kMmaCols) {
     double v = 0.0;
-    for (int c = c0; c <= c1; ++c) v += (double)p.bias_slots[mma_slot(g.geo, block, c) * kMmaCols + tid];
+    for (int64_t slot = slot0; slot <= slot1; slot += 1 << sib) v += (double)p.bias_slots[slot * kMmaCols + tid];
     const int64_t f = ((int64_t)s << g.geo.log_nf) + cbase + g.geo.col(tid);
     if (f < p.dbias_len) p.dbias[f] = (float)v;
   }

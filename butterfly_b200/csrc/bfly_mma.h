@@ -72,6 +72,14 @@ struct MmaGroup {
   MmaStage st[kMmaMaxStages];
 };
 
+// Row tiles of a block by 2^log_tiles: `count` parts, whose operator gradients (and column sums) are added up in float64.
+struct MmaParts {
+  int log_tiles, count;
+  BFLY_HD int of(int tile) const { return tile >> log_tiles; }
+  BFLY_HD bool ends(int tile) const { return ((tile + 1) & ((1 << log_tiles) - 1)) == 0; }
+  BFLY_HD bool begins(int tile) const { return tile > 0 && (tile & ((1 << log_tiles) - 1)) == 0; }
+};
+
 // Rows of the caller: (row, stack, column) at p[row * sB + stack * sS + column], columns from `cols` on read as zero and
 // are not written.  flat > 0: the stacks are side by side in one matrix of `flat` columns, the last ones cut short.
 struct MmaRowsIO {
@@ -89,6 +97,7 @@ BFLY_HD int mma_cols(const MmaRowsIO& r, int stack, int log_nf) {
 struct MmaPass {
   MmaGeom geo;
   int S, B, nq, nt;       // stacks, rows, blocks of a row, row tiles
+  MmaParts parts;
   const uint8_t* images;  // operators of the group, (stack, block)
   // forward: in -> out.  backward: gradient in -> out, x the activation that entered the group.  *_t: a plane instead of rows
   const float* in_t;
@@ -98,7 +107,7 @@ struct MmaPass {
   int reduce;             // backward: add to the output rows (their stack stride is 0)
   const float* bias;      // forward: bias[stack * nf + column] for flat positions below bias_len
   int bias_len;
-  float* slots;           // backward: operator gradients, slot = block of (stack, q) + CTA
+  float* slots;           // backward: operator gradients (mma_slot)
   float* bias_slots;      // backward: column sums of the incoming gradient, 64 per slot; may be null
   int* flag;              // set to 1 for values that are not ordinary
   const int* kept_flag;   // backward: the forward's, taken over; may be null
@@ -117,6 +126,7 @@ struct MmaPost {
   void* dtw[2];
   int64_t tw_stack[2];
   int S, nq, nt, ng, ctas;
+  MmaParts parts;
   int last_group, group[kMmaMaxGroups];  // number of the product's last group, and of g[i] (by the launch)
   const float* slots;     // (group, slot)
   int64_t slots_group;    // floats from a group to the next
@@ -132,9 +142,13 @@ struct MmaPost {
 // 2^sib, one block to a CTA of the group.
 BFLY_HD int64_t mma_first_tile(int64_t W, int G, int c) { return W * c / G; }
 BFLY_HD int mma_cta_of(int64_t W, int G, int64_t w) { return (int)(((w + 1) * G + W - 1) / W) - 1; }
-// CTAs of a pass, and where group c of them leaves the sums of a block: both walk up, so that no two share a slot.
+// CTAs of a pass, and where group c of them leaves its sums over part `part` of a block's row tiles (MmaParts): all three walk
+// up, so that no two sums share a slot.  Where a CTA begins with a part that is not a block's first, the slot in front of its own
+// stays free, and the CTA writes zeros there: the slots of a block are those from its first CTA's and part's to its last.
 BFLY_HD int mma_ctas(const MmaGeom& geo, int64_t tiles, int most) { return (int)(tiles < most ? tiles : most) >> geo.sib << geo.sib; }
-BFLY_HD int64_t mma_slot(const MmaGeom& geo, int64_t block, int c) { return block + ((int64_t)c << geo.sib); }
+BFLY_HD int64_t mma_slot(const MmaGeom& geo, const MmaParts& parts, int64_t block, int part, int c) {
+  return (((block >> geo.sib) * parts.count + part + c) << geo.sib) | (block & ((1 << geo.sib) - 1));
+}
 
 // ------------------------------------------------------------------ host planning
 
@@ -188,13 +202,27 @@ inline bool mma_groups(const std::vector<Stage>& st, int F, int log_n, std::vect
   return (int)out.size() <= kMmaMaxGroups;
 }
 
+// A float32 sum over the tiles of a long run is off by its roundings: 128 tiles of positive values, 16384 rows of 4096 columns,
+// 1.9e-7 for the gradient of the factors (phases 1.3e-7), parts of 32 tiles 1.1e-7.  A part more costs a slot, 32 KB written and
+// read where its rows are 2 MB.  Runs of up to 48 tiles (148 CTAs share the work) stay whole; few blocks, whose slots one CTA
+// each has to add up, get longer parts.
+inline MmaParts mma_parts(int64_t blocks, int64_t nt) {
+  MmaParts p{30, 1};
+  const int64_t run = std::min(nt, (blocks * nt + 147) / 148);
+  if (run > 48) p.log_tiles = blocks < 16 ? 7 : 5;
+  p.count = (int)(((nt - 1) >> p.log_tiles) + 1);
+  return p;
+}
+
 struct MmaLayout {
   std::vector<MmaGroup> g;
   int F, log_nf, nq;
   int64_t nt;                   // row tiles
+  MmaParts parts;
   size_t plane;                 // bytes of a plane
   size_t images;                // operators of all groups
   size_t slots, bias_slots;     // backward: operator gradients of all groups, bias sums
+  size_t slots_per_group(int S) const { return (size_t)S * nq * parts.count + kMmaBwMaxCtas; }
   // what a forward leaves: the flag, the activations between the groups, the operators
   size_t kept() const { return kMmaHead + (g.size() - 1) * plane + images; }
   // work space of a backward that starts from that (a gradient plane), and of one that makes it itself (the gradient takes

@@ -666,7 +666,7 @@ struct DryExec {
     if (p.out_t) plane(p.out_t, p); else io(p.out, p);
     // the last slot that a CTA can leave (mma_slot)
     const int used = mma_ctas(p.geo, (int64_t)p.S * p.nq * p.nt, ctas);
-    const int64_t last = mma_slot(p.geo, (int64_t)p.S * p.nq - 1, (used >> p.geo.sib) - 1) + 1;
+    const int64_t last = mma_slot(p.geo, p.parts, (int64_t)p.S * p.nq - 1, p.parts.of(p.nt - 1), (used >> p.geo.sib) - 1) + 1;
     in(p.slots, (size_t)last * kMmaSlotFloats * sizeof(float));
     if (p.bias_slots) in(p.bias_slots, (size_t)last * kMmaCols * sizeof(float));
     return BFLY_OK;
@@ -732,21 +732,36 @@ template <typename T> int check_mma_plan(const Problem& q, int most) {
     const int ctas = mma_ctas(g.geo, blocks * nt, most), sib = g.geo.sib, G = ctas >> sib;
     if (ctas < 1 || blocks % (1 << sib)) return 7;
     const int64_t W = (blocks >> sib) * nt;
-    std::vector<char> tile(blocks * nt, 0), slot(blocks + kMmaBwMaxCtas, 0);
+    std::vector<char> tile(blocks * nt, 0), slot(L.slots_per_group(q.S), 0);
+    std::vector<int64_t> owner(slot.size(), -1);
     for (int cta = 0; cta < ctas; ++cta) {
       const int c = cta >> sib;
-      int64_t last = -1;
-      for (int64_t w = mma_first_tile(W, G, c); w < mma_first_tile(W, G, c + 1); ++w) {
+      const int64_t begin = mma_first_tile(W, G, c), end = mma_first_tile(W, G, c + 1);
+      for (int64_t w = begin; w < end; ++w) {
         if (mma_cta_of(W, G, w) != c) return 8;
         const int64_t block = ((w / nt) << sib) + (cta & ((1 << sib) - 1));
         if (tile[block * nt + w % nt]++) return 9;
-        if (block != last) {
-          const int64_t at = mma_slot(g.geo, block, c);
-          if (at < 0 || at >= (int64_t)slot.size() || slot[at]++) return 10;
-          last = block;
-        }
+        const int t = (int)(w % nt), part = L.parts.of(t);
+        auto leave = [&](int64_t at) {
+          if (at < 0 || at >= (int64_t)slot.size() || slot[at]++) return false;
+          owner[at] = block;
+          return true;
+        };
+        if (w == begin && L.parts.begins(t) && !leave(mma_slot(g.geo, L.parts, block, part - 1, c))) return 10;
+        if ((t + 1 == nt || w + 1 == end || L.parts.ends(t)) && !leave(mma_slot(g.geo, L.parts, block, part, c))) return 10;
       }
     }
+    // what is added up for a block: slots that were left for it, all of them
+    int64_t left = 0, added = 0;
+    for (char s : slot) left += s;
+    for (int64_t block = 0; block < blocks; ++block) {
+      const int64_t first = (block >> sib) * nt;
+      const int64_t s0 = mma_slot(g.geo, L.parts, block, 0, mma_cta_of(W, G, first));
+      const int64_t s1 = mma_slot(g.geo, L.parts, block, L.parts.of((int)nt - 1), mma_cta_of(W, G, first + nt - 1));
+      for (int64_t s = s0; s <= s1; s += 1 << sib, ++added)
+        if (owner[s] != block) return 13;
+    }
+    if (left != added) return 14;
     for (char t : tile)
       if (!t) return 11;
   }

@@ -736,8 +736,9 @@ def test_plan_of_the_passes(emul, dtype):
             for nb in (1, 2, 3):
                 for base4 in (0, 1):
                     for inc in (0, 1):
-                        for B, S, ctas in ((1, 1, 148), (300, 3, 148), (5000, 1, 148), (4097, 5, 132), (129, 2, 7), (20000, 1, 160)):
-                            if B * S << log_n > 1 << 25:
+                        for B, S, ctas in ((1, 1, 148), (300, 3, 148), (5000, 1, 148), (4097, 5, 132), (129, 2, 7), (20000, 1, 160), (32768, 1, 148), (32768, 1, 64), (16384, 2, 128),
+                                           (1 << 20, 1, 148), (8192 * 128, 1, 64)):
+                            if B * S << log_n > 1 << 27 or (B > 1 << 19 and log_n > 7):
                                 continue
                             got = emul.bfly_emul_check_mma_plan(dtype, base4, B, S, log_n, nb, inc, ctas)
                             assert got <= 0, (log_n, nb, base4, inc, B, S, ctas, got)
