@@ -202,9 +202,9 @@ inline bool mma_groups(const std::vector<Stage>& st, int F, int log_n, std::vect
   return (int)out.size() <= kMmaMaxGroups;
 }
 
-// A float32 sum over the tiles of a long run is off by its roundings: 128 tiles of positive values, 16384 rows of 4096 columns,
-// 1.9e-7 for the gradient of the factors (phases 1.3e-7), parts of 32 tiles 1.1e-7.  A part more costs a slot, 32 KB written and
-// read where its rows are 2 MB.  Runs of up to 48 tiles (148 CTAs share the work) stay whole; few blocks, whose slots one CTA
+// A float32 sum over the tiles of a long run is off by its roundings: normal values, rows of 4096 columns, gradient of the factors
+// 1.7e-7 for 16384 rows and 2.6e-7 for 49152 in one part, 1.3e-7 and 1.8e-7 in parts of 32 tiles (phases 3.3e-7, 5.5e-7).  A
+// part more costs a slot, 32 KB written and read where its rows are 2 MB.  Runs of up to 48 tiles (148 CTAs share the work) stay whole; few blocks, whose slots one CTA
 // each has to add up, get longer parts.
 inline MmaParts mma_parts(int64_t blocks, int64_t nt) {
   MmaParts p{30, 1};
